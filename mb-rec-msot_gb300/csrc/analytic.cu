@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(AN_THREADS, 3) k_dmas_cf(
 constexpr int CT_WARPS = 4;
 __global__ void __launch_bounds__(32 * CT_WARPS) k_cumtrapz(const float *__restrict__ sig,
                                                             float *out, int cols,
-                                                            int T, int staged,
+                                                            int T, int ldo, int staged,
                                                             const float2 *__restrict__ fac) {
     extern __shared__ float ct_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(32 * CT_WARPS) k_cumtrapz(const float *__restr
     if (col >= cols) return;  // whole warp; no CTA-wide barriers below
     const int per = ((T + 31) / 32) | 1;  // odd: lanes' walks hit distinct banks
     const float *s = sig + (size_t)col * T;
-    float *o = out + (size_t)col * T;
+    float *o = out + (size_t)col * ldo;
     float *buf = staged ? ct_smem + (size_t)warp * (32 * per) : o;
     for (int t = lane; t < T; t += 32) buf[t] = __ldg(s + t);
     __syncwarp();
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(32 * CT_WARPS) k_cumtrapz(const float *__restr
 // each wavelength; psf is m (along T) x n (along D), column-major.
 __global__ void k_psf_same(const float *__restrict__ in, float *__restrict__ out,
                            const double *__restrict__ psf, int m, int n, double inv_sum, int D,
-                           int T) {
+                           int T, int ldo) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int d = blockIdx.y, w = blockIdx.z;
     if (t >= T) return;
@@ -223,7 +223,7 @@ __global__ void k_psf_same(const float *__restrict__ in, float *__restrict__ out
             acc += psf[a + (size_t)b * m] * (double)s[(size_t)dd * T + tt];
         }
     }
-    out[((size_t)w * D + d) * T + t] = (float)(acc * inv_sum);
+    out[((size_t)w * D + d) * ldo + t] = (float)(acc * inv_sum);
 }
 
 // backproject_waveeq.m:35-47: nearest-sample gather into the vector field, the
@@ -484,8 +484,9 @@ int msot_backproject_waveeq(const float *d_sig, int W, int D, int T, const doubl
     float *s1, *s2;
     const size_t n = (size_t)W * D * T;
     const int P = nx * nz;
+    const int ld = (T + 3) / 4 * 4;  // the GEMM's operand: 16-byte aligned columns
     RC(m.get(&s1, n));
-    RC(m.get(&s2, n));
+    RC(m.get(&s2, (size_t)W * D * ld));
     RC(m.get(&fx, (size_t)W * P));
     RC(m.get(&fz, (size_t)W * P));
     const double dt = 1.0 / fs;
@@ -504,17 +505,17 @@ int msot_backproject_waveeq(const float *d_sig, int W, int D, int T, const doubl
     if (!staged) ct_smem = 0;
     RC(set_smem(k_cumtrapz, ct_smem));
     KLAUNCH(k_cumtrapz<<<div_up(W * D, CT_WARPS), 32 * CT_WARPS, ct_smem, st>>>(
-        d_sig, one ? s2 : s1, W * D, T, staged, dfac));
+        d_sig, one ? s2 : s1, W * D, T, one ? ld : T, staged, dfac));
     if (!one) {
         RC(m.put(&dpsf, psf, (size_t)psf_m * psf_n));
         KLAUNCH(k_psf_same<<<dim3(div_up(T, 128), D, W), 128, 0, st>>>(s1, s2, dpsf, psf_m, psf_n,
-                                                                     1.0 / psum, D, T));
+                                                                     1.0 / psum, D, T, ld));
     }
     MSOT_LAUNCH_CHECK();
     // s1 = K(acq, acq) * s2 * dt : one column-major GEMM over all (d, w)
     // columns, on the tensor cores (gemm_tc.cu)
     const float *Ksub = d_K + (size_t)crop * K_n + crop;
-    RC(tc_sgemm(T, D * W, T, (float)dt, Ksub, K_n, s2, T, s1, T, st));
+    RC(tc_sgemm(T, D * W, T, (float)dt, Ksub, K_n, s2, ld, s1, T, st));
     const dim3 grid(div_up(nz, AN_TZ), div_up(nx, AN_TX), div_up(W, AN_FR));
     KLAUNCH(k_bp_gather<<<grid, AN_THREADS, 0, st>>>(s1, idx, cs, nx, nz, W, D, T, dt * c, fx, fz));
     KLAUNCH(k_div_fliplr<<<dim3(div_up(P, 256), W), 256, 0, st>>>(fx, fz, drx, drz, nx, nz, d_out));

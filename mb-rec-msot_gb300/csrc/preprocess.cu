@@ -20,9 +20,9 @@
 //
 // GPU: k_prep_columns (one CTA per column: crop, window, demean; FP64 means)
 // and, for the zero-phase filter, the circular convolution with
-// h = ifft(|H|^2) as one FP32 GEMM with the T x T circulant (cuBLAS SGEMM,
-// a plain library GEMM): 2 T^2 flops per column at the SGEMM rate instead of
-// an arbitrary-length FFT.
+// h = ifft(|H|^2) as one FP32 GEMM with the T x T circulant on the tensor
+// cores (gemm_tc.cu): 2 T^2 flops per column instead of an arbitrary-length
+// FFT.
 
 #include <cmath>
 #include <complex>
@@ -107,12 +107,12 @@ __device__ __forceinline__ double warp_total(const Sum1 &q) {
 constexpr int PC_WARPS = 4;
 __global__ void __launch_bounds__(32 * PC_WARPS) k_prep_columns(
     const float *raw, int T_raw, int n_crop, int T, const float *__restrict__ win, int demean,
-    float *out, int cols, int stride) {
+    float *out, int cols, int ldo) {
     extern __shared__ float pc_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int c = blockIdx.x * PC_WARPS + warp;
     if (c >= cols) return;  // whole warp; no CTA-wide barriers below
-    float *col = pc_smem + (size_t)warp * stride;
+    float *col = pc_smem + (size_t)warp * T;
     const float *src = raw + (size_t)c * T_raw + n_crop;
     Sum1 s;
     for (int t = lane; t < T; t += 32) {
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(32 * PC_WARPS) k_prep_columns(
             s.add(v);
         }
     }
-    float *dst = out + (size_t)c * T;
+    float *dst = out + (size_t)c * ldo;
     const float m = demean ? (float)(warp_total(s) / T) : 0.f;
     for (int t = lane; t < T; t += 32) dst[t] = demean ? col[t] - m : col[t];
 }
@@ -152,7 +152,8 @@ struct msot_prep {
     int T_raw = 0, n_crop = 0, T = 0, max_cols = 0, demean = 0;
     float *win = nullptr;   // [T] window |h|, or null
     float *circ = nullptr;  // [T][T] circulant of ifft(|H|^2) (column-major), or null
-    float *work = nullptr;  // [max_cols][T] GEMM input
+    float *work = nullptr;  // [max_cols][ld()] GEMM input
+    int ld() const { return (T + 3) / 4 * 4; }  // 16-byte aligned columns
     ~msot_prep() {
         cudaFree(win);
         cudaFree(circ);
@@ -254,7 +255,7 @@ int msot_prep_create(int T_raw, int n_crop, int window_order, double window_low,
         if ((e = cudaMemcpy(pp->circ, C.data(), sizeof(float) * C.size(),
                             cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail(e);
-        if ((e = cudaMalloc(&pp->work, sizeof(float) * (size_t)max_cols * T)) != cudaSuccess)
+        if ((e = cudaMalloc(&pp->work, sizeof(float) * (size_t)max_cols * pp->ld())) != cudaSuccess)
             return fail(e);
     }
     *out = pp;
@@ -286,11 +287,12 @@ int msot_prep_apply(msot_prep_t p, const float *d_raw, float *d_out, int n_cols,
     int rc = set_smem(k_prep_columns, smem);
     if (rc) return rc;
     KLAUNCH(k_prep_columns<<<div_up(n_cols, PC_WARPS), 32 * PC_WARPS, smem, st>>>(
-        d_raw, p->T_raw, p->n_crop, p->T, p->win, p->demean, dst, n_cols, p->T));
+        d_raw, p->T_raw, p->n_crop, p->T, p->win, p->demean, dst, n_cols,
+        p->circ ? p->ld() : p->T));
     MSOT_LAUNCH_CHECK();
     // the zero-phase filter: the T x T circulant times the columns, on the
     // tensor cores (gemm_tc.cu)
-    if (p->circ) return tc_sgemm(p->T, n_cols, p->T, 1.f, p->circ, p->T, p->work, p->T, d_out,
+    if (p->circ) return tc_sgemm(p->T, n_cols, p->T, 1.f, p->circ, p->T, p->work, p->ld(), d_out,
                                  p->T, st);
     return MSOT_OK;
 }

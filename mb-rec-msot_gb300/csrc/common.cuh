@@ -109,6 +109,12 @@ struct Plan {
     // register pair m and lane, (re a, re b, im a, im b) of w^(lane k1) for
     // k1 = brev5(2m), brev5(2m + 1); conj w^(lane n) for n = 2m, 2m + 1; and
     // H[lane + 32 k2] for k2 = brev5(2m), brev5(2m + 1)  ([16][32] each)
+    // support of the interpolation per detector, [first, last + 1) samples over
+    // the taps of its pixels (SIR: the whole row), and the 1024-point
+    // convolution's tiles per column pair that it needs, forward and transpose
+    int2 *conv_rng = nullptr;
+    int conv_nt_f = 0, conv_nt_a = 0;
+    int conv_diff = 0;  // fft_hfb holds the spectrum of the taps' running sum
     float4 *fft_twb = nullptr, *fft_twn = nullptr, *fft_hfb = nullptr, *fft_hab = nullptr;
     // prefilter
     int Kx = -1, Kz = -1;   // -1: no prefilter along that axis
@@ -149,11 +155,11 @@ inline int set_smem(K kern, size_t bytes) {
 // k_das_fwd3 launches per storage format of the interpolation input (xpm of
 // FP32, BF16 or FP16 values; inv_s: the FP16 inverse scales, else null)
 int das_fwd_run_f32(const Plan &pl, const void *xpm, float *raw, int W, float scale,
-                    const float *inv_s, bool ell, int wt, cudaStream_t st);
+                    const float *inv_s, bool ell, int wt, const int2 *skip, cudaStream_t st);
 int das_fwd_run_bf16(const Plan &pl, const void *xpm, float *raw, int W, float scale,
-                     const float *inv_s, bool ell, int wt, cudaStream_t st);
+                     const float *inv_s, bool ell, int wt, const int2 *skip, cudaStream_t st);
 int das_fwd_run_f16(const Plan &pl, const void *xpm, float *raw, int W, float scale,
-                    const float *inv_s, bool ell, int wt, cudaStream_t st);
+                    const float *inv_s, bool ell, int wt, const int2 *skip, cudaStream_t st);
 
 
 // tensor-core convolutions of the warm-start U-Net on (1) or off (0); unet.cu
@@ -222,7 +228,7 @@ int launch_prefilter(const Plan &pl, const float *in, float *out, int W, bool tr
 int launch_to_pixmajor(const Plan &pl, const float *in, float *out, int W, cudaStream_t st);
 int launch_permute(const Plan &pl, const float *in, float *out, int W, cudaStream_t st);
 int launch_das_forward(const Plan &pl, const float *x_pi, float *raw, int W, float scale,
-                       cudaStream_t st);
+                       cudaStream_t st, bool to_conv);
 int launch_das_adjoint(const Plan &pl, const float *raw, float *x, int W, float scale,
                        cudaStream_t st);
 int launch_conv(const Plan &pl, const float *in, float *out, int W, bool transpose,
@@ -231,8 +237,10 @@ int launch_sir_forward(const Plan &pl, const float *x_pi, float *raw, int W, flo
                        cudaStream_t st);
 int launch_sir_adjoint(const Plan &pl, const float *raw, float *x, int W, float scale,
                        cudaStream_t st);
+// to_conv: raw is read by the 1024-point convolution, which takes only each
+// detector's support (Plan::conv_rng), so tiles outside it are not written
 int interp_forward(const Plan &pl, const float *x_pi, float *raw, int W, float scale,
-                   cudaStream_t st);
+                   cudaStream_t st, bool to_conv = false);
 int interp_adjoint(const Plan &pl, const float *raw, float *x, int W, float scale,
                    cudaStream_t st);
 int apply_forward(const Plan &pl, const float *img, float *sino, int W, cudaStream_t st);

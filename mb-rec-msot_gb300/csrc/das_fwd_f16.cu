@@ -4,8 +4,8 @@
 namespace msot {
 
 int das_fwd_run_f16(const Plan &pl, const void *xpm, float *raw, int W, float scale,
-                   const float *inv_s, bool ell, int wt, cudaStream_t st) {
-    return das_fwd_run<__half>(pl, xpm, raw, W, scale, inv_s, ell, wt, st);
+                   const float *inv_s, bool ell, int wt, const int2 *skip, cudaStream_t st) {
+    return das_fwd_run<__half>(pl, xpm, raw, W, scale, inv_s, ell, wt, skip, st);
 }
 
 }  // namespace msot

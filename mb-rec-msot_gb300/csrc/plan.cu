@@ -98,7 +98,7 @@ static void free_plan(Plan &p) {
                     p.scr_sino, p.fwd_off, p.fwd_ent, p.blk_tau, p.blk_span,
                     p.scr_part, p.fft_tw, p.fft_hf, p.fft_ha, p.fft_twb, p.fft_twn,
                     p.fft_hfb, p.fft_hab, p.st_info, p.st_u, p.st_off, p.st_ent,
-                    p.h16_sc, p.fwd_ell, p.fwd_ell_off};
+                    p.h16_sc, p.fwd_ell, p.fwd_ell_off, p.conv_rng};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     p = Plan();
@@ -250,6 +250,16 @@ static int build(const msot_plan_desc *d, Plan &p) {
         felloff.push_back((int32_t)fell.size());
     }
 
+    // --- support of the interpolation per detector: taps floor(tau) - F ..
+    // floor(tau) + F + 1 of its pixels; SIR responses may reach the whole row
+    std::vector<int2> rng(p.D, make_int2(0, p.T));
+    for (int det = 0; det < p.D && !has_sir; ++det) {
+        const int32_t *tf = tfx.data() + (size_t)det * p.P;
+        const auto mm = std::minmax_element(tf, tf + p.P);
+        rng[det] = make_int2(std::max(0, (*mm.first >> fb) - p.F),
+                             std::min(p.T, (*mm.second >> fb) + p.F + 2));
+    }
+
     // --- adjoint blocks: 64x64 pixels, travel times and bucket span per detector --------
     std::vector<int32_t> btau;
     std::vector<int2> bspan;
@@ -379,13 +389,24 @@ static int build(const msot_plan_desc *d, Plan &p) {
         const double two_pi = 6.283185307179586476925286766559;
         for (int t = 0; t < N; ++t)
             ftw[t] = make_float2((float)std::cos(two_pi * t / N), (float)-std::sin(two_pi * t / N));
+        // taps that sum to zero: the forward direction of the 1024-point path
+        // takes differenced input and the taps' running sum (operator.cu)
+        std::vector<double> hf0(d->ir, d->ir + p.L);
+        double sum = 0.0, mag = 0.0;
+        for (double v : hf0) sum += v, mag += std::fabs(v);
+        if (p.fft_log4n == 5 && std::fabs(sum) <= 1e-11 * mag) {
+            p.conv_diff = 1;
+            double run = 0.0;
+            for (int k = 0; k < p.L; ++k) hf0[k] = run += d->ir[k];
+            hf0[p.L - 1] = 0.0;
+        }
         // direct DFT of the short tap vectors: H[f] = sum_k h[k] e^{-2 pi i f k / N} / N
         for (int f = 0; f < N; ++f) {
             double fr = 0, fi = 0, ar = 0, ai = 0;
             for (int k = 0; k < p.L; ++k) {
                 const double ang = -two_pi * (double)(((long)f * k) % N) / N;
                 const double c = std::cos(ang), sn = std::sin(ang);
-                const double hf = d->ir[k] / p.norm, ha = d->ir[p.L - 1 - k] / p.norm;
+                const double hf = hf0[k] / p.norm, ha = d->ir[p.L - 1 - k] / p.norm;
                 fr += hf * c; fi += hf * sn;
                 ar += ha * c; ai += ha * sn;
             }
@@ -395,6 +416,16 @@ static int build(const msot_plan_desc *d, Plan &p) {
     }
     std::vector<float4> ftwb, ftwn, fhfb, fhab;
     if (p.fft_log4n == 5) {
+        // tiles that the widest column pair (neighbouring detectors, or the
+        // last and the first of two instances) needs
+        const int V = 1024 - p.L + 1, h = p.L / 2;
+        for (int det = 0; det < p.D; ++det) {
+            const int2 a = rng[det], b = rng[(det + 1) % p.D];
+            const int lo = std::min(a.x, b.x), hi = std::max(a.y, b.y);
+            p.conv_nt_a = std::max(p.conv_nt_a, div_up(hi - lo, V));
+            p.conv_nt_f = std::max(p.conv_nt_f,
+                                   div_up(std::min(p.T, hi + h) - std::max(0, lo - h), V));
+        }
         auto brev5 = [](int i) {
             return ((i & 1) << 4) | ((i & 2) << 2) | (i & 4) | ((i & 8) >> 2) | ((i & 16) >> 4);
         };
@@ -471,6 +502,7 @@ static int build(const msot_plan_desc *d, Plan &p) {
         UP(p.fft_twn, ftwn);
         UP(p.fft_hfb, fhfb);
         UP(p.fft_hab, fhab);
+        UP(p.conv_rng, rng);
     }
     if (p.Kx >= 0) {
         std::vector<float> v(px.begin(), px.end());

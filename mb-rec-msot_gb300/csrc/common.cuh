@@ -78,6 +78,12 @@ struct Plan {
     int32_t *blk_tau = nullptr;    // [n_blk][D][BLK_PPT][BLK_THREADS] (TAU_PAD outside)
     int2 *blk_span = nullptr;      // [n_blk][D] first / last bucket of the block
     int blk_span_max = 0;          // largest last - first + 1
+    // batched adjoint (das_adj.cu), null / 0 where the plan has no such table:
+    // per 32 x 32 sub-block and detector the bucket span, and per pixel the
+    // knot row and the position between it and the next
+    int2 *adj5_span = nullptr;     // [4 n_blk][D]
+    uint32_t *adj5_ent = nullptr;  // [4 n_blk][D][1024]
+    int adj5_span_max = 0, adj5_rowbits = 0;
     int adj_groups_max = 0;        // detector groups the partial buffer is sized for
     float *scr_part = nullptr;     // [adj_groups_max][max_batch][P] adjoint partial sums
     struct SolverCache *solver = nullptr;  // solver workspace and captured CUDA graphs
@@ -221,6 +227,18 @@ class TimedScope {
             return MSOT_ECUDA;                                                         \
         }                                                                              \
     } while (0)
+
+// batched DAS forward, lanes over instances (das_fwd_lanes.cu): FP32 input in
+// [ceil(W / wt)][P][wt], wt = 16 or 32
+int launch_das_forward_lanes(const Plan &pl, const float *xpm, float *raw, int W, int wt,
+                             float scale, const int2 *skip, cudaStream_t st);
+// batched DAS adjoint, lanes over instances (das_adj.cu)
+int adj5_build(Plan &p, size_t &bytes);
+bool adj5_usable(const Plan &pl, int W);
+int launch_das_adjoint5(const Plan &pl, const float *raw, float *x, int W, float scale,
+                        cudaStream_t st);
+// x[i] = scale * sum over groups of part[g * n + i], in order; operator.cu
+int sum_parts(const float *part, float *x, size_t n, int groups, float scale, cudaStream_t st);
 
 // operator chains (operator.cu)
 int launch_prefilter(const Plan &pl, const float *in, float *out, int W, bool transpose,

@@ -160,7 +160,8 @@ __global__ void __launch_bounds__(256, WT >= 16 ? 2 : 4) k_das_fwd3(const int32_
             const int t = t0 + (int)threadIdx.x;
             if ((int)threadIdx.x < TB && t < T) {
 #pragma unroll
-                for (int i = 0; i < WT; ++i) raw[((size_t)(w0 + i) * D + d) * T + t] = 0.f;
+                for (int i = 0; i < WT; ++i)
+                    if (w0 + i < W) raw[((size_t)(w0 + i) * D + d) * T + t] = 0.f;
             }
             return;
         }
@@ -258,7 +259,9 @@ __global__ void __launch_bounds__(256, WT >= 16 ? 2 : 4) k_das_fwd3(const int32_
             v1 += M1[-k];
         }
         const float acc = fmaf(v1 - v0, inv_r, u0 + u1);
-        raw[((size_t)(w0 + i) * D + d) * T + t] = acc * (inv_s ? scale * __ldg(inv_s + w0 + i) : scale);
+        if (w0 + i < W)
+            raw[((size_t)(w0 + i) * D + d) * T + t] =
+                acc * (inv_s ? scale * __ldg(inv_s + w0 + i) : scale);
     }
 }
 
@@ -266,7 +269,7 @@ template <int WT, int F, typename XT, bool ELL>
 inline int das_fwd_launch_t(const Plan &pl, const XT *xpm, float *raw, int W, float scale,
                             const float *inv_s, const int2 *skip, cudaStream_t st) {
     constexpr int NB = 256, TB = NB - 2 * F - 2;
-    dim3 grid(div_up(pl.T, TB), pl.D, W / WT);
+    dim3 grid(div_up(pl.T, TB), pl.D, div_up(W, WT));
     const size_t smem = (size_t)4 * WT * NB * sizeof(float);
     int rc;
     if ((rc = set_smem(k_das_fwd3<WT, F, XT, ELL>, smem)) != MSOT_OK) return rc;

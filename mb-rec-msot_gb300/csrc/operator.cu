@@ -1202,26 +1202,52 @@ static bool use_staged(const Plan &pl, int wt) {
     return fwd_kernel(pl) == 1 && fwd_staged_fits(pl, wt);
 }
 
-// instances per CTA of the DAS forward: the autotuner's pick (16, 8, 4, 2),
-// else the largest of 8, 4, 2 dividing W
+// the lanes-over-instances kernel (das_fwd_lanes.cu) serves batches above 8 of
+// the FP32 input unless the autotuner or a knob chose another kernel
+static bool fwd_lanes(const Plan &pl) {
+    return !pl.tune_fwd_staged && g_fwd_ell.load() && !pl.image_fmt;
+}
+
+// instances per CTA of the DAS forward, the last tile part-filled: the
+// autotuner's pick (16, 8, 4, 2), else 32 or 16 for the lanes kernel, else the
+// next power of two up to 8
 int das_fwd_wt(const Plan &pl, int W) {
     if (pl.tune_fwd_wt && W % pl.tune_fwd_wt == 0) return pl.tune_fwd_wt;
-    return pick_wt(W, 1, 8);
+    if (!fwd_lanes(pl)) {
+        int wt = 1;  // a part-filled tile of 8 costs less than W narrow ones
+        while (wt < W && wt < 8) wt *= 2;
+        return wt;
+    }
+    if (W > 8) return (W + 31) / 32 * 32 - W < 16 ? 32 : 16;
+    int wt = 1;
+    while (wt < W) wt *= 2;
+    return wt;
 }
 
 int launch_das_forward(const Plan &pl, const float *xpm, float *raw, int W, float scale,
                        cudaStream_t st, bool to_conv) {
     TimedScope ts_(KID_INTERP_FWD, st);
     const int wt = das_fwd_wt(pl, W);
-    if (use_staged(pl, wt)) return launch_das_forward_staged(pl, xpm, raw, W, wt, scale, st);
+    if (wt > 8 && fwd_lanes(pl))
+        return launch_das_forward_lanes(pl, xpm, raw, W, wt, scale,
+                                        to_conv ? pl.conv_rng : nullptr, st);
+    if (use_staged(pl, wt) && W % wt == 0) return launch_das_forward_staged(pl, xpm, raw, W, wt, scale, st);
     // k_das_fwd3 in the plan's storage format (das_fwd_f32.cu, das_fwd_bf16.cu,
     // das_fwd_f16.cu), on the interleaved entry table where chosen
     const bool ell = fwd_kernel(pl) == 4 && pl.fwd_ell_off;
     const int2 *skip = to_conv ? pl.conv_rng : nullptr;
-    if (pl.image_fmt == 1) return das_fwd_run_bf16(pl, xpm, raw, W, scale, nullptr, ell, wt, skip, st);
+    if (pl.image_fmt == 1)
+        return das_fwd_run_bf16(pl, xpm, raw, W, scale, nullptr, ell, wt, skip, st);
     if (pl.image_fmt == 2)
         return das_fwd_run_f16(pl, xpm, raw, W, scale, pl.h16_sc + pl.max_batch, ell, wt, skip, st);
     return das_fwd_run_f32(pl, xpm, raw, W, scale, nullptr, ell, wt, skip, st);
+}
+
+int sum_parts(const float *part, float *x, size_t n, int groups, float scale, cudaStream_t st) {
+    KLAUNCH(k_sum_parts<<<(unsigned)std::min<size_t>(4096, (n + 255) / 256), 256, 0, st>>>(
+        part, x, n, groups, n, scale));
+    MSOT_LAUNCH_CHECK();
+    return MSOT_OK;
 }
 
 // DAS adjoint by pixel blocks; raw [W][D][T] -> x [W][P].
@@ -1235,7 +1261,6 @@ static int das_adj_launch(const Plan &pl, const float *raw, float *x, int W, flo
     const int base = pl.n_blk * (W / WT);
     int groups = std::max(1, std::min(pl.D, div_up(2 * sm_count(), base)));
     groups = std::min(groups, std::max(1, pl.adj_groups_max * pl.max_batch / W));
-    groups = std::min(groups, pl.adj_groups_max);
     const int dpg = div_up(pl.D, groups);
     groups = div_up(pl.D, dpg);
     const size_t stride = (size_t)W * pl.P;
@@ -1257,10 +1282,7 @@ static int das_adj_launch(const Plan &pl, const float *raw, float *x, int W, flo
         ADJ4_LAUNCH(0);
 #undef ADJ4_LAUNCH
     MSOT_LAUNCH_CHECK();
-    KLAUNCH(k_sum_parts<<<(unsigned)std::min<size_t>(4096, div_up((int)stride, 256)), 256, 0,
-                          st>>>(pl.scr_part, x, stride, groups, stride, scale));
-    MSOT_LAUNCH_CHECK();
-    return MSOT_OK;
+    return sum_parts(pl.scr_part, x, stride, groups, scale, st);
 }
 
 template <int WT>
@@ -1286,8 +1308,12 @@ static int das_adj_f(const Plan &pl, const float *raw, float *x, int W, float sc
 int launch_das_adjoint(const Plan &pl, const float *raw, float *x, int W, float scale,
                        cudaStream_t st) {
     TimedScope ts_(KID_INTERP_ADJ, st);
+    // the batched kernel unless the autotuner found a wt of k_das_adj4 faster
     int wt = pick_wt(W, 1, 2);
-    if (pl.tune_adj_wt && W % pl.tune_adj_wt == 0) wt = pl.tune_adj_wt;
+    if (pl.tune_adj_wt && W % pl.tune_adj_wt == 0)
+        wt = pl.tune_adj_wt;
+    else if (adj5_usable(pl, W))
+        return launch_das_adjoint5(pl, raw, x, W, scale, st);
     if (wt == 4) return das_adj_f<4>(pl, raw, x, W, scale, st);
     if (wt == 2) return das_adj_f<2>(pl, raw, x, W, scale, st);
     return das_adj_f<1>(pl, raw, x, W, scale, st);

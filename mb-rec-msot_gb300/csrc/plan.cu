@@ -98,7 +98,7 @@ static void free_plan(Plan &p) {
                     p.scr_sino, p.fwd_off, p.fwd_ent, p.blk_tau, p.blk_span,
                     p.scr_part, p.fft_tw, p.fft_hf, p.fft_ha, p.fft_twb, p.fft_twn,
                     p.fft_hfb, p.fft_hab, p.st_info, p.st_u, p.st_off, p.st_ent,
-                    p.h16_sc, p.fwd_ell, p.fwd_ell_off, p.conv_rng};
+                    p.adj5_span, p.adj5_ent, p.h16_sc, p.fwd_ell, p.fwd_ell_off, p.conv_rng};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     p = Plan();
@@ -481,6 +481,7 @@ static int build(const msot_plan_desc *d, Plan &p) {
         UP(p.fwd_ell_off, felloff);
         UP(p.blk_tau, btau);
         UP(p.blk_span, bspan);
+        if ((rc = adj5_build(p, B)) != MSOT_OK) return rc;
     }
     if (has_sir) {
         UP(p.sir, sirf);
@@ -515,7 +516,10 @@ static int build(const msot_plan_desc *d, Plan &p) {
 #undef UP
     const size_t W = (size_t)p.max_batch;
     if ((rc = alloc(&p.scr_img0, W * p.P, B)) != MSOT_OK) return rc;
-    if ((rc = alloc(&p.scr_img1, W * p.P, B)) != MSOT_OK) return rc;
+    // the forward's input is padded to whole instance tiles (at most 32); the
+    // padding is read, never used
+    if ((rc = alloc(&p.scr_img1, (W + 31) / 32 * 32 * p.P, B)) != MSOT_OK) return rc;
+    MSOT_CUDA_TRY(cudaMemset(p.scr_img1, 0, (W + 31) / 32 * 32 * p.P * sizeof(float)));
     if ((rc = alloc(&p.scr_sino, W * p.D * p.T, B)) != MSOT_OK) return rc;
     if ((rc = alloc(&p.h16_sc, 2 * W, B)) != MSOT_OK) return rc;
     p.pre_gain_x = p.pre_gain_z = 1.f;  // bounds of |prefiltered| / max |input|

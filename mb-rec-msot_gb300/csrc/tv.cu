@@ -1689,8 +1689,14 @@ extern "C" int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tun
     // 4 the same on the interleaved table) and instances per CTA
     // (apply_forward: prefilter, forward, conv)
     {
-        double best = 1e30;
+        // fwd_wt and fwd_staged report the best of these; the plan takes it only
+        // where it beats the built-in choice (0)
+        double best = 1e30, builtin = 0.0;
         int pick = 0, pick_kernel = 0;
+        pl.tune_fwd_wt = pl.tune_fwd_staged = 0;
+        if ((rc = tune_time(st, 3, builtin,
+                            [&] { return apply_forward(pl, img, sino, batch, st); })))
+            return rc;
         for (int kernel : {1, 2, 4}) {
             if (kernel == 1 && !pl.st_tt) continue;
             if (kernel == 4 && !pl.fwd_ell_off) continue;
@@ -1706,16 +1712,22 @@ extern "C" int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tun
                 if (ms < best) best = ms, pick = wt, pick_kernel = kernel;
             }
         }
-        pl.tune_fwd_wt = pick;
-        pl.tune_fwd_staged = pick_kernel;
+        pl.tune_fwd_wt = best < builtin ? pick : 0;
+        pl.tune_fwd_staged = best < builtin ? pick_kernel : 0;
         res.fwd_wt = pick;
         res.fwd_staged = pick_kernel;
-        res.fwd_ms = pick ? best : 0.0;
+        res.fwd_ms = std::min(best, builtin);
     }
     // DAS adjoint: instances per CTA (apply_transpose)
     {
-        double best = 1e30;
+        // adj_wt reports the best k_das_adj4 tile; the plan takes it only where it
+        // beats the built-in choice (0: the batched kernel from 3 instances up)
+        double best = 1e30, builtin = 0.0;
         int pick = 0;
+        pl.tune_adj_wt = 0;
+        if ((rc = tune_time(st, 3, builtin,
+                            [&] { return apply_transpose(pl, sino, img2, batch, st); })))
+            return rc;
         for (int wt : {4, 2, 1}) {
             if (batch % wt) continue;
             pl.tune_adj_wt = wt;
@@ -1725,7 +1737,7 @@ extern "C" int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tun
                 return rc;
             if (ms < best) best = ms, pick = wt;
         }
-        pl.tune_adj_wt = pick;
+        pl.tune_adj_wt = best < builtin ? pick : 0;
         res.adj_wt = pick;
     }
     // IR convolution register cap (apply_transpose: conv, adjoint, prefilter)

@@ -135,106 +135,122 @@ __global__ void k_prefilter(const float *__restrict__ in, float *__restrict__ ou
 }
 
 // ---------------------------------------------------------------------------
-// Both prefilter axes in one pass through shared memory.  CTA = (tile of TX
-// columns ix, instance w); it stages the columns ix0 - KM .. ix0 + TX + KM - 1
-// (circular) of the image, filters every staged column along z into a second
-// buffer, then filters along x into the TX output columns.  Each thread
-// slides a register window over 8 consecutive outputs, so a tap costs one
-// FMA and (8 + 2 KM) / 8 / (2 KM + 1) shared loads.  Taps are zero-padded to
-// the compile-time half width KM >= K.  out_mode 0 = [W][P], 2 = [W/wt][P][wt].
+// Both prefilter axes in one pass through shared memory.  CTA = (32 x 32 pixel
+// tile, IPC instances); it stages the tile and KM pixels around it (circular),
+// filters the staged columns along z into a second buffer, then along x.  Each
+// thread slides a register window over 8 (z) or 4 (x) consecutive outputs, so
+// a tap costs one FMA and a fraction of a shared load.  Taps are zero-padded
+// to the compile-time half width KM >= K.  out_mode 0 = [W][P], 2 =
+// [W/wt][P][wt]; there, with FP32 and wt a multiple of 4, IPC = 4 and a
+// pixel's four instances leave as one 16-byte store.
+//
+// Square tiles instead of 32 whole columns: 16 CTAs instead of 4 for one image
+// of 128 x 128 px (18 -> 7 us), and any grid size (400 x 400 px took one
+// launch per axis with every tap from global memory: 13 images 133 -> 28
+// us); batch 64 at 128 x 128 px 23 -> 14 to 16 us, the stores were the bound.
 // ---------------------------------------------------------------------------
-constexpr int PF_TX = 32, PF_R = 8, PF_THREADS = 256;
+constexpr int PF_T = 32, PF_RZ = 8, PF_RX = 4, PF_THREADS = 256;
 
 __device__ __forceinline__ int wrap_mod(int a, int n) {
     a %= n;
     return a < 0 ? a + n : a;
 }
 
-template <int KM>
+template <int KM, int IPC>
 __global__ void __launch_bounds__(PF_THREADS) k_prefilter2d(
     const float *__restrict__ in, float *__restrict__ out, const float *__restrict__ taps_x,
     const float *__restrict__ taps_z, int Kx, int Kz, int nx, int nz, int W, int transpose,
     int out_mode, int wt, int fmt, const float *__restrict__ hsc) {
-    constexpr int NC = PF_TX + 2 * KM;  // staged columns
+    constexpr int NC = PF_T + 2 * KM;  // staged columns and rows
+    constexpr int LA = NC | 1, LB = PF_T + 1;  // odd strides: lanes over columns hit distinct banks
     constexpr int NTAP = 2 * KM + 1;
     constexpr int NW = PF_THREADS / 32;
     extern __shared__ float pf_smem[];
-    const int ld = nz | 1;         // odd column stride: lanes over columns hit distinct banks
-    float *A = pf_smem;            // [NC][ld] staged input
-    float *B = A + NC * ld;        // [NC][ld] z-filtered
-    float *hz = B + NC * ld;       // [NTAP] tap for offset k at hz[k + KM]
+    float *A = pf_smem;               // [NC][LA] staged input
+    float *B = A + NC * LA;           // [IPC][NC][LB] z-filtered
+    float *hz = B + IPC * NC * LB;    // [NTAP] tap for offset k at hz[k + KM]
     float *hx = hz + NTAP;
-    const int w = blockIdx.y, ix0 = blockIdx.x * PF_TX;
+    const int w0 = blockIdx.z * IPC, ix0 = blockIdx.x * PF_T, iz0 = blockIdx.y * PF_T;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const float *src = in + (size_t)w * nx * nz;
     for (int k = threadIdx.x; k < NTAP; k += PF_THREADS) {
         const int o = k - KM;
         hz[k] = (o >= -Kz && o <= Kz) ? taps_z[transpose ? Kz - o : Kz + o] : 0.f;
         hx[k] = (o >= -Kx && o <= Kx) ? taps_x[transpose ? Kx - o : Kx + o] : 0.f;
     }
-    // stage: one warp per column, lanes along z
-    for (int c = warp; c < NC; c += NW) {
-        const float *scol = src + (size_t)wrap_mod(ix0 - KM + c, nx) * nz;
-        float *dcol = A + c * ld;
-        for (int z = lane; z < nz; z += 32) dcol[z] = __ldg(scol + z);
-    }
-    __syncthreads();
-    // z pass, lanes over columns: B[c][z] = sum_k hz[k] A[c][z - k (circular)]
-    const int nzc = (nz + PF_R - 1) / PF_R;
-    constexpr int NCG = (NC + 31) / 32;
-    for (int it = warp; it < NCG * nzc; it += NW) {
-        const int cg = it / nzc, z0 = (it - cg * nzc) * PF_R;
-        const int c = cg * 32 + lane;
-        if (c < NC) {
-            const float *col = A + c * ld;
-            float win[PF_R + 2 * KM];
+    constexpr int RPL = (NC + 31) / 32;  // staged rows per lane
+    int row[RPL];
 #pragma unroll
-            for (int i = 0; i < PF_R + 2 * KM; ++i) {
-                int z = z0 - KM + i;
-                z = (z >= 0 && z < nz) ? z : wrap_mod(z, nz);
-                win[i] = col[z];
+    for (int j = 0; j < RPL; ++j) row[j] = wrap_mod(iz0 - KM + lane + 32 * j, nz);
+#pragma unroll 1
+    for (int i = 0; i < IPC; ++i) {
+        const float *src = in + (size_t)min(w0 + i, W - 1) * nx * nz;
+        if (i) __syncthreads();  // the z pass before is done with A
+        // one warp per column, lanes along z
+        for (int c = warp; c < NC; c += NW) {
+            const float *scol = src + (size_t)wrap_mod(ix0 - KM + c, nx) * nz;
+#pragma unroll
+            for (int j = 0; j < RPL; ++j)
+                if (lane + 32 * j < NC) A[c * LA + lane + 32 * j] = __ldg(scol + row[j]);
+        }
+        __syncthreads();
+        // z pass, lanes over columns: B[c][z] = sum_k hz[k] A[c][z + KM - k]
+        constexpr int NCG = (NC + 31) / 32;
+        for (int it = warp; it < NCG * (PF_T / PF_RZ); it += NW) {
+            const int c = (it % NCG) * 32 + lane, z0 = (it / NCG) * PF_RZ;
+            if (c < NC) {
+                const float *col = A + c * LA + z0;
+                float win[PF_RZ + 2 * KM];
+#pragma unroll
+                for (int j = 0; j < PF_RZ + 2 * KM; ++j) win[j] = col[j];
+                float acc[PF_RZ];
+#pragma unroll
+                for (int j = 0; j < PF_RZ; ++j) acc[j] = 0.f;
+#pragma unroll
+                for (int k = -KM; k <= KM; ++k) {
+                    const float h = hz[k + KM];
+#pragma unroll
+                    for (int j = 0; j < PF_RZ; ++j) acc[j] = fmaf(h, win[j - k + KM], acc[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < PF_RZ; ++j) B[(i * NC + c) * LB + z0 + j] = acc[j];
             }
-            float acc[PF_R];
-#pragma unroll
-            for (int j = 0; j < PF_R; ++j) acc[j] = 0.f;
-#pragma unroll
-            for (int k = -KM; k <= KM; ++k) {
-                const float h = hz[k + KM];
-#pragma unroll
-                for (int j = 0; j < PF_R; ++j) acc[j] = fmaf(h, win[j - k + KM], acc[j]);
-            }
-#pragma unroll
-            for (int j = 0; j < PF_R; ++j)
-                if (z0 + j < nz) B[c * ld + z0 + j] = acc[j];
         }
     }
     __syncthreads();
     // x pass, lanes along z: out[ix0 + c][z] = sum_k hx[k] B[c + KM - k][z]
-    constexpr int NXC = PF_TX / PF_R;
-    for (int it = threadIdx.x; it < NXC * nz; it += PF_THREADS) {
-        const int cc = it / nz, z = it - cc * nz, c0 = cc * PF_R;
-        float win[PF_R + 2 * KM];
+    const int iz = iz0 + lane;
+    for (int c0 = warp * PF_RX; c0 < PF_T; c0 += NW * PF_RX) {
+        float acc[IPC][PF_RX];
 #pragma unroll
-        for (int i = 0; i < PF_R + 2 * KM; ++i) win[i] = B[(c0 + i) * ld + z];
-        float acc[PF_R];
+        for (int i = 0; i < IPC; ++i) {
+            float win[PF_RX + 2 * KM];
 #pragma unroll
-        for (int j = 0; j < PF_R; ++j) acc[j] = 0.f;
+            for (int j = 0; j < PF_RX + 2 * KM; ++j) win[j] = B[(i * NC + c0 + j) * LB + lane];
 #pragma unroll
-        for (int k = -KM; k <= KM; ++k) {
-            const float h = hx[k + KM];
+            for (int j = 0; j < PF_RX; ++j) acc[i][j] = 0.f;
 #pragma unroll
-            for (int j = 0; j < PF_R; ++j) acc[j] = fmaf(h, win[j - k + KM], acc[j]);
+            for (int k = -KM; k <= KM; ++k) {
+                const float h = hx[k + KM];
+#pragma unroll
+                for (int j = 0; j < PF_RX; ++j) acc[i][j] = fmaf(h, win[j - k + KM], acc[i][j]);
+            }
         }
+        if (iz >= nz) continue;
 #pragma unroll
-        for (int j = 0; j < PF_R; ++j) {
+        for (int j = 0; j < PF_RX; ++j) {
             const int ix = ix0 + c0 + j;
             if (ix >= nx) break;
-            const size_t p = (size_t)ix * nz + z;
-            if (out_mode == 2)
-                store_interp_input(out, ((size_t)(w / wt) * nx * nz + p) * wt + w % wt, acc[j],
-                                   fmt, hsc, w);
-            else
-                out[(size_t)w * nx * nz + p] = acc[j];
+            const size_t P = (size_t)nx * nz, p = (size_t)ix * nz + iz;
+            if constexpr (IPC == 4) {
+                // instances past W are the tile's padding
+                *reinterpret_cast<float4 *>(out + ((size_t)(w0 / wt) * P + p) * wt + w0 % wt) =
+                    make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
+            } else if (out_mode == 2) {
+                store_interp_input(out, ((size_t)(w0 / wt) * P + p) * wt + w0 % wt, acc[0][j],
+                                   fmt, hsc, w0);
+            } else {
+                out[(size_t)w0 * P + p] = acc[0][j];
+            }
         }
     }
 }
@@ -1123,36 +1139,46 @@ int launch_prefilter(const Plan &pl, const float *in, float *out, int W, bool tr
     return MSOT_OK;
 }
 
-// both axes in one launch where the staged tile fits shared memory; returns
-// 1 (nothing launched) when the caller must use the per-axis kernels
-template <int KM>
-static int prefilter2d_km(const Plan &pl, const float *in, float *out, int W, bool transpose,
-                          int out_mode, cudaStream_t st) {
-    constexpr int NC = PF_TX + 2 * KM;
-    const size_t smem = (size_t)(2 * NC * (pl.nz | 1) + 2 * (2 * KM + 1)) * sizeof(float);
-    if (smem > 200 * 1024) return 1;
-    MSOT_CUDA_TRY(raise_max_dynamic_smem((const void *)k_prefilter2d<KM>, smem));
-    const dim3 grid((unsigned)((pl.nx + PF_TX - 1) / PF_TX), (unsigned)W);
-    const int wt = out_mode == 2 ? das_fwd_wt(pl, W) : 1;
-    const int fmt = out_mode == 2 ? pl.image_fmt : 0;
-    if (fmt == 2)
-        KLAUNCH(k_h16_scale<<<W, 256, 0, st>>>(in, pl.P, pl.pre_gain_x * pl.pre_gain_z,
-                                               pl.h16_sc, pl.max_batch));
-    KLAUNCH(k_prefilter2d<KM><<<grid, PF_THREADS, smem, st>>>(
+template <int KM, int IPC>
+static int prefilter2d_run(const Plan &pl, const float *in, float *out, int W, bool transpose,
+                           int out_mode, int wt, int fmt, cudaStream_t st) {
+    constexpr int NC = PF_T + 2 * KM;
+    constexpr size_t smem =
+        (size_t)(NC * (NC | 1) + IPC * NC * (PF_T + 1) + 2 * (2 * KM + 1)) * sizeof(float);
+    int rc = set_smem(k_prefilter2d<KM, IPC>, smem);
+    if (rc) return rc;
+    const dim3 grid((unsigned)div_up(pl.nx, PF_T), (unsigned)div_up(pl.nz, PF_T),
+                    (unsigned)div_up(W, IPC));
+    KLAUNCH(k_prefilter2d<KM, IPC><<<grid, PF_THREADS, smem, st>>>(
         in, out, pl.pre_x, pl.pre_z, pl.Kx, pl.Kz, pl.nx, pl.nz, W, transpose ? 1 : 0, out_mode,
         wt, fmt, pl.h16_sc));
     MSOT_LAUNCH_CHECK();
     return MSOT_OK;
 }
 
+template <int KM>
+static int prefilter2d_km(const Plan &pl, const float *in, float *out, int W, bool transpose,
+                          int out_mode, cudaStream_t st) {
+    const int wt = out_mode == 2 ? das_fwd_wt(pl, W) : 1;
+    const int fmt = out_mode == 2 ? pl.image_fmt : 0;
+    if (fmt == 2)
+        KLAUNCH(k_h16_scale<<<W, 256, 0, st>>>(in, pl.P, pl.pre_gain_x * pl.pre_gain_z,
+                                               pl.h16_sc, pl.max_batch));
+    if (out_mode == 2 && fmt == 0 && wt % 4 == 0)
+        return prefilter2d_run<KM, 4>(pl, in, out, W, transpose, out_mode, wt, fmt, st);
+    return prefilter2d_run<KM, 1>(pl, in, out, W, transpose, out_mode, wt, fmt, st);
+}
+
+// both axes in one launch; returns 1 (nothing launched) when the caller must
+// use the per-axis kernels (one axis only, the SIR path's order, wide taps)
 int launch_prefilter2d(const Plan &pl, const float *in, float *out, int W, bool transpose,
                        int out_mode, cudaStream_t st) {
     if (pl.Kx < 0 || pl.Kz < 0 || (out_mode != 0 && out_mode != 2)) return 1;
-    TimedScope ts_(KID_PREFILTER, st);
     const int K = std::max(pl.Kx, pl.Kz);
-    if (K <= 8) return prefilter2d_km<8>(pl, in, out, W, transpose, out_mode, st);
-    if (K <= 16) return prefilter2d_km<16>(pl, in, out, W, transpose, out_mode, st);
-    return 1;
+    if (K > 16 || div_up(pl.nz, PF_T) > 65535) return 1;
+    TimedScope ts_(KID_PREFILTER, st);
+    return K <= 8 ? prefilter2d_km<8>(pl, in, out, W, transpose, out_mode, st)
+                  : prefilter2d_km<16>(pl, in, out, W, transpose, out_mode, st);
 }
 
 int launch_permute(const Plan &pl, const float *in, float *out, int W, cudaStream_t st) {

@@ -133,6 +133,16 @@ struct Plan {
     int2 *sir_se = nullptr;        // [NS] 0-based inclusive start/end
     int32_t *sir_tiles = nullptr;  // [n_patch][D][PATCH] 0-based SIR column
     int32_t *sir_pi = nullptr;     // [D][P] SIR column in scatter order
+    // per (column, piece) the composite rows and per (detector, pixel) the pairs
+    // sorted by window start (forward) / by pixel (adjoint), sir.cu; sir_tab
+    // null: the kernels of operator.cu on the four tables above
+    float2 *sir_tab = nullptr;     // [3 NS][S + 2F + 1]
+    int4 *sir_fent = nullptr;      // [D][P] (row offset, start << 16 | length, f, pixel)
+    int4 *sir_aent = nullptr;      // [ceil(P / 32)][D][32]
+    int2 *sir_aspan = nullptr;     // [ceil(P / 32)][D] samples the block's windows span
+    int sir_span_max = 0;
+    int32_t *sir_off = nullptr;    // [D][sir_nj + 1] forward pairs per window start
+    int sir_jmin = 0, sir_nj = 0, sir_maxlen = 0;
     // scratch for the operator chains
     int max_batch = 0;
     float *scr_img0 = nullptr, *scr_img1 = nullptr;  // [max_batch][P]
@@ -228,6 +238,14 @@ class TimedScope {
         }                                                                              \
     } while (0)
 
+// interpolation with SIR columns (sir.cu)
+int sir_build(Plan &p, const int32_t *tfx, const int32_t *sidx, const std::vector<int2> &se,
+              size_t &bytes);
+int sir_build_table(Plan &p);
+int launch_sir_forward2(const Plan &pl, const float *xpm, float *raw, int W, int wt, float scale,
+                        cudaStream_t st);
+int launch_sir_adjoint2(const Plan &pl, const float *raw, float *x, int W, float scale,
+                        cudaStream_t st);
 // batched DAS forward, lanes over instances (das_fwd_lanes.cu): FP32 input in
 // [ceil(W / wt)][P][wt], wt = 16 or 32
 int launch_das_forward_lanes(const Plan &pl, const float *xpm, float *raw, int W, int wt,
@@ -322,6 +340,7 @@ extern std::atomic<int> g_fwd_staged;
 // instances per CTA of the DAS forward at batch W: the interpolation input is
 // laid out [W/wt][P][wt] (pixel-major within an instance tile).  operator.cu
 int das_fwd_wt(const Plan &pl, int W);
+bool scatter_order(const Plan &pl);  // k_sir_fwd's image order instead; operator.cu
 
 // C (M x N) = alpha A (M x K) B (K x N), column-major FP32, on the tensor
 // cores with a 3 x TF32 split (FP32-level accuracy); gemm_tc.cu

@@ -19,9 +19,11 @@ namespace msot {
 // CTA = (tile of TB = 256 - 2F - 2 output samples, detector, WT instances);
 // the image is [W/WT][P][WT].
 // Phase 1: one bucket per thread reduces the four moments of its pixels,
-// loading FWD_UNR (entry, pixel) pairs at a time; phase 2: each output sample
+// loading FWD_UNR_OF<WT> (entry, pixel) pairs at a time (four at two and four
+// instances: 75 -> 67 us for 4 images of 200 x 200 px; eight for one image ran
+// slower); phase 2: each output sample
 // applies the (2F+2)-tap filter over the bucket moments.
-constexpr int FWD_UNR = 2;
+template <int WT> constexpr int FWD_UNR_OF = WT == 2 || WT == 4 ? 4 : 2;
 
 // one pixel's WT instance values of the interpolation input, FP32 or BF16
 // (widened exactly: a BF16 value is the upper half of its FP32 pattern)
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(256, WT >= 16 ? 2 : 4) k_das_fwd3(const int32_
                                                   const float *__restrict__ inv_s = nullptr,
                                                   const int32_t *__restrict__ ell_off = nullptr,
                                                   const int2 *__restrict__ skip = nullptr) {
-    constexpr int NB = 256;
+    constexpr int NB = 256, FWD_UNR = FWD_UNR_OF<WT>;
     constexpr int TB = NB - 2 * F - 2;
     extern __shared__ float mom[];  // [4][WT][NB], bucket fastest (dynamic: 4 KB x WT)
     const int d = blockIdx.y, w0 = blockIdx.z * WT;
@@ -194,10 +196,16 @@ __global__ void __launch_bounds__(256, WT >= 16 ? 2 : 4) k_das_fwd3(const int32_
             const float step = __int_as_float((127 - fb) << 23);  // 2^-fb
             // the entries of the next group load while this group's gathers
             // are in flight (one dependent latency per group, not two)
+            // (0, -1) past the list's end, where the last entry is loaded again: the
+            // address stays inside the table
+            auto entry = [&](int j) {
+                const int2 q = __ldg(e + (size_t)min(j, j1 - 1) * ES);
+                return j < j1 ? q : make_int2(0, -1);
+            };
             int2 qn[FWD_UNR];
 #pragma unroll
             for (int u = 0; u < FWD_UNR; ++u)
-                qn[u] = j0 + u < j1 ? __ldg(e + (size_t)(j0 + u) * ES) : make_int2(0, -1);
+                qn[u] = entry(j0 + u);
             for (int j = j0; j < j1; j += FWD_UNR) {
                 int2 q[FWD_UNR];
                 float xv[FWD_UNR][WT];
@@ -208,8 +216,7 @@ __global__ void __launch_bounds__(256, WT >= 16 ? 2 : 4) k_das_fwd3(const int32_
                     load_pixel<WT>(xpm + ((size_t)blockIdx.z * P + max(q[u].y, 0)) * WT, xv[u]);
 #pragma unroll
                 for (int u = 0; u < FWD_UNR; ++u)
-                    qn[u] = j + FWD_UNR + u < j1 ? __ldg(e + (size_t)(j + FWD_UNR + u) * ES)
-                                                 : make_int2(0, -1);
+                    qn[u] = entry(j + FWD_UNR + u);
 #pragma unroll
                 for (int u = 0; u < FWD_UNR; ++u) {
                     if (q[u].y < 0) break;

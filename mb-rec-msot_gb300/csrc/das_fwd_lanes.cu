@@ -81,8 +81,10 @@ __global__ void __launch_bounds__(F6_THREADS, 3) k_das_fwd6(
             auto fetch = [&](int c) {
 #pragma unroll
                 for (int k = 0; k < CH / LPG; ++k) {
+                    // the address stays inside the table where the list has ended
                     const int j = c + k * LPG + l;
-                    q[k] = j < n ? __ldg(e + j0 + j) : make_int2(0, -1);
+                    q[k] = __ldg(e + min(j0 + min(j, max(n - 1, 0)), P - 1));
+                    if (j >= n) q[k] = make_int2(0, -1);
                 }
             };
             fetch(0);
@@ -106,7 +108,7 @@ __global__ void __launch_bounds__(F6_THREADS, 3) k_das_fwd6(
                             __shfl_sync(0xffffffffu, pix[(h + k) / LPG], (h + k) % LPG, LPG);
                         f[k] = __shfl_sync(0xffffffffu, fr[(h + k) / LPG], (h + k) % LPG, LPG);
                         v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (p >= 0) v[k] = __ldg(x + (size_t)p * LPG);
+                        if (p >= 0) v[k] = __ldg(x + (size_t)max(p, 0) * LPG);
                     }
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {

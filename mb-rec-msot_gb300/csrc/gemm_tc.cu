@@ -102,8 +102,10 @@ __device__ __forceinline__ void g_load(GRegs<NT> &R, const float *A, int lda, co
         const int n = n0 + (u >> 1) * 8 + (lane & 7);
         const int k = k0 + 4 * ((u & 1) * 4 + (lane >> 3));
         const float *col = B + (size_t)n * ldb + k;
-        if (n < N && bvec && k + 3 < K) {
-            R.b[j] = __ldg(reinterpret_cast<const float4 *>(col));
+        if (bvec && k + 3 < K) {
+            // past N the last column again: those columns of C are not stored
+            R.b[j] = __ldg(reinterpret_cast<const float4 *>(
+                B + (size_t)min(n, N - 1) * ldb + min(k, (K - 1) & ~3)));
         } else {
             float v[4];
 #pragma unroll

@@ -445,7 +445,15 @@ __global__ void k_sum_parts(const float *__restrict__ part, float *__restrict__ 
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (size_t)gridDim.x * blockDim.x) {
         float v = 0.f;
-        for (int g = 0; g < groups; ++g) v += __ldg(part + g * stride + i);
+        for (int g0 = 0; g0 < groups; g0 += 8) {  // eight loads in flight
+            float p[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                p[k] = g0 + k < groups ? __ldg(part + (g0 + k) * stride + i) : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (g0 + k < groups) v += p[k];
+        }
         x[i] = v * scale;
     }
 }
@@ -1231,14 +1239,14 @@ static bool use_staged(const Plan &pl, int wt) {
 // the lanes-over-instances kernel (das_fwd_lanes.cu) serves batches above 8 of
 // the FP32 input unless the autotuner or a knob chose another kernel
 static bool fwd_lanes(const Plan &pl) {
-    return !pl.tune_fwd_staged && g_fwd_ell.load() && !pl.image_fmt;
+    return !pl.tune_fwd_staged && g_fwd_ell.load() && !pl.image_fmt && !pl.S;
 }
 
 // instances per CTA of the DAS forward, the last tile part-filled: the
 // autotuner's pick (16, 8, 4, 2), else 32 or 16 for the lanes kernel, else the
 // next power of two up to 8
 int das_fwd_wt(const Plan &pl, int W) {
-    if (pl.tune_fwd_wt && W % pl.tune_fwd_wt == 0) return pl.tune_fwd_wt;
+    if (pl.tune_fwd_wt && W % pl.tune_fwd_wt == 0 && !pl.S) return pl.tune_fwd_wt;
     if (!fwd_lanes(pl)) {
         int wt = 1;  // a part-filled tile of 8 costs less than W narrow ones
         while (wt < W && wt < 8) wt *= 2;
@@ -1367,6 +1375,8 @@ static int sir_fwd_nt(const Plan &pl, const float *x_pi, float *raw, float scale
 int launch_sir_forward(const Plan &pl, const float *x_pi, float *raw, int W, float scale,
                        cudaStream_t st) {
     TimedScope ts_(KID_INTERP_FWD, st);
+    if (pl.sir_tab)
+        return launch_sir_forward2(pl, x_pi, raw, W, das_fwd_wt(pl, W), scale, st);
     const int wt = pick_wt(W, pl.T, 4);
     const int ns = fwd_split(pl, W / wt);
     if (ns > 1) MSOT_CUDA_TRY(cudaMemsetAsync(raw, 0, sizeof(float) * W * pl.D * pl.T, st));
@@ -1400,6 +1410,9 @@ static int sir_adj_nt(const Plan &pl, const float *raw, float *x, float scale, d
 int launch_sir_adjoint(const Plan &pl, const float *raw, float *x, int W, float scale,
                        cudaStream_t st) {
     TimedScope ts_(KID_INTERP_ADJ, st);
+    // 128 x 128 px: 220 / 356 us here for one / two images against 450 / 460 us with
+    // a half warp per pixel, 591 against 465 for three
+    if (pl.sir_tab && W >= 3) return launch_sir_adjoint2(pl, raw, x, W, scale, st);
     const int wt = pick_wt(W, 1, 2);
     dim3 grid(pl.n_patch, W / wt);
     if (wt == 2) return sir_adj_nt<2>(pl, raw, x, scale, grid, st);
@@ -1494,6 +1507,10 @@ int interp_adjoint(const Plan &pl, const float *raw, float *x, int W, float scal
                 : launch_das_adjoint(pl, raw, x, W, scale, st);
 }
 
+// the image order the interpolation takes: perm[] (k_sir_fwd) or pixel-major
+// tiles of das_fwd_wt instances
+bool scatter_order(const Plan &pl) { return pl.S && !pl.sir_tab; }
+
 static int forward_to_raw(const Plan &pl, const float *img, int W, cudaStream_t st);
 
 int apply_forward(const Plan &pl, const float *img, float *sino, int W, cudaStream_t st) {
@@ -1503,7 +1520,7 @@ int apply_forward(const Plan &pl, const float *img, float *sino, int W, cudaStre
         return launch_conv(pl, pl.scr_sino, sino, W, false, st);
     }
     float *xpi = pl.scr_img1;
-    const int mode = pl.S ? 1 : 2;  // scatter order (SIR) or pixel-major (bucket moments)
+    const int mode = scatter_order(pl) ? 1 : 2;
     if ((rc = launch_prefilter2d(pl, img, xpi, W, false, mode, st)) <= 0) {
         if (rc) return rc;
     } else if (pl.Kz >= 0 && pl.Kx >= 0) {
@@ -1515,7 +1532,7 @@ int apply_forward(const Plan &pl, const float *img, float *sino, int W, cudaStre
         if ((rc = launch_prefilter(pl, img, xpi, W, false, false, 1.f, mode, st))) return rc;
     } else if (pl.Kx >= 0) {
         if ((rc = launch_prefilter(pl, img, xpi, W, false, true, 1.f, mode, st))) return rc;
-    } else if (pl.S) {
+    } else if (scatter_order(pl)) {
         if ((rc = launch_permute(pl, img, xpi, W, st))) return rc;
     } else {
         if ((rc = launch_to_pixmajor(pl, img, xpi, W, st))) return rc;
@@ -1528,7 +1545,7 @@ int apply_forward(const Plan &pl, const float *img, float *sino, int W, cudaStre
 static int forward_to_raw(const Plan &pl, const float *img, int W, cudaStream_t st) {
     int rc;
     float *xpi = pl.scr_img1;
-    const int mode = pl.S ? 1 : 2;
+    const int mode = scatter_order(pl) ? 1 : 2;
     if ((rc = launch_prefilter2d(pl, img, xpi, W, false, mode, st)) <= 0) {
         if (rc) return rc;
     } else if (pl.Kz >= 0 && pl.Kx >= 0) {
@@ -1540,7 +1557,7 @@ static int forward_to_raw(const Plan &pl, const float *img, int W, cudaStream_t 
         if ((rc = launch_prefilter(pl, img, xpi, W, false, false, 1.f, mode, st))) return rc;
     } else if (pl.Kx >= 0) {
         if ((rc = launch_prefilter(pl, img, xpi, W, false, true, 1.f, mode, st))) return rc;
-    } else if (pl.S) {
+    } else if (scatter_order(pl)) {
         if ((rc = launch_permute(pl, img, xpi, W, st))) return rc;
     } else {
         if ((rc = launch_to_pixmajor(pl, img, xpi, W, st))) return rc;
@@ -1738,7 +1755,7 @@ int msot_interp_forward(msot_plan_t plan, const float *d_coeffs, float *d_raw, i
     int rc = check_batch(plan, batch, d_coeffs, d_raw);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    if (plan->p.S) {
+    if (scatter_order(plan->p)) {
         if ((rc = launch_permute(plan->p, d_coeffs, plan->p.scr_img1, batch, st))) return rc;
     } else {
         if ((rc = launch_to_pixmajor(plan->p, d_coeffs, plan->p.scr_img1, batch, st))) return rc;

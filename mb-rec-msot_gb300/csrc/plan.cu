@@ -98,7 +98,8 @@ static void free_plan(Plan &p) {
                     p.scr_sino, p.fwd_off, p.fwd_ent, p.blk_tau, p.blk_span,
                     p.scr_part, p.fft_tw, p.fft_hf, p.fft_ha, p.fft_twb, p.fft_twn,
                     p.fft_hfb, p.fft_hab, p.st_info, p.st_u, p.st_off, p.st_ent,
-                    p.adj5_span, p.adj5_ent, p.h16_sc, p.fwd_ell, p.fwd_ell_off, p.conv_rng};
+                    p.adj5_span, p.adj5_ent, p.sir_tab, p.sir_fent,
+                    p.sir_aent, p.sir_aspan, p.sir_off, p.h16_sc, p.fwd_ell, p.fwd_ell_off, p.conv_rng};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     p = Plan();
@@ -362,6 +363,12 @@ static int build(const msot_plan_desc *d, Plan &p) {
         sirf.resize((size_t)p.NS * p.S);
         for (size_t i = 0; i < sirf.size(); ++i) sirf[i] = (float)d->sir[i];
         (void)maxlen;
+        const int rc = sir_build(p, tfx.data(), d->sir_idx, se, p.device_bytes);
+        if (rc != MSOT_OK) return rc;
+        if (p.sir_tab) {  // k_sir_fwd's tables stay behind (k_sir_adj serves 1 and 2 images)
+            tpi.clear();
+            spi.clear();
+        }
     }
 
     // --- IR, prefilter, normalisation ----------------------------------------------
@@ -486,6 +493,7 @@ static int build(const msot_plan_desc *d, Plan &p) {
     if (has_sir) {
         UP(p.sir, sirf);
         UP(p.sir_se, se);
+        if (p.sir_tab && (rc = sir_build_table(p)) != MSOT_OK) return rc;
         UP(p.sir_tiles, stiles);
         UP(p.sir_pi, spi);
     }
@@ -533,14 +541,16 @@ static int build(const msot_plan_desc *d, Plan &p) {
         for (float t : pz) g += std::fabs((double)t);
         p.pre_gain_z = (float)g;
     }
-    if (!has_sir) {
+    if (!has_sir || p.sir_tab) {
         // detector groups of the adjoint: enough CTAs to fill the GPU twice,
         // at most 512 partial images in flight
         p.adj_groups_max = std::max(1, std::min(p.D, (int)std::min<size_t>(32, 512 / W)));
         if ((rc = alloc(&p.scr_part, (size_t)p.adj_groups_max * W * p.P, B)) != MSOT_OK)
             return rc;
     }
-
+    // the kernels and fills above run on the default stream: done before the plan
+    // is used on another stream or destroyed again
+    MSOT_CUDA_TRY(cudaStreamSynchronize(nullptr));
     return MSOT_OK;
 }
 

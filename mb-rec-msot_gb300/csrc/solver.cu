@@ -161,7 +161,7 @@ __global__ void k_l2_v_img(const float *__restrict__ atu, const float *__restric
                            const float *__restrict__ lul, double sr2) {
     float acc = 0.f;
     const Scal &q = sc[grp(blockIdx.y, coupled)];
-    const bool done = q.done;
+    const bool done = q.done || q.improved == 3;  // marked by the scalar kernel after this one
     const float ib = (float)(1.0 / q.beta), be = (float)q.beta;
     const float c_l = (float)sl, c_r = (float)(sl * sr), c_b = (float)sb;
     const float c_l2 = (float)(sl * sr2);
@@ -251,10 +251,12 @@ __global__ void k_l2_scalar(Scal *sc, int stage, const double *p1, int n1, const
         } else if (stage == 1) {
             const double a2 = group_sum(p1, n1, nullptr, 0, g, W, coupled);
             LANE0_ONLY;
+            if (q.improved == 3) q.done = 1;  // converged in the step before: x is final
             if (!q.done) {
                 q.alpha = sqrt(a2);
                 if (!(q.alpha > 0.0) || !isfinite(q.alpha)) q.done = 1;
             }
+            q.gamma = q.alpha / q.beta;  // for the next u update
         } else {
             const double b2 = group_sum(p1, n1, p2, n2, g, W, coupled);
             LANE0_ONLY;
@@ -286,11 +288,6 @@ __global__ void k_l2_scalar(Scal *sc, int stage, const double *p1, int n1, const
     }
 }
 
-// gamma = alpha / beta for the next u update
-__global__ void k_l2_gamma(Scal *sc, int G) {
-    for (int g = threadIdx.x; g < G; g += blockDim.x) sc[g].gamma = sc[g].alpha / sc[g].beta;
-}
-
 // v /= alpha ; on init also d = 0, x = w, xmin = w
 __global__ void k_l2_scale_v(float *v, float *d, float *x, float *xmin, const float *wv,
                              size_t N, int init, const Scal *sc, int coupled) {
@@ -319,11 +316,6 @@ __global__ void k_l2_dx(const float *v, float *d, float *x, float *xmin, size_t 
         x[k] = xn;
         if (q.improved != 2) xmin[k] = xn;
     }
-}
-
-__global__ void k_l2_mark_converged(Scal *sc, int G) {
-    for (int g = threadIdx.x; g < G; g += blockDim.x)
-        if (sc[g].improved == 3) sc[g].done = 1;
 }
 
 // w = max(xmin - vm, 0) ; vm += w - xmin
@@ -408,6 +400,15 @@ static int make_work(const Plan &pl, int W, Work &wk) {
     return MSOT_OK;
 }
 
+// A second stream for the image-side vector kernels of an LSQR step, which
+// depend on nothing the operator launches between fork() and join() write: at
+// one image of 128 x 128 px each of them costs as long as a third of an
+// operator kernel.  Null stream: everything stays on st.
+struct SideStream {
+    cudaStream_t s = nullptr;
+    cudaEvent_t out = nullptr, back = nullptr;
+};
+
 struct Ctx {
     const Plan &pl;
     int W;
@@ -416,7 +417,23 @@ struct Ctx {
     size_t NS, NI;
     int nbs, nbi;
     Work &wk;
+    const SideStream *side = nullptr;
     double *P(int slot) const { return wk.part + (size_t)slot * W * 256; }
+    // a stream ordered after the work on st so far; join() orders st after it
+    int fork(cudaStream_t &s) const {
+        s = st;
+        if (!side || !side->s) return MSOT_OK;
+        MSOT_CUDA_TRY(cudaEventRecord(side->out, st));
+        MSOT_CUDA_TRY(cudaStreamWaitEvent(side->s, side->out, 0));
+        s = side->s;
+        return MSOT_OK;
+    }
+    int join() const {
+        if (!side || !side->s) return MSOT_OK;
+        MSOT_CUDA_TRY(cudaEventRecord(side->back, side->s));
+        MSOT_CUDA_TRY(cudaStreamWaitEvent(st, side->back, 0));
+        return MSOT_OK;
+    }
 };
 
 #define TRY(x)                                                                             \
@@ -453,14 +470,19 @@ static int l2_outer(const Ctx &c, const float *b, float *wv, float *vm, double s
     const int nx = c.pl.nx, nz = c.pl.nz;
     const size_t ns = c.NS / c.W, ni = c.NI / c.W;
     const dim3 gs(c.nbs, c.W), gi(c.nbi, c.W);
-    const int G = c.coupled ? 1 : c.W;
     cudaStream_t st = c.st;
     // The sinogram part of u is updated inside the forward operator's
     // convolution where the plan allows it (no A v round trip through HBM);
     // nps = partial sums per instance that the update leaves in P(0).
     const bool fuse = forward_update_fusable(c.pl, c.W);
     int nps = c.nbs;
+    cudaStream_t s2 = st;
     // init: u = b_aug - A_aug w
+    TRY(c.fork(s2));
+    if (lap) KLAUNCH(k_del2<<<gi, RED_THREADS, 0, s2>>>(wv, tl, nx, nz));
+    KLAUNCH(k_l2_init_img<<<gi, RED_THREADS, 0, s2>>>(wv, vm, ur, ub, ni, sl, sr, sb, has_reg, c.P(1),
+                                              c.P(2), tl, ul, sr2));
+    MSOT_LAUNCH_CHECK();
     if (fuse) {
         TRY(apply_forward_update(c.pl, wv, us, b, c.W, 0, (float)sl, k.sc, c.coupled, c.P(0),
                                  &nps, st));
@@ -469,9 +491,7 @@ static int l2_outer(const Ctx &c, const float *b, float *wv, float *vm, double s
         KLAUNCH(k_sino_update<<<gs, RED_THREADS, 0, st>>>(tmp_s, b, us, ns, 0, sl, k.sc,
                                                           c.coupled, c.P(0)));
     }
-    if (lap) KLAUNCH(k_del2<<<gi, RED_THREADS, 0, st>>>(wv, tl, nx, nz));
-    KLAUNCH(k_l2_init_img<<<gi, RED_THREADS, 0, st>>>(wv, vm, ur, ub, ni, sl, sr, sb, has_reg, c.P(1),
-                                              c.P(2), tl, ul, sr2));
+    TRY(c.join());
     KLAUNCH(k_l2_scalar<<<1, 1024, 0, st>>>(k.sc, 0, c.P(0), nps, c.P(1), c.nbi, c.P(2), c.nbi, normb2,
                                    sl, sb, c.W, c.coupled, 1e-8));
     MSOT_LAUNCH_CHECK();
@@ -485,7 +505,11 @@ static int l2_outer(const Ctx &c, const float *b, float *wv, float *vm, double s
     KLAUNCH(k_l2_scale_v<<<gi, RED_THREADS, 0, st>>>(v, d, x, xmin, wv, ni, 1, k.sc, c.coupled));
     MSOT_LAUNCH_CHECK();
     for (int it = 0; it < 2; ++it) {
-        KLAUNCH(k_l2_gamma<<<1, 256, 0, st>>>(k.sc, G));
+        TRY(c.fork(s2));
+        if (lap) KLAUNCH(k_del2<<<gi, RED_THREADS, 0, s2>>>(v, tl, nx, nz));
+        KLAUNCH(k_l2_u_img<<<gi, RED_THREADS, 0, s2>>>(v, ur, ub, ni, sl, sr, sb, has_reg, k.sc,
+                                               c.coupled, c.P(1), tl, ul, sr2));
+        MSOT_LAUNCH_CHECK();
         if (fuse) {
             TRY(apply_forward_update(c.pl, v, us, nullptr, c.W, 1, (float)sl, k.sc, c.coupled,
                                      c.P(0), &nps, st));
@@ -494,16 +518,17 @@ static int l2_outer(const Ctx &c, const float *b, float *wv, float *vm, double s
             KLAUNCH(k_sino_update<<<gs, RED_THREADS, 0, st>>>(tmp_s, nullptr, us, ns, 1, sl, k.sc,
                                                               c.coupled, c.P(0)));
         }
-        if (lap) KLAUNCH(k_del2<<<gi, RED_THREADS, 0, st>>>(v, tl, nx, nz));
-        KLAUNCH(k_l2_u_img<<<gi, RED_THREADS, 0, st>>>(v, ur, ub, ni, sl, sr, sb, has_reg, k.sc,
-                                               c.coupled, c.P(1), tl, ul, sr2));
+        TRY(c.join());
         KLAUNCH(k_l2_scalar<<<1, 1024, 0, st>>>(k.sc, 2, c.P(0), nps, c.P(1), c.nbi, nullptr, 0,
                                        nullptr, sl, sb, c.W, c.coupled, 1e-8));
-        KLAUNCH(k_l2_dx<<<gi, RED_THREADS, 0, st>>>(v, d, x, xmin, ni, k.sc, c.coupled));
-        KLAUNCH(k_l2_mark_converged<<<1, 256, 0, st>>>(k.sc, G));
+        // the last A^T of lsqr only feeds its stopping test
+        if (it == 0) TRY(c.fork(s2));
+        KLAUNCH(k_l2_dx<<<gi, RED_THREADS, 0, it == 0 ? s2 : st>>>(v, d, x, xmin, ni, k.sc,
+                                                                   c.coupled));
         MSOT_LAUNCH_CHECK();
-        if (it == 1) break;  // the last A^T of lsqr only feeds its stopping test
+        if (it == 1) break;
         TRY(apply_transpose(c.pl, us, tmp_i, c.W, st));
+        TRY(c.join());
         if (lap) KLAUNCH(k_del2<<<gi, RED_THREADS, 0, st>>>(ul, tl, nx, nz));
         KLAUNCH(k_l2_v_img<<<gi, RED_THREADS, 0, st>>>(tmp_i, ur, ub, v, ni, sl, sr, sb, has_reg, 0,
                                                k.sc, c.coupled, c.P(1), tl, sr2));
@@ -525,6 +550,7 @@ struct SolverCache {
     Work wk;
     cudaStream_t stream = nullptr;  // non-blocking stream the graphs are captured on
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
+    SideStream side;
     cudaGraphExec_t l2_exec = nullptr;
     int l2_W = -1, l2_has_reg = -1, l2_coupled = -1;
     double l2_sr = -1.0, l2_sr2 = -1.0;
@@ -538,7 +564,10 @@ static SolverCache *cache_for(Plan &pl, int W, int &rc) {
     if (!sc->stream) {
         if (cudaStreamCreateWithFlags(&sc->stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&sc->ev_in, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&sc->ev_out, cudaEventDisableTiming) != cudaSuccess) {
+            cudaEventCreateWithFlags(&sc->ev_out, cudaEventDisableTiming) != cudaSuccess ||
+            cudaStreamCreateWithFlags(&sc->side.s, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&sc->side.out, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&sc->side.back, cudaEventDisableTiming) != cudaSuccess) {
             set_error("solver: stream creation failed");
             rc = MSOT_ECUDA;
             return sc;
@@ -567,6 +596,9 @@ void solver_cache_free(Plan &pl) {
     if (pl.solver->stream) cudaStreamDestroy(pl.solver->stream);
     if (pl.solver->ev_in) cudaEventDestroy(pl.solver->ev_in);
     if (pl.solver->ev_out) cudaEventDestroy(pl.solver->ev_out);
+    if (pl.solver->side.s) cudaStreamDestroy(pl.solver->side.s);
+    if (pl.solver->side.out) cudaEventDestroy(pl.solver->side.out);
+    if (pl.solver->side.back) cudaEventDestroy(pl.solver->side.back);
     free_work(pl.solver->wk);
     delete pl.solver;
     pl.solver = nullptr;
@@ -599,7 +631,7 @@ static int solve_l2(Plan &pl, const float *b_in, float *rec, int W, int num_iter
     MSOT_CUDA_TRY(cudaStreamWaitEvent(st, sc->ev_in, 0));
     Work &wk = sc->wk;
     const size_t NS = (size_t)W * pl.D * pl.T, NI = (size_t)W * pl.P;
-    Ctx c{pl, W, coupled, st, NS, NI, nblk_for(NS / W), nblk_for(NI / W), wk};
+    Ctx c{pl, W, coupled, st, NS, NI, nblk_for(NS / W), nblk_for(NI / W), wk, &sc->side};
     const int has_reg = lambdaL2 > 0;
     const double sr = has_reg ? std::sqrt(lambdaL2) : 0.0;
     // incorporate_l2_reg_into_model_functions.m:8-18: the second term only

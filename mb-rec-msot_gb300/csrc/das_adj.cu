@@ -10,12 +10,12 @@
 // neighbouring rows: acc += (1 - g) K[j] + g K[j + 1].
 //
 // The lanes of a pixel hold NI instances, four each, so a row read is
-// NI x 4 contiguous bytes: random rows of 8 pixels cost 6 shared wavefronts
-// per 128-bit load at NI = 16, where the table with one or two instances per
+// NI x 4 contiguous bytes: a 128-bit load of a warp takes 4 shared wavefronts
+// at NI = 32 and 6 at NI = 16 (two random rows per 8 lanes), where the table with one or two instances per
 // thread (k_das_adj4: lanes over pixels, random 16-byte rows) paid about 10 for
 // a quarter of the values.  (pixel, detector) pairs come as 4 bytes, knot row
 // and g in fixed point, decoded once per 4 NI values.  Measured at batch 64,
-// 128 x 128 px, 256 detectors: 322 us (k_das_adj4) -> 269 us.
+// 128 x 128 px, 256 detectors: 322 us (k_das_adj4) -> 211 us (NI = 32).
 //
 // Bound: shared-memory wavefronts of the row reads, then the issue slots of
 // the decode and of the knot table (U and V run along the samples: 12
@@ -27,8 +27,11 @@
 
 namespace msot {
 
-constexpr int A5_THREADS = 256, A5_SIDE = 32, A5_PIX = A5_SIDE * A5_SIDE;
-constexpr int A5_PAD = 1;  // seg rows of NI + 1 words: staging stores along t are conflict-free
+constexpr int A5_SIDE = 32, A5_PIX = A5_SIDE * A5_SIDE;
+template <int NI> constexpr int a5_threads = NI == 32 ? 512 : 256;
+// seg rows of NI + 2 words: even, for the knots' 8-byte loads, and staging
+// stores along t meet each bank twice only
+constexpr int A5_PAD = 2;
 
 struct Adj5Const {
     float inv_r, ce1;       // 1 / r, (r - F) / r
@@ -107,16 +110,17 @@ __global__ void __launch_bounds__(256) k_adj5_entries(const int32_t *__restrict_
 // Grid (sub-block, instance tile, detector group); instances w0 + 0 .. NI - 1,
 // those past W read as zero and are not stored.
 template <int NI, int F>
-__global__ void __launch_bounds__(A5_THREADS, 2) k_das_adj5(
+__global__ void __launch_bounds__(a5_threads<NI>, NI == 32 ? 1 : 2) k_das_adj5(
     const uint32_t *__restrict__ ent, const int2 *__restrict__ bspan,
     const float *__restrict__ s, float *__restrict__ part, int nx, int nz, int nbx, int D,
     int T, int W, Adj5Const cst, int seg_rows, int knot_rows, int det_per_group,
     size_t part_stride) {
+    constexpr int A5_THREADS = a5_threads<NI>;
     constexpr int LPG = NI / 4;                  // lanes per pixel
     constexpr int NG = A5_THREADS / LPG;         // pixels in flight
     constexpr int PPG = A5_PIX / NG;             // pixels per lane group
     constexpr int RS = NI + A5_PAD;              // words per seg row
-    constexpr int NRUN = A5_THREADS / NI;        // runs of the knot table
+    constexpr int NP = NI / 2, NRUN = A5_THREADS / NP;  // runs of the knot table
     extern __shared__ __align__(16) float a5_smem[];
     float *K = a5_smem;                          // [knot_rows][NI]
     float *seg0 = K + (size_t)knot_rows * NI;    // [2][seg_rows][RS]
@@ -134,8 +138,16 @@ __global__ void __launch_bounds__(A5_THREADS, 2) k_das_adj5(
         const int n = sp.y - sp.x + 1 + 2 * F + 3;
         if (sp.y < sp.x) return;
         float *seg = seg0 + (size_t)buf * seg_rows * RS;
+        const bool inside = sp.x - F >= 0 && sp.x - F + n <= T && w0 + NI <= W;
         for (int w = warp; w < NI; w += A5_THREADS / 32) {
             const float *src = s + ((size_t)min(w0 + w, W - 1) * D + d) * T;
+            if (inside) {
+                uint32_t dst = smem_u32(seg + lane * RS + w);
+                src += sp.x - F + lane;
+                for (int k = lane; k < n; k += 32, src += 32, dst += 32 * RS * 4)
+                    cp_async4(dst, src);
+                continue;
+            }
             const bool in = w0 + w < W;
             for (int k = lane; k < n; k += 32) {
                 const int tt = sp.x - F + k;
@@ -148,7 +160,7 @@ __global__ void __launch_bounds__(A5_THREADS, 2) k_das_adj5(
         }
     };
     if (d_begin < d_end) stage(d_begin, 0);
-    const int run = t / NI, inst = t % NI;
+    const int run = t / NP, inst = t % NP * 2;
     const int grp_px = t / LPG, l4 = (t % LPG) * 4;
     for (int d = d_begin; d < d_end; ++d) {
         const int buf = (d - d_begin) & 1;
@@ -166,29 +178,34 @@ __global__ void __launch_bounds__(A5_THREADS, 2) k_das_adj5(
             const int b0 = run * per, b1 = min(nb + 1, b0 + per);
             const float *g = seg0 + (size_t)buf * seg_rows * RS + inst + (size_t)(b0 + F) * RS;
             if (b0 < b1) {
-                float U = 0.f, V0 = 0.f, V1 = 0.f;
+                // two instances side by side in packed arithmetic
+                auto ld = [&](int k) { return *reinterpret_cast<const float2 *>(g + k * RS); };
+                auto two = [](float v) { return make_float2(v, v); };
+                const float2 m1 = two(-1.f);
+                float2 U = two(0.f), V0 = U, V1 = U;
 #pragma unroll
                 for (int k = F - 1; k >= 0; --k) {
-                    const float v = g[-k * RS];
-                    U = fmaf(1.f - (float)k * cst.inv_r, v, U);
-                    V0 += v;
+                    const float2 v = ld(-k);
+                    U = ffma2(two(1.f - (float)k * cst.inv_r), v, U);
+                    V0 = fadd2(V0, v);
                 }
 #pragma unroll
                 for (int k = F; k >= 1; --k) {
-                    const float v = g[k * RS];
-                    U = fmaf(1.f - (float)k * cst.inv_r, v, U);
-                    V1 += v;
+                    const float2 v = ld(k);
+                    U = ffma2(two(1.f - (float)k * cst.inv_r), v, U);
+                    V1 = fadd2(V1, v);
                 }
-                float V = V1 - V0, sl = g[-F * RS];
+                float2 V = ffma2(V0, m1, V1), sl = ld(-F);
                 float *row = K + (size_t)3 * b0 * NI + inst;
                 for (int b = b0; b < b1; ++b) {
-                    const float sh = g[(F + 1) * RS], s1 = g[RS], sn = g[(1 - F) * RS];
-                    row[0] = fmaf(cst.ce1, sl, U);
-                    row[NI] = fmaf(cst.q1, V, fmaf(cst.cl, sl, U));
-                    row[2 * NI] = fmaf(cst.q2, V, fmaf(cst.ch, sh, U));
+                    const float2 sh = ld(F + 1), s1 = ld(1), sn = ld(1 - F);
+                    float2 *o = reinterpret_cast<float2 *>(row);
+                    o[0] = ffma2(two(cst.ce1), sl, U);
+                    o[NP] = ffma2(two(cst.q1), V, ffma2(two(cst.cl), sl, U));
+                    o[2 * NP] = ffma2(two(cst.q2), V, ffma2(two(cst.ch), sh, U));
                     row += 3 * NI;
-                    U = fmaf(cst.ce1, sh - sn, fmaf(V, cst.inv_r, U));
-                    V += (sh - s1) + (sn - s1);
+                    U = ffma2(two(cst.ce1), ffma2(sn, m1, sh), ffma2(V, two(cst.inv_r), U));
+                    V = fadd2(V, fadd2(ffma2(s1, m1, sh), ffma2(s1, m1, sn)));
                     sl = sn;
                     g += RS;
                 }
@@ -279,7 +296,7 @@ static int adj5_launch(const Plan &pl, const float *raw, float *part, int W, int
     int rc = set_smem(k_das_adj5<NI, F>, smem);
     if (rc) return rc;
     const dim3 grid(4 * pl.n_blk, div_up(W, NI), groups);
-    KLAUNCH(k_das_adj5<NI, F><<<grid, A5_THREADS, smem, st>>>(
+    KLAUNCH(k_das_adj5<NI, F><<<grid, a5_threads<NI>, smem, st>>>(
         pl.adj5_ent, pl.adj5_span, raw, part, pl.nx, pl.nz, pl.n_blk_x, pl.D, pl.T, W,
         adj5_const(pl), pl.adj5_span_max + 2 * pl.F + 3, 3 * pl.adj5_span_max + 4, dpg, stride));
     MSOT_LAUNCH_CHECK();
@@ -303,10 +320,10 @@ static int adj5_f(const Plan &pl, const float *raw, float *part, int W, int grou
 }
 
 // instances per tile: the widest that W fills to more than half and whose
-// tables leave two CTAs per SM; 0: none does
+// tables leave two CTAs per SM (one of twice the threads at 32); 0: none does
 static int adj5_ni(const Plan &pl, int W) {
-    int ni = W > 8 ? 16 : 8;
-    while (ni >= 8 && adj5_smem(pl, ni) > 110 * 1024) ni /= 2;
+    int ni = W > 16 && (W + 31) / 32 * 32 - W < 16 ? 32 : W > 8 ? 16 : 8;
+    while (ni >= 8 && adj5_smem(pl, ni) > (ni == 32 ? 222 : 110) * 1024) ni /= 2;
     return ni >= 8 ? ni : 0;
 }
 
@@ -321,7 +338,7 @@ int launch_das_adjoint5(const Plan &pl, const float *raw, float *x, int W, float
     const int ni = adj5_ni(pl, W);
     // detector groups: the fewest that come close to filling whole waves of two
     // CTAs per SM (each group writes a partial image)
-    const int base = 4 * pl.n_blk * div_up(W, ni), slots = 2 * sm_count();
+    const int base = 4 * pl.n_blk * div_up(W, ni), slots = (ni == 32 ? 1 : 2) * sm_count();
     const int most = std::max(1, std::min({pl.adj_groups_max * pl.max_batch / W, pl.D, 32}));
     int groups = 1;
     double best = 0.0;
@@ -333,7 +350,8 @@ int launch_das_adjoint5(const Plan &pl, const float *raw, float *x, int W, float
     const int dpg = div_up(pl.D, groups);
     groups = div_up(pl.D, dpg);
     const size_t stride = (size_t)W * pl.P;
-    const int rc = ni == 16 ? adj5_f<16>(pl, raw, pl.scr_part, W, groups, dpg, stride, st)
+    const int rc = ni == 32   ? adj5_f<32>(pl, raw, pl.scr_part, W, groups, dpg, stride, st)
+                   : ni == 16 ? adj5_f<16>(pl, raw, pl.scr_part, W, groups, dpg, stride, st)
                             : adj5_f<8>(pl, raw, pl.scr_part, W, groups, dpg, stride, st);
     if (rc) return rc;
     return sum_parts(pl.scr_part, x, stride, groups, scale, st);

@@ -543,8 +543,8 @@ static int build(const msot_plan_desc *d, Plan &p) {
     }
     if (!has_sir || p.sir_tab) {
         // detector groups of the adjoint: enough CTAs to fill the GPU twice,
-        // at most 512 partial images in flight
-        p.adj_groups_max = std::max(1, std::min(p.D, (int)std::min<size_t>(32, 512 / W)));
+        // at most 640 partial images in flight
+        p.adj_groups_max = std::max(1, std::min(p.D, (int)std::min<size_t>(32, 640 / W)));
         if ((rc = alloc(&p.scr_part, (size_t)p.adj_groups_max * W * p.P, B)) != MSOT_OK)
             return rc;
     }

@@ -25,13 +25,17 @@ template <int NI> constexpr int f6_dg = 64 / NI;                    // detectors
 template <int NI> constexpr int f6_row = f6_dg<NI> * F6_NB + 32 / NI;  // conflict-free stores
 
 template <int NI, int F>
-__global__ void __launch_bounds__(F6_THREADS, 3) k_das_fwd6(
+__global__ void __launch_bounds__(F6_THREADS, F <= 2 ? 2 : 3) k_das_fwd6(
     const int32_t *__restrict__ off, const int2 *__restrict__ ent,
     const float *__restrict__ xpm, float *__restrict__ raw, int P, int D, int T, int W, int fb,
     float inv_r, float ce1, float ce2, float scale, const int2 *__restrict__ skip) {
     constexpr int LPG = NI / 4, NG = F6_THREADS / LPG, DG = f6_dg<NI>, ROW = f6_row<NI>;
     constexpr int PER = NG / DG;  // buckets of a detector in flight: 16
-    constexpr int TB = F6_NB - 2 * F - 2, CH = 8;
+    // Pixels in flight per lane group.  Coarse radii (F <= 2, long lists) take
+    // eight at two CTAs per SM, which leaves more of L1 to the pixels: 13 images
+    // of 400 x 400 px, 512 detectors 962 -> 601 us; lists of a dozen entries
+    // lose to the padding (64 images of 128 x 128 px 208 -> 233 us with eight).
+    constexpr int TB = F6_NB - 2 * F - 2, CH = 8, BT = F <= 2 ? 8 : 4;
     extern __shared__ float mom[];  // [4][NI][ROW], bucket fastest
     const int d0 = blockIdx.y * DG, w0 = blockIdx.z * NI;
     const int t0 = blockIdx.x * TB, b_lo = t0 - F - 1;
@@ -98,12 +102,12 @@ __global__ void __launch_bounds__(F6_THREADS, 3) k_das_fwd6(
                 }
                 if (c + CH < most) fetch(c + CH);
 #pragma unroll
-                for (int h = 0; h < CH; h += 4) {
+                for (int h = 0; h < CH; h += BT) {
                     if (c + h >= most) break;  // uniform in the warp
-                    float4 v[4];
-                    float f[4];
+                    float4 v[BT];
+                    float f[BT];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
+                    for (int k = 0; k < BT; ++k) {
                         const int p =
                             __shfl_sync(0xffffffffu, pix[(h + k) / LPG], (h + k) % LPG, LPG);
                         f[k] = __shfl_sync(0xffffffffu, fr[(h + k) / LPG], (h + k) % LPG, LPG);
@@ -111,7 +115,7 @@ __global__ void __launch_bounds__(F6_THREADS, 3) k_das_fwd6(
                         if (p >= 0) v[k] = __ldg(x + (size_t)max(p, 0) * LPG);
                     }
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
+                    for (int k = 0; k < BT; ++k) {
                         const float e1 = fmaxf(0.f, fmaf(-f[k], inv_r, ce1));
                         const float e2 = fmaxf(0.f, fmaf(f[k], inv_r, -ce2));
                         const float2 a = make_float2(v[k].x, v[k].y),

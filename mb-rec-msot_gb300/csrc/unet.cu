@@ -87,20 +87,76 @@ __global__ void __launch_bounds__(256) k_conv3(const float *__restrict__ in, int
     }
 }
 
+// The network's first layer (forward, CI = 1 or 2 input channels): a thread per
+// pixel keeps its CI x 9 inputs in registers and runs over 32 output channels,
+// four weights per shared-memory load, so that the stores (the layer's output
+// is 32 times its input) bound it.  The same sums in the same order as k_conv3,
+// which stages eight input channels whatever Ci is.  64 images,
+// 128^2 px, 32 outputs: 35 us (k_conv3: 212).
+template <int CI>
+__global__ void __launch_bounds__(256) k_conv3_in(const float *__restrict__ in,
+                                                  const __nv_bfloat16 *__restrict__ w,
+                                                  const float *__restrict__ bias,
+                                                  float *__restrict__ out, int Co, int H, int Wd,
+                                                  int relu) {
+    __shared__ __align__(16) float s_w[CI * 9][32];
+    const int co0 = blockIdx.y * 32, n = blockIdx.z;
+    for (int i = threadIdx.x; i < CI * 9 * 32; i += 256) {
+        const int o = i % 32, ck = i / 32;
+        s_w[ck][o] =
+            co0 + o < Co ? __bfloat162float(w[(size_t)(co0 + o) * CI * 9 + ck]) : 0.f;
+    }
+    __syncthreads();
+    const int p = blockIdx.x * 256 + threadIdx.x, HW = H * Wd;
+    if (p >= HW) return;
+    const int y = p / Wd, x = p % Wd;
+    float v[CI * 9];
+#pragma unroll
+    for (int c = 0; c < CI; ++c)
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const int yy = y + k / 3 - 1, xx = x + k % 3 - 1;
+            v[c * 9 + k] = yy >= 0 && yy < H && xx >= 0 && xx < Wd
+                               ? in[((size_t)n * CI + c) * HW + yy * Wd + xx]
+                               : 0.f;
+        }
+    float *po = out + ((size_t)n * Co + co0) * HW + p;
+    for (int o = 0; o < 32 && co0 + o < Co; o += 4) {
+        float a[4] = {};
+#pragma unroll
+        for (int ck = 0; ck < CI * 9; ++ck) {
+            const float4 q = *reinterpret_cast<const float4 *>(&s_w[ck][o]);
+            a[0] = fmaf(q.x, v[ck], a[0]);
+            a[1] = fmaf(q.y, v[ck], a[1]);
+            a[2] = fmaf(q.z, v[ck], a[2]);
+            a[3] = fmaf(q.w, v[ck], a[3]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (co0 + o + j >= Co) break;
+            float r = a[j] + (bias ? bias[co0 + o + j] : 0.f);
+            if (relu) r = fmaxf(r, 0.f);
+            po[(size_t)(o + j) * HW] = r;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Tensor-core 3x3 convolution (tcgen05.mma kind::tf32, accumulator in TMEM).
 //
-// Implicit GEMM per CTA: D[m][o] (m = pixel of an 8 x 16 tile, o = NT output
-// channels) += sum over taps k and input channels i of A_k[m][i] B_k[i][o],
-// A_k the input shifted by tap k, B_k[i][o] = w(o, i, k).  Input channels
-// go through shared memory TC_CK at a time; each MMA consumes K = 8 channels.
-// Both operands are K-major in the canonical no-swizzle layout: core
-// matrices of 8 rows x 16 bytes (4 channels), 128 contiguous bytes; LBO =
+// Implicit GEMM per CTA: D[m][o] (m = pixel of an 8-wide, 16-high tile, o =
+// NT output channels) += sum over taps k and input channels i of A_k[m][i]
+// B_k[i][o], A_k the input shifted by tap k, B_k[i][o] = w(o, i, k).  Input
+// channels go through shared memory TC_CK at a time; each MMA consumes K = 8
+// channels.  Both operands are K-major in the canonical no-swizzle layout:
+// core matrices of 8 rows x 16 bytes (4 channels), 128 contiguous bytes; LBO =
 // distance of the core matrices adjacent in K, SBO = in M (or N).
-//   A: three copies kx = 0..2 of the 10 x 16 halo window starting at column
-//      kx (core matrix (halo row, 8-column group)), so tap (ky, kx) is copy
-//      kx from halo row ky: rows of D map to pixel (m / 16, m % 16).
-//   B: [tap][channel group][o / 8][o % 8][channel % 4].
+//   A: the halo window, 18 rows of 10 pixels of 16 bytes, per group of four
+//      channels.  A core matrix is eight pixels of a row of the tile, SBO
+//      a row of the window, and tap (ky, kx) starts ky rows and kx pixels on:
+//      descriptors start on any 16 bytes, so no tap needs a copy of its own.
+//   B: [tap][channel group][o / 8][o % 8][channel % 4], through a ring of
+//      TC_NB taps.
 // Activations are rounded to TF32 (cvt.rna) when staged; BF16 weights are
 // exact in TF32.  Every wait is bounded: on a timeout the CTA sets *err,
 // skips its stores and still frees its TMEM.
@@ -108,12 +164,15 @@ __global__ void __launch_bounds__(256) k_conv3(const float *__restrict__ in, int
 constexpr int TC_TY = 8, TC_TX = 16;              // pixel tile (M = 128)
 constexpr int TC_CK = 32;                         // input channels per stage
 constexpr int TC_HY = TC_TY + 2;                  // halo rows
-constexpr int TC_LBO_A = TC_HY * 2 * 128;         // 2560 B: next 4 channels
-constexpr int TC_ACOPY = (TC_CK / 4) * TC_LBO_A;  // 20480 B per kx copy
-constexpr int TC_THREADS = 256;
-
+constexpr int TC_THREADS = 256;                   // of the weight gradient
+constexpr int TC_H = 16, TC_W = 8;                // the convolution's pixel tile (M = 128)
+constexpr int TC_WY = TC_H + 2;                   // its window
+constexpr int TC_WX = TC_W + 2;
+constexpr int TC_LBO_A = TC_WY * TC_WX * 16;      // 2880 B: next 4 channels
+constexpr int TC_CONV = (TC_WY * TC_WX + 31) / 32 * 32;  // threads: one per pixel of the window
+constexpr int TC_NB = 4;                          // ring of taps of weights
 __host__ __device__ constexpr size_t tc_smem_bytes(int NT) {
-    return 3 * (size_t)TC_ACOPY + 9 * (size_t)NT * 128;
+    return (TC_CK / 4) * (size_t)TC_LBO_A + (size_t)TC_NB * NT * TC_CK * 4;
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -169,76 +228,76 @@ __device__ __forceinline__ void tc_bulk_load(uint32_t dst, const void *src, uint
         : "memory");
 }
 
-// Input channels ci0 .. ci0 + 31 of the tile's halo window, staged in two
-// steps so that the loads of one stage are all in flight together (and can
-// overlap the previous stage's MMAs): tc_load_input fills registers, task t
-// (< 1440) = 4 channels of halo pixel (row hy, column hx), hx fastest, and
-// tc_store_input writes them as one 16-byte vector into each kx copy that
-// holds the pixel.  Eight consecutive lanes write eight consecutive pixels
-// (the eight 16-byte rows of a core matrix): no bank conflicts.
-constexpr int TC_HX = TC_TX + 2;
-constexpr int TC_NT_IN = (TC_CK / 4) * TC_HY * TC_HX;  // 1440 tasks
-constexpr int TC_IN_PER = (TC_NT_IN + TC_THREADS - 1) / TC_THREADS;
-struct TcIn {
-    float4 q[TC_IN_PER];
-};
-__device__ __forceinline__ void tc_load_input(TcIn &R, const float *inn, int Ci, int ci0, int H,
-                                              int Wd, int ty0, int tx0, bool) {
-    const size_t plane = (size_t)H * Wd;
+// Input channels of the tile's halo window, staged in two steps so that the
+// loads of one stage are all in flight together (and can overlap the previous
+// stage's MMAs).  One thread serves one pixel of the window: tc_load_input
+// reads its TC_CK channels into registers, tc_store_input writes them, four
+// channels to a 16-byte vector; consecutive lanes write consecutive vectors.
+// With tasks of (pixel, 4 channels) instead, two thirds of the kernel's
+// instructions were the tasks' addresses.
+// p: the pixel in the first of the nc > 0 channels that the image still has
+__device__ __forceinline__ void tc_load_input(float (&R)[TC_CK], const float *p, bool inside,
+                                              int nc, size_t plane) {
 #pragma unroll
-    for (int u = 0; u < TC_IN_PER; ++u) {
-        const int t = threadIdx.x + u * TC_THREADS;
-        const int hx = t % TC_HX, hy = (t / TC_HX) % TC_HY, cq = t / (TC_HX * TC_HY);
-        const int y = ty0 + hy - 1, x = tx0 + hx - 1, c = ci0 + 4 * cq;
-        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t < TC_NT_IN && y >= 0 && y < H && x >= 0 && x < Wd) {
-            const float *p0 = inn + (size_t)c * plane + (size_t)y * Wd + x;
-            q.x = c < Ci ? p0[0] : 0.f;
-            q.y = c + 1 < Ci ? p0[plane] : 0.f;
-            q.z = c + 2 < Ci ? p0[2 * plane] : 0.f;
-            q.w = c + 3 < Ci ? p0[3 * plane] : 0.f;
-        }
-        R.q[u] = q;
+    for (int c = 0; c < TC_CK; ++c) {
+        R[c] = inside && c < nc ? *p : 0.f;
+        if (c + 1 < nc) p += plane;
     }
 }
-__device__ __forceinline__ void tc_store_input(const TcIn &R, float *sA) {
+__device__ __forceinline__ void tc_store_input(const float (&R)[TC_CK], float *sA) {
+    if (threadIdx.x >= TC_WY * TC_WX) return;  // the last warp's spare lanes
 #pragma unroll
-    for (int u = 0; u < TC_IN_PER; ++u) {
-        const int t = threadIdx.x + u * TC_THREADS;
-        if (t >= TC_NT_IN) break;
-        const int hx = t % TC_HX, hy = (t / TC_HX) % TC_HY, cq = t / (TC_HX * TC_HY);
-        const float4 v = make_float4(tc_tf32(R.q[u].x), tc_tf32(R.q[u].y), tc_tf32(R.q[u].z),
-                                     tc_tf32(R.q[u].w));
-        float *base = sA + cq * (TC_LBO_A / 4) + hy * 64;
-#pragma unroll
-        for (int kx = 0; kx < 3; ++kx) {
-            const int xx = hx - kx;
-            if (xx >= 0 && xx < TC_TX)
-                *reinterpret_cast<float4 *>(base + kx * (TC_ACOPY / 4) + (xx >> 3) * 32 +
-                                            (xx & 7) * 4) = v;
-        }
-    }
+    for (int q = 0; q < TC_CK / 4; ++q)
+        *reinterpret_cast<float4 *>(sA + q * (TC_LBO_A / 4) + threadIdx.x * 4) =
+            make_float4(tc_tf32(R[4 * q]), tc_tf32(R[4 * q + 1]), tc_tf32(R[4 * q + 2]),
+                        tc_tf32(R[4 * q + 3]));
 }
 
+// in2: with it the input is the concatenation of `in` (C1 channels, upsampled
+// 2x; C1 a multiple of TC_CK) and in2 (the other Ci - C1) -- a decoder's first
+// convolution, whose concatenated input is then never written (0.75 of the
+// 3.5 ms of a prediction of 64 images of 128 x 128 px).
+// epi: what the layer's output goes through on its way out of the registers --
+// the 2 x 2 average of the next level (pool [N][Co][H/2][Wd/2], H and Wd even;
+// the sums of k_pool), or the 1 x 1 convolution that ends the network (w1, b1,
+// out1 [N][H][Wd], Co == NT; the sums of k_conv1; out is then not written).
 // wpk: the layer's weights packed per (output tile, channel stage) in the
 // shared-memory B layout (NT * 288 floats each, TF32-exact), see
 // k_pack_weights; bias may be null (data gradient)
+// What bounds it: latency (the loads of a stage are 32 channels deep, a layer
+// of 32 channels has one stage and nothing to hide them behind), then the
+// re-reads of A by nine taps.  So four small CTAs per SM: with kx copies of A
+// and all nine taps of weights resident (98 and 135 KB) two and one fitted.
+// 64 images, 128^2 px at 32 channels: 32 -> 32 channels 150 us (was 190), a
+// decoder's 96 -> 32 channels 240 (was 360, and 380 to write its input); all
+// ten layers 1.38 ms (was 2.25).  Measured and left out: two tiles per CTA
+// (half the weight traffic, two CTAs per SM: 20 % slower at every level) and
+// stages of 16 channels (another order of the sum: its last bits flip TF32
+// roundings downstream).
+struct TcEpi {
+    float *pool = nullptr;
+    const float *w1 = nullptr, *b1 = nullptr;
+    float *out1 = nullptr;
+};
 template <int NT>
-__global__ void __launch_bounds__(TC_THREADS) k_conv3_tc(const float *__restrict__ in, int Ci,
-                                                         const float *__restrict__ wpk,
-                                                         const float *__restrict__ bias,
-                                                         float *__restrict__ out, int Co, int H,
-                                                         int Wd, int relu, int tiles_x, int vec) {
+__global__ void __launch_bounds__(TC_CONV, 4)
+    k_conv3_tc(const float *__restrict__ in, const float *__restrict__ in2, int C1, int Ci,
+               const float *__restrict__ wpk, const float *__restrict__ bias,
+               float *__restrict__ out, int Co, int H, int Wd, int relu, int tiles_x,
+               TcEpi epi) {
     static_assert(NT == 32 || NT == 64, "N tile");
     extern __shared__ __align__(1024) uint8_t tc_smem[];
+    constexpr int ROW_A = TC_WX * 16, TAP = NT * TC_CK * 4;
     float *sA = reinterpret_cast<float *>(tc_smem);
-    float *sB = reinterpret_cast<float *>(tc_smem + 3 * TC_ACOPY);
-    __shared__ __align__(8) uint64_t mbar[2];  // [0] MMAs done, [1] weights landed
+    const uint32_t a0 = smem_u32(tc_smem), b0 = a0 + (TC_CK / 4) * TC_LBO_A;
+    // [0] the stage's MMAs done, then per ring slot: weights landed, weights read
+    __shared__ __align__(8) uint64_t mbar[1 + 2 * TC_NB];
     __shared__ uint32_t tmem_slot;
-    const int ty0 = (blockIdx.x / tiles_x) * TC_TY, tx0 = (blockIdx.x % tiles_x) * TC_TX;
+    const int ty0 = (blockIdx.x / tiles_x) * TC_H, tx0 = (blockIdx.x % tiles_x) * TC_W;
     const int co0 = blockIdx.y * NT, n = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t bar = smem_u32(&mbar[0]), bar_w = smem_u32(&mbar[1]);
+    const uint32_t bar = smem_u32(&mbar[0]), bar_f = smem_u32(&mbar[1]);
+    const uint32_t bar_e = smem_u32(&mbar[1 + TC_NB]);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(&tmem_slot)),
@@ -246,56 +305,94 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv3_tc(const float *__restrict
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (threadIdx.x == 32) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_w));
+        for (int i = 0; i < 1 + 2 * TC_NB; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * i));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tm = tmem_slot;
-    const float *inn = in + (size_t)n * Ci * H * Wd;
     const int nstage = (Ci + TC_CK - 1) / TC_CK;
     const float *wt = wpk + (size_t)blockIdx.y * nstage * (NT * 288);
-    constexpr uint32_t WBYTES = NT * 288 * 4;
+    // the last warp's last lane has no pixel of the window: it issues the MMAs
+    const bool issuer = threadIdx.x == TC_CONV - 1;
+    const int ntap = 9 * nstage;
+    int loaded = 0, used = 0;  // taps of weights requested and waited for (issuer)
+    bool dead = false;         // issuer: a wait for weights ran out
+    auto load_tap = [&] {
+        tc_bulk_load(b0 + (loaded % TC_NB) * TAP, wt + (size_t)loaded * (NT * TC_CK), TAP,
+                     bar_f + 8 * (loaded % TC_NB));
+        ++loaded;
+    };
+    if (issuer)
+        while (loaded < TC_NB) load_tap();
+    const int up = in2 ? 1 : 0;
+    const float *inn = in + (size_t)n * C1 * (H >> up) * (Wd >> up);
+    const float *inn2 = up ? in2 + (size_t)n * (Ci - C1) * H * Wd : nullptr;
+    // this thread's pixel of the window, and its offset in either input
+    const int hx = threadIdx.x % TC_WX, hy = threadIdx.x / TC_WX;
+    const int py = ty0 + hy - 1, px = tx0 + hx - 1;
+    const bool pin = hy < TC_WY && py >= 0 && py < H && px >= 0 && px < Wd;
+    const int off1 = pin ? (py >> up) * (Wd >> up) + (px >> up) : 0, off2 = pin ? py * Wd + px : 0;
+    auto load = [&](float(&R)[TC_CK], int s) {
+        const bool one = s * TC_CK < C1;
+        const int c = one ? s * TC_CK : s * TC_CK - C1, nc = (one ? C1 : Ci - C1) - c;
+        const size_t plane = one ? (size_t)(H >> up) * (Wd >> up) : (size_t)H * Wd;
+        tc_load_input(R, (one ? inn + off1 : inn2 + off2) + c * plane, pin, nc, plane);
+    };
     bool ok = true;
     int issued = 0;
-    TcIn R;
-    tc_load_input(R, inn, Ci, 0, H, Wd, ty0, tx0, vec != 0);
+    float R[TC_CK];
+    load(R, 0);
     for (int s = 0; s < nstage; ++s) {
         if (s > 0) {  // the previous stage's MMAs must be done with shared memory
-            const bool mine = tc_mbar_wait(bar, (uint32_t)(s - 1) & 1u);
+            const bool mine = tc_mbar_wait(bar, (uint32_t)(s - 1) & 1u) && !dead;
             ok = !__syncthreads_or(!mine);
             if (!ok) break;
         }
-        if (threadIdx.x == 0) tc_bulk_load(smem_u32(sB), wt + (size_t)s * NT * 288, WBYTES, bar_w);
         tc_store_input(R, sA);
         // generic-proxy stores -> visible to the tensor core (async proxy)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        // the next stage's loads go out first (warp 0 included) and overlap
-        // this stage's MMAs
-        if (s + 1 < nstage) tc_load_input(R, inn, Ci, (s + 1) * TC_CK, H, Wd, ty0, tx0, vec != 0);
-        if (threadIdx.x == 0) {
-            if (!tc_mbar_wait(bar_w, (uint32_t)s & 1u)) atomicExch(&g_unet_tc_err, 1);
+        // the next stage's loads go out first (the issuer's warp included) and
+        // overlap this stage's MMAs
+        if (s + 1 < nstage) load(R, s + 1);
+        if (issuer) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
             constexpr uint32_t idesc = tc_idesc_tf32(128, NT);
 #pragma unroll 1
-            for (int k = 0; k < 9; ++k) {
-                const int ky = k / 3, kx = k % 3;
+            for (int k = 0; k < 9 && !dead; ++k) {
+                const int slot = used % TC_NB;
+                if (!tc_mbar_wait(bar_f + 8 * slot, (uint32_t)(used / TC_NB) & 1u)) {
+                    dead = true;
+                    break;
+                }
+                ++used;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t ak = a0 + (k / 3) * ROW_A + (k % 3) * 16;
 #pragma unroll
                 for (int q = 0; q < TC_CK / 8; ++q) {
-                    const uint64_t da = tc_mdesc(
-                        a0 + kx * TC_ACOPY + ky * 256 + q * 2 * TC_LBO_A, TC_LBO_A, 128);
-                    const uint64_t db =
-                        tc_mdesc(b0 + k * NT * 128 + q * 2 * (NT * 16), NT * 16, 128);
+                    const uint64_t da = tc_mdesc(ak + q * 2 * TC_LBO_A, TC_LBO_A, ROW_A);
+                    const uint64_t db = tc_mdesc(b0 + slot * TAP + q * 2 * (NT * 16), NT * 16, 128);
                     const uint32_t acc = (s | k | q) != 0;
                     asm volatile(
                         "{\n\t.reg .pred p;\n\t"
                         "setp.ne.b32 p, %4, 0;\n\t"
                         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tm),
                         "l"(da), "l"(db), "r"(idesc), "r"(acc));
+                }
+                asm volatile(
+                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                        bar_e + 8 * slot)
+                    : "memory");
+                // the slot of the tap before this one takes the next tap of the ring
+                if (used > 1 && loaded < ntap) {
+                    const int g = used - 2;
+                    if (tc_mbar_wait(bar_e + 8 * (g % TC_NB), (uint32_t)(g / TC_NB) & 1u))
+                        load_tap();
+                    else
+                        dead = true;
                 }
             }
             asm volatile(
@@ -306,45 +403,71 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv3_tc(const float *__restrict
         issued = s + 1;
     }
     if (ok) {
-        const bool mine = tc_mbar_wait(bar, (uint32_t)(nstage - 1) & 1u);
+        const bool mine = tc_mbar_wait(bar, (uint32_t)(nstage - 1) & 1u) && !dead;
         ok = !__syncthreads_or(!mine);
     }
     if (!ok) {
-        if (threadIdx.x == 0) atomicExch(&g_unet_tc_err, 1);
-        // give the MMAs and the weight copy in flight a second bounded chance
+        if (issuer) atomicExch(&g_unet_tc_err, 1);
+        // give the MMAs and the weight copies in flight a second bounded chance
         // before the TMEM and the shared memory are released
         if (issued > 0) tc_mbar_wait(bar, (uint32_t)(issued - 1) & 1u);
-        if (threadIdx.x == 0 && issued < nstage) tc_mbar_wait(bar_w, (uint32_t)issued & 1u);
+        for (; issuer && used < loaded; ++used)
+            tc_mbar_wait(bar_f + 8 * (used % TC_NB), (uint32_t)(used / TC_NB) & 1u);
+        __syncthreads();
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (= pixels), columns
-    // (w / 4) NT / 2 .. + NT / 2 (= output channels)
+    // epilogue: warp w < 4 reads TMEM lanes 32 w .. 32 w + 31 (= pixels), all
+    // NT columns (= output channels)
     const int m = (warp & 3) * 32 + lane;
-    const int y = ty0 + m / TC_TX, x = tx0 + m % TC_TX;
+    const int y = ty0 + m / TC_W, x = tx0 + m % TC_W;
     const bool inside = ok && y < H && x < Wd;
+    const size_t oplane = (size_t)H * Wd;
+    float *po = out + ((size_t)n * Co + co0) * oplane + (inside ? (size_t)y * Wd + x : 0);
+    // the lane of an even row and column averages its own 2 x 2 pixels
+    const bool pools = epi.pool && inside && !(lane & 9);
+    const size_t pplane = oplane / 4;
+    float *pp = epi.pool + ((size_t)n * Co + co0) * pplane +
+                (pools ? (size_t)(y / 2) * (Wd / 2) + x / 2 : 0);
+    float a1 = epi.w1 ? epi.b1[0] : 0.f;
+    if (warp < 4) {
 #pragma unroll
-    for (int j0 = (warp >> 2) * (NT / 2); j0 < (warp >> 2) * (NT / 2) + NT / 2; j0 += 16) {
-        uint32_t r[16];
-        const uint32_t ta = tm + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)j0;
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, "
-            "%10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-              "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-              "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(ta));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (inside) {
+        for (int j0 = 0; j0 < NT; j0 += 16) {
+            uint32_t r[16];
+            const uint32_t ta = tm + ((uint32_t)(warp * 32) << 16) + (uint32_t)j0;
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, "
+                "%10, %11, %12, %13, %14, %15}, [%16];"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                  "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                  "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                : "r"(ta));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int o = co0 + j0 + j;
-                if (o < Co) {
-                    float v = __uint_as_float(r[j]) + (bias ? bias[o] : 0.f);
-                    if (relu) v = fmaxf(v, 0.f);
-                    out[(((size_t)n * Co + o) * H + y) * Wd + x] = v;
+            for (int j = 0; j < 16; ++j) {  // Co is a multiple of NT
+                float v = __uint_as_float(r[j]) + (bias ? bias[co0 + j0 + j] : 0.f);
+                if (relu) v = fmaxf(v, 0.f);
+                r[j] = __float_as_uint(v);
+            }
+            if (epi.w1) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    a1 = fmaf(epi.w1[j0 + j], __uint_as_float(r[j]), a1);
+            } else if (inside) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j, po += oplane) *po = __uint_as_float(r[j]);
+            }
+            if (epi.pool) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j, pp += pplane) {
+                    const float v = __uint_as_float(r[j]);
+                    float s = v + __shfl_xor_sync(~0u, v, 1);
+                    s += __shfl_down_sync(~0u, v, TC_W);
+                    s += __shfl_down_sync(~0u, v, TC_W + 1);
+                    if (pools) *pp = 0.25f * s;
                 }
             }
         }
+        if (epi.w1 && inside) epi.out1[(size_t)n * oplane + (size_t)y * Wd + x] = a1;
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -378,7 +501,7 @@ __global__ void k_pack_weights(const __nv_bfloat16 *__restrict__ wb, float *__re
         const int per = E.NT * 288;
         const int blk = (int)(j / per), r = (int)(j % per);
         const int cot = blk / E.nstage, stg = blk % E.nstage;
-        const int k = r / (E.NT * 32), r2 = r % (E.NT * 32);
+        const int k = r / (E.NT * TC_CK), r2 = r % (E.NT * TC_CK);
         const int cg = r2 / (E.NT * 4), r3 = r2 % (E.NT * 4);
         const int o = cot * E.NT + (r3 / 32) * 8 + (r3 % 32) / 4;
         const int c = stg * TC_CK + cg * 4 + r3 % 4;
@@ -896,17 +1019,25 @@ inline bool tc_shape(int Ci, int Co) { return Ci >= 8 && Co % 32 == 0; }
 inline int tc_nt(int Co) { return Co % 64 == 0 ? 64 : 32; }
 
 template <int NT>
-int conv3_tc(const float *in, int Ci, const float *wpk, const float *bias, float *out, int Co,
-             int S, int N, int relu, cudaStream_t st) {
+int conv3_tc_nt(const float *in, const float *in2, int C1, int Ci, const float *wpk,
+                const float *bias, float *out, int Co, int S, int N, int relu, const TcEpi &epi,
+                cudaStream_t st) {
     const size_t smem = tc_smem_bytes(NT);
     MSOT_CUDA_TRY(raise_max_dynamic_smem((const void *)k_conv3_tc<NT>, smem));
-    const int tx = (S + TC_TX - 1) / TC_TX, ty = (S + TC_TY - 1) / TC_TY;
-    const int vec = (S % 4 == 0) && ((uintptr_t)in % 16 == 0);
+    const int tx = (S + TC_W - 1) / TC_W, ty = (S + TC_H - 1) / TC_H;
     dim3 grid(tx * ty, Co / NT, N);
-    KLAUNCH(k_conv3_tc<NT><<<grid, TC_THREADS, smem, st>>>(in, Ci, wpk, bias, out, Co, S, S, relu,
-                                                          tx, vec));
+    KLAUNCH(k_conv3_tc<NT><<<grid, TC_CONV, smem, st>>>(in, in2, C1, Ci, wpk, bias, out, Co, S, S,
+                                                       relu, tx, epi));
     MSOT_LAUNCH_CHECK();
     return MSOT_OK;
+}
+// in2, C1, epi: see k_conv3_tc
+int conv3_tc(const float *in, const float *in2, int C1, int Ci, const float *wpk,
+             const float *bias, float *out, int Co, int S, int N, int relu, const TcEpi &epi,
+             cudaStream_t st) {
+    return tc_nt(Co) == 64
+               ? conv3_tc_nt<64>(in, in2, C1, Ci, wpk, bias, out, Co, S, N, relu, epi, st)
+               : conv3_tc_nt<32>(in, in2, C1, Ci, wpk, bias, out, Co, S, N, relu, epi, st);
 }
 
 // 3x3 "same" convolution of [N][Ci][S][S] into [N][Co][S][S]: on the tensor
@@ -917,8 +1048,16 @@ template <bool TRANS>
 int conv3(const float *in, int Ci, const __nv_bfloat16 *w, const float *wpk, const float *bias,
           float *out, int Co, int S, int N, int relu, cudaStream_t st) {
     if (g_unet_tc.load() && wpk)
-        return tc_nt(Co) == 64 ? conv3_tc<64>(in, Ci, wpk, bias, out, Co, S, N, relu, st)
-                               : conv3_tc<32>(in, Ci, wpk, bias, out, Co, S, N, relu, st);
+        return conv3_tc(in, nullptr, Ci, Ci, wpk, bias, out, Co, S, N, relu, TcEpi(), st);
+    if (!TRANS && Ci <= 2) {
+        const dim3 g((S * S + 255) / 256, (Co + 31) / 32, N);
+        if (Ci == 1)
+            KLAUNCH(k_conv3_in<1><<<g, 256, 0, st>>>(in, w, bias, out, Co, S, S, relu));
+        else
+            KLAUNCH(k_conv3_in<2><<<g, 256, 0, st>>>(in, w, bias, out, Co, S, S, relu));
+        MSOT_LAUNCH_CHECK();
+        return MSOT_OK;
+    }
     const int tx = (S + CT - 1) / CT;
     dim3 grid(tx * tx, (Co + COT - 1) / COT, N);
     KLAUNCH(k_conv3<TRANS><<<grid, 256, 0, st>>>(in, Ci, w, bias, out, Co, S, S, relu, tx));
@@ -972,13 +1111,25 @@ int conv_bwd(msot_unet *u, const ConvL &c, const float *x, const float *y, const
     return MSOT_OK;
 }
 
-int forward(msot_unet *u, const float *in, int N, cudaStream_t st) {
+// train: backward() follows and reads the decoders' concatenated inputs
+int forward(msot_unet *u, const float *in, int N, bool train, cudaStream_t st) {
     int rc;
     const int L = u->L;
+    const bool use_tc = g_unet_tc.load();
     const float *x = in;
     for (int l = 0; l < L; ++l) {
         if ((rc = conv_fwd(u, u->enc_a[l], x, u->ea[l], N, st))) return rc;
-        if ((rc = conv_fwd(u, u->enc_b[l], u->ea[l], u->e[l], N, st))) return rc;
+        const ConvL &c = u->enc_b[l];
+        if (l + 1 < L && use_tc && c.pk_fwd != NO_PACK) {
+            TcEpi epi;
+            epi.pool = u->pool[l];
+            if ((rc = conv3_tc(u->ea[l], nullptr, c.Ci, c.Ci, u->wpk + c.pk_fwd,
+                                   u->par + c.b_off, u->e[l], c.Co, c.S, N, 1, epi, st)))
+                return rc;
+            x = u->pool[l];
+            continue;
+        }
+        if ((rc = conv_fwd(u, c, u->ea[l], u->e[l], N, st))) return rc;
         if (l + 1 < L) {
             const int S = u->side[l];
             const size_t n = (size_t)N * u->ch[l] * (S / 2) * (S / 2);
@@ -989,6 +1140,24 @@ int forward(msot_unet *u, const float *in, int N, cudaStream_t st) {
     const float *dn = u->e[L - 1];
     for (int l = L - 2; l >= 0; --l) {
         const int S = u->side[l], Cu = u->ch[l + 1], Ce = u->ch[l], Ct = Cu + Ce;
+        const ConvL &c = u->dec_c[l];
+        if (!train && use_tc && c.pk_fwd != NO_PACK && Cu % TC_CK == 0) {
+            rc = conv3_tc(dn, u->e[l], Cu, Ct, u->wpk + c.pk_fwd, u->par + c.b_off, u->da[l],
+                              c.Co, S, N, 1, TcEpi(), st);
+            if (rc) return rc;
+            const ConvL &d = u->dec_d[l];
+            if (l == 0 && d.pk_fwd != NO_PACK && d.Co == tc_nt(d.Co)) {
+                TcEpi epi;
+                epi.w1 = u->par + u->out_w;
+                epi.b1 = u->par + u->out_b;
+                epi.out1 = u->outb;
+                return conv3_tc(u->da[l], nullptr, d.Ci, d.Ci, u->wpk + d.pk_fwd,
+                                    u->par + d.b_off, u->d[l], d.Co, d.S, N, 1, epi, st);
+            }
+            if ((rc = conv_fwd(u, d, u->da[l], u->d[l], N, st))) return rc;
+            dn = u->d[l];
+            continue;
+        }
         KLAUNCH(k_up_into<<<nblk((size_t)N * Cu * S * S), 256, 0, st>>>(dn, u->cat[l], N, Cu, Ct,
                                                                          S / 2, S / 2));
         KLAUNCH(k_chan_copy<<<nblk((size_t)N * Ce * S * S), 256, 0, st>>>(
@@ -1262,7 +1431,7 @@ int msot_unet_forward(msot_unet_t u, const float *d_in, float *d_out, int n, voi
     int rc = check_net(u, n, d_in, d_out);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    if ((rc = forward(u, d_in, n, st))) return rc;
+    if ((rc = forward(u, d_in, n, false, st))) return rc;
     MSOT_CUDA_TRY(cudaMemcpyAsync(d_out, u->outb, sizeof(float) * n * u->S * u->S,
                                   cudaMemcpyDeviceToDevice, st));
     return MSOT_OK;
@@ -1273,7 +1442,7 @@ int msot_unet_gradients(msot_unet_t u, const float *d_in, const float *d_target,
     int rc = check_net(u, n, d_in, d_target);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    if ((rc = forward(u, d_in, n, st))) return rc;
+    if ((rc = forward(u, d_in, n, true, st))) return rc;
     if ((rc = backward(u, d_in, d_target, n, st))) return rc;
     if (loss)
         MSOT_CUDA_TRY(cudaMemcpyAsync(loss, u->loss, sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -300,6 +300,7 @@ constexpr int TVC_THREADS = 512;
 constexpr int TVC_MAXC = 16;  // largest cluster
 // u, x, bub1, bub2, r, rt, p (two buffers), q, uc, uh, vh, xmin
 constexpr int TVC_NV = 13;
+constexpr int TVC_NV_REG = 9;  // without uh, and rt, M uc, M q in registers
 enum TvcVec { V_U = 0, V_X, V_B1, V_B2, V_R, V_RT, V_P0, V_P1, V_Q, V_UC, V_UH, V_VH, V_XMIN };
 
 // Thread mapping inside a slab: thread t owns row iz = t % N of the columns
@@ -631,6 +632,16 @@ __global__ void __launch_bounds__(TVC_THREADS, 2)
 // Two stencils and two cluster sums per step, as before; every vector read
 // remotely in a phase was written before the cluster barrier that opened
 // it, and is rewritten only after the next one.
+//
+// KM > 0: a thread owns at most KM groups and keeps the vectors that no other
+// thread reads (rt, M uc, M q) in registers: nine vectors of shared memory
+// instead of thirteen, so that larger images fit a smaller cluster, which
+// matters because the barriers and not the pixels bound a step: an image of
+// 200 x 200 takes 0.53 ms with 16 CTAs and 0.58 with 8 (with thirteen vectors
+// it needed the 16: 0.57), and twice as many clusters of 8 run at once --
+// 8 images 0.60 ms (was 1.01), 28 images 1.06 (was 1.90).  One CTA per SM
+// and 128 registers; KM = 4 spills a little (160 x 160 px: 0.72 ms with
+// 4 CTAs, 0.48 with 8 and KM = 2).
 // ---------------------------------------------------------------------------
 struct F4 {
     float v[4];
@@ -689,14 +700,20 @@ __device__ __forceinline__ F4 tvc4_M(const Tvc4Ctx &c, int oi, int lc, int l, Ha
     return o;
 }
 
-#define TVC4_FOR(c) for (int lc = (c).lc0, l = lc * (c).N + (c).iz0; lc < (c).nl; lc += (c).G, l += (c).G * (c).N)
+// loop over this thread's groups e (lc, l); KU copies of the body
+#define TVC4_FOR(c)                                                                        \
+    _Pragma("unroll KU") for (int e = 0, lc = (c).lc0, l = lc * (c).N + (c).iz0;           \
+                              KM ? e < KM : lc < (c).nl;                                   \
+                              ++e, lc += (c).G, l += (c).G * (c).N) if (!KM || lc < (c).nl)
 
-template <bool GM>
-__global__ void __launch_bounds__(TVC_THREADS, 2)
+template <bool GM, int KM>
+__global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
     k_tv_prox_cl4(const float *__restrict__ g_all, const TvState *__restrict__ st,
                   double mu_const, int coupled, float *__restrict__ out_all, int N, int C,
                   int nloc, float *__restrict__ gwork) {
     namespace cg = cooperative_groups;
+    static_assert(!GM || KM == 0, "global vectors: none in registers");
+    constexpr int KU = KM ? KM : 1;
     extern __shared__ float4 tvc_smem[];
     __shared__ float wsum[64];
     __shared__ float red[2 * TVC_MAXC * 2];
@@ -730,9 +747,23 @@ __global__ void __launch_bounds__(TVC_THREADS, 2)
     const int V = nloc * N;
     float *S = c.sm;
     int ou = V_U * V, ox = V_X * V;
-    const int ob1 = V_B1 * V, ob2 = V_B2 * V, orr = V_R * V, ort = V_RT * V, oq = V_Q * V,
-              ouc = V_UC * V, ovh = V_VH * V, oxm = V_XMIN * V;
-    const int omq = V_P0 * V, omuc = V_P1 * V;  // M q and M uc (no p, no uh here)
+    const int ob1 = V_B1 * V, ob2 = V_B2 * V, orr = V_R * V, oq = (KM ? 5 : V_Q) * V,
+              ouc = (KM ? 6 : V_UC) * V, ovh = (KM ? 7 : V_VH) * V, oxm = (KM ? 8 : V_XMIN) * V;
+    // rt, M q and M uc (no p, no uh here): in registers with KM
+    const int ort = V_RT * V, omq = V_P0 * V, omuc = V_P1 * V;
+    F4 rrt[KU], rmq[KU], rmuc[KU];
+    auto put = [&](F4 &reg, int o, const F4 &v) {
+        if constexpr (KM > 0)
+            reg = v;
+        else
+            st4(S + o, v);
+    };
+    auto get = [&](const F4 &reg, int o) {
+        if constexpr (KM > 0)
+            return reg;
+        else
+            return ld4(S + o);
+    };
     int par = 0, n_sweeps = 0, n_cg = 0;
     float A = 0.f, B = 0.f;
     float n2b = 0.f, rho = 0.f, rho1 = 1.f, normrmin = 0.f;
@@ -784,7 +815,7 @@ __global__ void __launch_bounds__(TVC_THREADS, 2)
                 n2 = fmaf(rh.v[k], rh.v[k], n2);
             }
             st4(S + orr + l, rh);
-            st4(S + ort + l, rh);
+            put(rrt[KM ? e : 0], ort + l, rh);
             st4(S + ox + l, zero4);
             st4(S + oxm + l, zero4);
         }
@@ -828,16 +859,16 @@ __global__ void __launch_bounds__(TVC_THREADS, 2)
                 float a_rtvh = 0.f;
                 TVC4_FOR(c) {
                     const F4 muc = tvc4_M(c, ouc, lc, l, halo_uc);
-                    st4(S + omuc + l, muc);
+                    put(rmuc[KM ? e : 0], omuc + l, muc);
                     F4 vh = muc;
                     if (!first) {
-                        const F4 mq = ld4(S + omq + l), vo = ld4(S + ovh + l);
+                        const F4 mq = get(rmq[KM ? e : 0], omq + l), vo = ld4(S + ovh + l);
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             vh.v[k] = fmaf(beta, fmaf(beta, vo.v[k], mq.v[k]), muc.v[k]);
                     }
                     st4(S + ovh + l, vh);
-                    const F4 rt = ld4(S + ort + l);
+                    const F4 rt = get(rrt[KM ? e : 0], ort + l);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) a_rtvh = fmaf(rt.v[k], vh.v[k], a_rtvh);
                 }
@@ -850,8 +881,10 @@ __global__ void __launch_bounds__(TVC_THREADS, 2)
                 float a_rr = 0.f, a_rtr = 0.f;
                 TVC4_FOR(c) {
                     const F4 mv = tvc4_M(c, ovh, lc, l, halo_vh);
-                    const F4 uv = ld4(S + ouc + l), vh = ld4(S + ovh + l), muc = ld4(S + omuc + l);
-                    const F4 xv = ld4(S + ox + l), rv = ld4(S + orr + l), rt = ld4(S + ort + l);
+                    const F4 uv = ld4(S + ouc + l), vh = ld4(S + ovh + l);
+                    const F4 muc = get(rmuc[KM ? e : 0], omuc + l);
+                    const F4 xv = ld4(S + ox + l), rv = ld4(S + orr + l);
+                    const F4 rt = get(rrt[KM ? e : 0], ort + l);
                     F4 q, mq, xn, rn;
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
@@ -863,7 +896,7 @@ __global__ void __launch_bounds__(TVC_THREADS, 2)
                         a_rtr = fmaf(rt.v[k], rn.v[k], a_rtr);
                     }
                     st4(S + oq + l, q);
-                    st4(S + omq + l, mq);
+                    put(rmq[KM ? e : 0], omq + l, mq);
                     st4(S + ox + l, xn);
                     st4(S + orr + l, rn);
                 }
@@ -1177,11 +1210,10 @@ int blocks_per_instance(int W) {
 // 0: cluster path where it fits, 1: force the global-memory kernel
 std::atomic<int> g_prox_path{0};
 
-// cluster geometry of the shared-memory-resident prox for an N x N image:
-// the smallest cluster whose slab fits two CTAs per SM (portable sizes up to
-// 8), else one CTA per SM (up to 16); none if the image does not fit.
+// cluster geometry of the shared-memory-resident prox for W images of N x N:
+// C CTAs per image, KM groups per thread with vectors in registers (0: none).
 struct TvcGeom {
-    int C = 0, nloc = 0;
+    int C = 0, nloc = 0, KM = 0;
     size_t smem = 0;
 };
 
@@ -1189,39 +1221,65 @@ struct TvcGeom {
 // cluster with its vectors in the global-memory workspace
 std::atomic<int> g_tv_cluster{0};
 
-TvcGeom tvc_geometry(int N, int force = 0) {
+constexpr size_t TVC_TWO = 113 * 1024, TVC_ONE = 225 * 1024;  // two CTAs per SM, one
+constexpr int TVC_KM = 4;                                     // most groups in registers
+
+// the geometry with C CTAs per image, C = 0 in it if the image does not fit
+TvcGeom tvc_fit(int N, int C) {
     TvcGeom g;
-    if (N > TVC_THREADS) return g;
-    if (const int Cf = force ? force : g_tv_cluster.load()) {
-        if (Cf < 0) return g;  // no shared-memory geometry: the global-memory form
-        const int nloc = (N + Cf - 1) / Cf;
-        const size_t bytes = (size_t)TVC_NV * nloc * N * sizeof(float);
-        if (bytes <= 225 * 1024) {
-            g.C = Cf;
-            g.nloc = nloc;
-            g.smem = bytes;
-        }
-        return g;
-    }
-    const size_t two_per_sm = 113 * 1024, one_per_sm = 225 * 1024;
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int C = 1; C <= (pass ? 16 : 8); C *= 2) {
-            const int nloc = (N + C - 1) / C;
-            const size_t bytes = (size_t)TVC_NV * nloc * N * sizeof(float);
-            if (bytes <= (pass ? one_per_sm : two_per_sm)) {
-                g.C = C;
-                g.nloc = nloc;
-                g.smem = bytes;
-                return g;
-            }
+    const int nloc = (N + C - 1) / C;
+    size_t bytes = (size_t)TVC_NV * nloc * N * sizeof(float);
+    if (bytes > TVC_TWO && N % 4 == 0) {
+        const int G = TVC_THREADS / (N / 4), km = std::max(2, (nloc + G - 1) / G);
+        const size_t few = (size_t)TVC_NV_REG * nloc * N * sizeof(float);
+        if (km <= TVC_KM && few <= TVC_ONE) {
+            g.KM = km;
+            bytes = few;
         }
     }
+    if (bytes > TVC_ONE) return TvcGeom();
+    g.C = C;
+    g.nloc = nloc;
+    g.smem = bytes;
     return g;
+}
+
+int tvc_active(const TvcGeom &g, int N);
+
+// The smallest cluster whose slab fits two CTAs per SM (portable sizes up to
+// 8); else, one CTA per SM, the register form whose rounds of clusters cost
+// least: rounds x (1 + 2e-4 x pixels of a CTA), the slope fitted to one round
+// of 2600, 3200, 5000 and 6400 pixels (0.53, 0.48, 0.58, 0.72 ms).  So one
+// image of 200 x 200 has 16 CTAs and eight images have 8 each; 28 images of
+// 160 x 160 have 4 CTAs each (0.74 ms; with 8: 0.83).
+TvcGeom tvc_geometry(int N, int W, int force = 0) {
+    if (N > TVC_THREADS) return TvcGeom();
+    if (const int Cf = force ? force : g_tv_cluster.load())
+        // negative: no shared-memory geometry, the global-memory form
+        return Cf < 0 ? TvcGeom() : tvc_fit(N, Cf);
+    for (int C = 1; C <= 8; C *= 2)
+        if ((size_t)TVC_NV * ((N + C - 1) / C) * N * sizeof(float) <= TVC_TWO) return tvc_fit(N, C);
+    TvcGeom best, smallest;
+    double cost = 1e30;
+    for (int C = 16; C >= 1; C /= 2) {
+        const TvcGeom g = tvc_fit(N, C);
+        if (!g.C) break;
+        smallest = g;
+        const int act = g.KM ? tvc_active(g, N) : 0;
+        if (act < 1) continue;
+        const double t = (double)((W + act - 1) / act) * (1.0 + 2e-4 * g.nloc * N);
+        if (t < cost) {
+            cost = t;
+            best = g;
+        }
+    }
+    return best.C ? best : smallest;
 }
 
 template <class K>
 static cudaError_t tvc_config(K kern, const TvcGeom &gm, int W, cudaStream_t st,
-                              cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, bool &fits) {
+                              cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int &clusters) {
+    clusters = 0;
     cudaError_t e = raise_max_dynamic_smem((const void *)kern, gm.smem);
     if (e != cudaSuccess) return e;
     if (gm.C > 8) {
@@ -1239,30 +1297,54 @@ static cudaError_t tvc_config(K kern, const TvcGeom &gm, int W, cudaStream_t st,
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    int clusters = 0;
     e = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
     if (e != cudaSuccess || clusters < 1) {
         (void)cudaGetLastError();
-        fits = false;
-        return cudaSuccess;
+        clusters = 0;
     }
-    fits = true;
     return cudaSuccess;
+}
+
+// the kernel of a geometry for N % 4 == 0: 4 z-pixels per thread
+using TvcKernel4 = void (*)(const float *, const TvState *, double, int, float *, int, int, int,
+                            float *);
+TvcKernel4 tvc_kernel4(const TvcGeom &g) {
+    switch (g.KM) {
+    case 2: return k_tv_prox_cl4<false, 2>;
+    case 3: return k_tv_prox_cl4<false, 3>;
+    case 4: return k_tv_prox_cl4<false, 4>;
+    default: return k_tv_prox_cl4<false, 0>;
+    }
+}
+
+// clusters of a geometry that the GPU runs at once, 0 if it cannot run it
+int tvc_active(const TvcGeom &g, int N) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    int n = 0;
+    const cudaError_t e =
+        N % 4 == 0 ? tvc_config(tvc_kernel4(g), g, 1, nullptr, cfg, at, n)
+                   : tvc_config(k_tv_prox_cl, g, 1, nullptr, cfg, at, n);
+    return e == cudaSuccess ? n : 0;
 }
 
 cudaError_t tvc_launch(const TvcGeom &gm, const float *z, const TvState *sv, double mu,
                        int coupled, float *out, int W, int N, cudaStream_t st, bool &fits) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[1];
+    int clusters = 0;
     // 4 z-pixels per thread where N allows (16-byte aligned groups)
     if (N % 4 == 0 && N / 4 <= TVC_THREADS) {
-        cudaError_t e = tvc_config(k_tv_prox_cl4<false>, gm, W, st, cfg, at, fits);
+        const TvcKernel4 kern = tvc_kernel4(gm);
+        cudaError_t e = tvc_config(kern, gm, W, st, cfg, at, clusters);
+        fits = clusters > 0;
         if (e != cudaSuccess || !fits) return e;
         ++g_launch_count;
-        return cudaLaunchKernelEx(&cfg, k_tv_prox_cl4<false>, z, sv, mu, coupled, out, N, gm.C,
-                                  gm.nloc, (float *)nullptr);
+        return cudaLaunchKernelEx(&cfg, kern, z, sv, mu, coupled, out, N, gm.C, gm.nloc,
+                                  (float *)nullptr);
     }
-    cudaError_t e = tvc_config(k_tv_prox_cl, gm, W, st, cfg, at, fits);
+    cudaError_t e = tvc_config(k_tv_prox_cl, gm, W, st, cfg, at, clusters);
+    fits = clusters > 0;
     if (e != cudaSuccess || !fits) return e;
     ++g_launch_count;
     return cudaLaunchKernelEx(&cfg, k_tv_prox_cl, z, sv, mu, coupled, out, N, gm.C, gm.nloc);
@@ -1278,7 +1360,7 @@ cudaError_t tvc_launch_gm(const float *z, const TvState *sv, double mu, int coup
     // the slabs must fit the workspace of TV_NVEC vectors per image
     if (N % 4 != 0 || N / 4 > TVC_THREADS || (size_t)C * TVC_NV * nloc > (size_t)TV_NVEC * N)
         return cudaSuccess;
-    auto kern = k_tv_prox_cl4<true>;
+    auto kern = k_tv_prox_cl4<true, 0>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
@@ -1310,7 +1392,7 @@ cudaError_t tvc_launch_gm(const float *z, const TvState *sv, double mu, int coup
 int tv_prox(const float *z, const TvState *sv, double mu, int coupled, float *out, float *work,
             int W, int N, cudaStream_t st, int cluster) {
     TimedScope ts(KID_TV_PROX, st);
-    const TvcGeom gm = tvc_geometry(N, cluster);
+    const TvcGeom gm = tvc_geometry(N, W, cluster);
     if (g_prox_path.load() == 0 && gm.C) {
         bool fits = false;
         const cudaError_t e = tvc_launch(gm, z, sv, mu, coupled, out, W, N, st, fits);
@@ -1771,7 +1853,7 @@ extern "C" int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tun
         double best = 1e30;
         int pick = 0;
         for (int C : {0, 1, 2, 4, 8, 16, -1}) {
-            if (C > 0 && !tvc_geometry(pl.nx, C).C) continue;
+            if (C > 0 && !tvc_geometry(pl.nx, batch, C).C) continue;
             if (C < 0 && pl.nx % 4 != 0) continue;
             double ms;
             if ((rc = tune_time(st, 2, ms, [&] {

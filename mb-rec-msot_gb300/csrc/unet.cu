@@ -268,9 +268,9 @@ __device__ __forceinline__ void tc_store_input(const float (&R)[TC_CK], float *s
 // of 32 channels has one stage and nothing to hide them behind), then the
 // re-reads of A by nine taps.  So four small CTAs per SM: with kx copies of A
 // and all nine taps of weights resident (98 and 135 KB) two and one fitted.
-// 64 images, 128^2 px at 32 channels: 32 -> 32 channels 150 us (was 190), a
-// decoder's 96 -> 32 channels 240 (was 360, and 380 to write its input); all
-// ten layers 1.38 ms (was 2.25).  Measured and left out: two tiles per CTA
+// 64 images, 128^2 px at 32 channels: 32 -> 32 channels 120 us (was 183), a
+// decoder's 96 -> 32 channels 286 (was 404, and 408 to write its input); all
+// thirteen layers of a four-level net 1.38 ms (was 2.40).  Measured and left out: two tiles per CTA
 // (half the weight traffic, two CTAs per SM: 20 % slower at every level) and
 // stages of 16 channels (another order of the sum: its last bits flip TF32
 // roundings downstream).

@@ -8,12 +8,12 @@
 //                 sweeps).  One CTA per image runs the whole prox on the
 //                 device (bounded loops, no host round trips), vectors in
 //                 global memory.
-//   k_tv_prox_cl / k_tv_prox_cl4  the same prox by one thread-block cluster
-//                 per image, the image split into column slabs held in
-//                 shared memory (neighbours over distributed shared memory);
-//                 cl4 handles 4 z-pixels per thread, and its GM form keeps
-//                 the vectors in an L2-resident workspace for images too large
-//                 for shared memory.  k_tv_prox is the fallback.
+//   k_tv_prox_cl4  the same prox by one thread-block cluster per image, the
+//                 image split into column slabs held in shared memory
+//                 (neighbours over distributed shared memory), 4 z-pixels per
+//                 thread; its GM form keeps the vectors in an L2-resident
+//                 workspace for images too large for shared memory.
+//                 k_tv_prox is the fallback.
 //   k_itv      <- ITV.m:5-6 (isotropic TV with MATLAB's gradient: central
 //                 differences inside, one-sided at the borders).
 //   msot_rec_nn_with_TV_reg <- rec_nn_with_TV_reg.m:20-54 and
@@ -298,20 +298,10 @@ __device__ unsigned long long g_tv_stats[2];
 
 constexpr int TVC_THREADS = 512;
 constexpr int TVC_MAXC = 16;  // largest cluster
-// u, x, bub1, bub2, r, rt, p (two buffers), q, uc, uh, vh, xmin
-constexpr int TVC_NV = 13;
-constexpr int TVC_NV_REG = 9;  // without uh, and rt, M uc, M q in registers
-enum TvcVec { V_U = 0, V_X, V_B1, V_B2, V_R, V_RT, V_P0, V_P1, V_Q, V_UC, V_UH, V_VH, V_XMIN };
-
-// Thread mapping inside a slab: thread t owns row iz = t % N of the columns
-// lc = t / N, t / N + G, ... (G = TVC_THREADS / N column groups; N <= 512).
-struct TvcCtx {
-    float *sm;        // this CTA's vectors
-    const float *sl;  // left neighbour's vectors (rank - 1), or null
-    const float *sr;  // right neighbour's vectors (rank + 1), or null
-    int N, nloc, nl, ix0, iz, G, lc0;
-    bool zlo, zhi;
-};
+// u, x, bub1, bub2, r, rt, M q, M uc, q, uc, vh, xmin
+constexpr int TVC_NV = 12;
+constexpr int TVC_NV_REG = 9;  // without rt, M uc, M q: in registers
+enum TvcVec { V_U = 0, V_X, V_B1, V_B2, V_R, V_RT, V_MQ, V_MUC, V_Q, V_UC, V_VH, V_XMIN };
 
 // the Bregman quantities b = Bub - d and b - d of one pixel from its Bub pair
 __device__ __forceinline__ void tvc_bd(float a1, float a2, float mu, float &b1, float &b2,
@@ -323,31 +313,6 @@ __device__ __forceinline__ void tvc_bd(float a1, float a2, float mu, float &b1, 
     b2 = a2 - d2;
     c1 = b1 - d1;
     c2 = b2 - d2;
-}
-
-// value of vector o at the left / right x-neighbour of (lc, iz), element l
-__device__ __forceinline__ float tvc_left(const TvcCtx &c, int o, int lc, int l) {
-    return lc == 0 ? c.sl[o + (c.nloc - 1) * c.N + c.iz] : c.sm[o + l - c.N];
-}
-__device__ __forceinline__ float tvc_right(const TvcCtx &c, int o, int lc, int l) {
-    return lc == c.nl - 1 ? c.sr[o + c.iz] : c.sm[o + l + c.N];
-}
-
-// (I + B'B) of vector oi at (lc, iz) (same stencil as tv_apply_M).  The
-// x-neighbours in the adjacent slabs are not read from oi there: halo(base,
-// k) recomputes them from that CTA's vectors (base = its shared memory, k =
-// the element), with the same float operations the owner used.
-template <class Halo>
-__device__ __forceinline__ float tvc_M(const TvcCtx &c, int oi, int lc, int l, Halo halo) {
-    const float *in = c.sm + oi;
-    const int ix = c.ix0 + lc;
-    const float v = in[l];
-    const float g1 = c.zlo ? v - in[l - 1] : 0.f;
-    const float g1n = c.zhi ? in[l + 1] - v : 0.f;
-    float g2 = 0.f, g2n = 0.f;
-    if (ix >= 1) g2 = v - (lc == 0 ? halo(c.sl, (c.nloc - 1) * c.N + c.iz) : in[l - c.N]);
-    if (ix + 1 < c.N) g2n = (lc == c.nl - 1 ? halo(c.sr, c.iz) : in[l + c.N]) - v;
-    return v + (g1 - g1n) + (g2 - g2n);
 }
 
 // Cluster-wide sums of two per-thread values, returned to every thread.
@@ -401,227 +366,14 @@ __device__ __forceinline__ void tvc_reduce(float a, float b, float &A, float &B,
     par ^= 1;
 }
 
-// loop over this thread's elements (lc, l) of the slab
-#define TVC_FOR(c) for (int lc = (c).lc0, l = lc * (c).N + (c).iz; lc < (c).nl; lc += (c).G, l += (c).G * (c).N)
-
-// CGS step structure (per step two cluster barriers, both inside the sums):
-//   uc = r + beta q ; p_new = uc + beta (q + beta p_old)     (local)
-//   __syncthreads ; vh = M p_new, halo p_new from the neighbour's r, q, p_old
-//   sum rt'vh -> alpha
-//   q = uc - alpha vh ; uh = uc + q ; x += alpha uh         (local)
-//   __syncthreads ; r -= alpha M uh, halo uh from the neighbour's uc, vh
-//   sum r'r, rt'r -> convergence, beta
-// p alternates between two buffers so that a neighbour can still read p_old
-// while this CTA writes p_new; every vector read remotely in a phase was
-// written before the barrier that opened the phase.
-__global__ void __launch_bounds__(TVC_THREADS, 2)
-    k_tv_prox_cl(const float *__restrict__ g_all, const TvState *__restrict__ st, double mu_const,
-                 int coupled, float *__restrict__ out_all, int N, int C, int nloc) {
-    namespace cg = cooperative_groups;
-    extern __shared__ float4 tvc_smem[];
-    __shared__ float wsum[64];
-    __shared__ float red[2 * TVC_MAXC * 2];
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank();
-    const int w = blockIdx.x / C, gw = coupled ? 0 : w;
-    if (st && st[gw].done) return;  // uniform over the cluster
-    TvcCtx c;
-    c.sm = reinterpret_cast<float *>(tvc_smem);
-    c.N = N;
-    c.nloc = nloc;
-    c.ix0 = rank * nloc;
-    c.nl = max(0, min(nloc, N - c.ix0));
-    c.G = TVC_THREADS / N;
-    c.iz = threadIdx.x % N;
-    c.lc0 = (int)threadIdx.x / N;
-    if (c.lc0 >= c.G) c.lc0 = c.nl;  // idle thread: empty loops
-    c.zlo = c.iz >= 1;
-    c.zhi = c.iz + 1 < N;
-    c.sl = rank > 0 ? cl.map_shared_rank(c.sm, rank - 1) : nullptr;
-    c.sr = rank + 1 < C ? cl.map_shared_rank(c.sm, rank + 1) : nullptr;
-    const float mu = (float)(st ? st[gw].mu : mu_const);
-    const float *g = g_all + (size_t)w * N * N + (size_t)c.ix0 * N;
-    const int V = nloc * N;
-    float *S = c.sm;
-    int ou = V_U * V, ox = V_X * V;  // swapped after every sweep
-    const int ob1 = V_B1 * V, ob2 = V_B2 * V, orr = V_R * V, ort = V_RT * V, oq = V_Q * V,
-              ouc = V_UC * V, ouh = V_UH * V, ovh = V_VH * V, oxm = V_XMIN * V;
-    int op = V_P0 * V, opo = V_P1 * V;  // p_new, p_old
-    int par = 0, n_sweeps = 0, n_cg = 0;
-    float A = 0.f, B = 0.f;
-    float n2b = 0.f, rho = 0.f, rho1 = 1.f, normrmin = 0.f;
-    TVC_FOR(c) {
-        S[ou + l] = g[l];
-        S[ob1 + l] = 0.f;
-        S[ob2 + l] = 0.f;
-    }
-    cl.sync();
-    for (int it = 0; it < TV_SB_MAX; ++it) {
-        ++n_sweeps;
-        // rhs = g - B'(b - d); r = rt = rhs; x = xmin = 0
-        float n2 = 0.f;
-        TVC_FOR(c) {
-            const int ix = c.ix0 + lc;
-            float b1, b2, c1, c2, t1, t2, e1, e2;
-            tvc_bd(S[ob1 + l], S[ob2 + l], mu, b1, b2, c1, c2);
-            float acc = 0.f;
-            if (c.zlo) acc += c1;
-            if (c.zhi) {
-                tvc_bd(S[ob1 + l + 1], S[ob2 + l + 1], mu, t1, t2, e1, e2);
-                acc -= e1;
-            }
-            float acc2 = 0.f;
-            if (ix >= 1) acc2 += c2;
-            if (ix + 1 < N) {
-                tvc_bd(tvc_right(c, ob1, lc, l), tvc_right(c, ob2, lc, l), mu, t1, t2, e1, e2);
-                acc2 -= e2;
-            }
-            const float rhs = g[l] - (acc + acc2);
-            S[orr + l] = rhs;
-            S[ort + l] = rhs;
-            S[ox + l] = 0.f;
-            S[oxm + l] = 0.f;
-            n2 = fmaf(rhs, rhs, n2);
-        }
-        tvc_reduce(n2, 0.f, A, B, wsum, red, par, C, rank);
-        n2b = sqrtf(A);
-        rho = A;  // rt' r of the first step (rt = r = rhs)
-        rho1 = 1.f;
-        normrmin = n2b;
-        float beta_next = 0.f;
-        bool converged = false;
-        if (n2b > 0.f) {
-            for (int cit = 0; cit < TV_CG_MAX; ++cit) {
-                ++n_cg;
-                const float beta = beta_next;
-                {
-                    const int t = op;
-                    op = opo;
-                    opo = t;
-                }
-                if (cit == 0) {
-                    TVC_FOR(c) {
-                        const float rv = S[orr + l];
-                        S[ouc + l] = rv;
-                        S[op + l] = rv;
-                    }
-                } else {
-                    TVC_FOR(c) {
-                        const float qv = S[oq + l];
-                        const float uv = fmaf(beta, qv, S[orr + l]);
-                        S[ouc + l] = uv;
-                        S[op + l] = fmaf(beta, fmaf(beta, S[opo + l], qv), uv);
-                    }
-                }
-                __syncthreads();  // p_new complete in this slab
-                const bool first = cit == 0;
-                const int opo_ = opo;
-                auto halo_p = [=](const float *b, int k) {
-                    const float rv = b[orr + k];
-                    if (first) return rv;
-                    const float qv = b[oq + k];
-                    const float uv = fmaf(beta, qv, rv);
-                    return fmaf(beta, fmaf(beta, b[opo_ + k], qv), uv);
-                };
-                float a_rtvh = 0.f;
-                TVC_FOR(c) {
-                    const float vhv = tvc_M(c, op, lc, l, halo_p);
-                    S[ovh + l] = vhv;
-                    a_rtvh = fmaf(S[ort + l], vhv, a_rtvh);
-                }
-                tvc_reduce(a_rtvh, 0.f, A, B, wsum, red, par, C, rank);
-                if (A == 0.f || !isfinite(A)) break;
-                const float alpha = rho / A;
-                TVC_FOR(c) {
-                    const float uv = S[ouc + l];
-                    const float qq = fmaf(-alpha, S[ovh + l], uv);
-                    S[oq + l] = qq;
-                    const float uh = uv + qq;
-                    S[ouh + l] = uh;
-                    S[ox + l] = fmaf(alpha, uh, S[ox + l]);
-                }
-                __syncthreads();  // uh complete in this slab
-                auto halo_uh = [=](const float *b, int k) {
-                    const float uv = b[ouc + k];
-                    return uv + fmaf(-alpha, b[ovh + k], uv);
-                };
-                float a_rr = 0.f, a_rtr = 0.f;
-                TVC_FOR(c) {
-                    const float rv = fmaf(-alpha, tvc_M(c, ouh, lc, l, halo_uh), S[orr + l]);
-                    S[orr + l] = rv;
-                    a_rr = fmaf(rv, rv, a_rr);
-                    a_rtr = fmaf(S[ort + l], rv, a_rtr);
-                }
-                tvc_reduce(a_rr, a_rtr, A, B, wsum, red, par, C, rank);
-                int f = 0;
-                {
-                    const float normr = sqrtf(A);
-                    if (normr <= 1e-5f * n2b) {
-                        f = TVB_CONVERGED;
-                    } else {
-                        if (normr < normrmin) {
-                            normrmin = normr;
-                            f |= TVB_IMPROVED;
-                        }
-                        rho1 = rho;
-                        rho = B;  // rt' r of the next step
-                        if (rho == 0.f || !isfinite(rho))
-                            f |= TVB_BREAK;
-                        else
-                            beta_next = rho / rho1;
-                    }
-                }
-                if (f & TVB_CONVERGED) {
-                    converged = true;
-                    break;
-                }
-                if (f & TVB_IMPROVED) {
-                    TVC_FOR(c) S[oxm + l] = S[ox + l];
-                }
-                if (f & TVB_BREAK) break;
-            }
-        }
-        if (!converged) {
-            TVC_FOR(c) S[ox + l] = S[oxm + l];
-        }
-        cl.sync();  // new u (in x) complete in every slab
-        // Bub = B u + b ; change of u
-        float dif = 0.f, nrm = 0.f;
-        TVC_FOR(c) {
-            float b1, b2, c1, c2;
-            tvc_bd(S[ob1 + l], S[ob2 + l], mu, b1, b2, c1, c2);
-            const float v = S[ox + l];
-            S[ob1 + l] = (c.zlo ? v - S[ox + l - 1] : 0.f) + b1;
-            S[ob2 + l] = (c.ix0 + lc >= 1 ? v - tvc_left(c, ox, lc, l) : 0.f) + b2;
-            const float e = S[ou + l] - v;
-            dif = fmaf(e, e, dif);
-            nrm = fmaf(v, v, nrm);
-        }
-        tvc_reduce(dif, nrm, A, B, wsum, red, par, C, rank);
-        const bool stop = !(B > 0.f) || sqrtf(A / B) <= 1e-3f;
-        const int t = ou;
-        ou = ox;
-        ox = t;
-        if (stop) break;
-    }
-    float *o = out_all + (size_t)w * N * N + (size_t)c.ix0 * N;
-    TVC_FOR(c) o[l] = S[ou + l];
-    if (rank == 0 && threadIdx.x == 0) {
-        atomicAdd(&g_tv_stats[0], (unsigned long long)n_sweeps);
-        atomicAdd(&g_tv_stats[1], (unsigned long long)n_cg);
-    }
-    cl.sync();  // no CTA leaves while a neighbour may still read its shared memory
-}
-#undef TVC_FOR
-
-// ---------------------------------------------------------------------------
-// The same cluster prox with 4 consecutive z-pixels per thread (N % 4 == 0):
-// 128-bit shared-memory accesses; thread t owns group jz = t % (N/4) (pixels
-// 4 jz .. 4 jz + 3) of the columns lc = t / (N/4), ... + G.  The split-Bregman
-// sweep is the scalar kernel's; its CGS step is the same recurrence written
-// with one CTA barrier less, carrying M p and M q instead of p and uh (M =
-// I + B'B is linear, so M p_new = M uc + beta (M q + beta M p_old) and
-// M uh = M uc + M q, M q = M uc - alpha M vh):
+// The cluster prox: 4 consecutive z-pixels per thread, columns padded to P =
+// N rounded up to 4 (the pad pixels stay 0), 128-bit shared-memory accesses;
+// thread t owns group jz = t % (P/4) (pixels 4 jz .. 4 jz + 3) of the columns
+// lc = t / (P/4), ... + G.  Its CGS step carries M p and M q instead of p and
+// uh (M = I + B'B is linear, so M p_new = M uc + beta (M q + beta M p_old) and
+// M uh = M uc + M q, M q = M uc - alpha M vh), which saves a CTA barrier.
+// Sides that are no multiple of 4 had a kernel of a pixel per thread: 28 images
+// of 199 x 199 2.77 ms, now 1.13; 81 x 81 0.57, now 0.45:
 //   A  uc = r + beta q                                        (local)
 //      __syncthreads
 //   B  Muc = M uc (halo uc from the neighbour's r, q); vh = Muc + beta (Mq +
@@ -629,16 +381,16 @@ __global__ void __launch_bounds__(TVC_THREADS, 2)
 //   C  Mvh = M vh (halo vh from the neighbour); q = uc - alpha vh;
 //      Mq = Muc - alpha Mvh; x += alpha (uc + q); r -= alpha (Muc + Mq);
 //      sums r'r, rt'r -> convergence, beta
-// Two stencils and two cluster sums per step, as before; every vector read
+// Two stencils and two cluster sums per step; every vector read
 // remotely in a phase was written before the cluster barrier that opened
 // it, and is rewritten only after the next one.
 //
 // KM > 0: a thread owns at most KM groups and keeps the vectors that no other
 // thread reads (rt, M uc, M q) in registers: nine vectors of shared memory
-// instead of thirteen, so that larger images fit a smaller cluster, which
+// instead of twelve, so that larger images fit a smaller cluster, which
 // matters because the barriers and not the pixels bound a step: an image of
 // 200 x 200 takes 0.53 ms with 16 CTAs and 0.58 with 8 (with thirteen vectors
-// it needed the 16: 0.57), and twice as many clusters of 8 run at once --
+// in shared memory it needed the 16: 0.57), and twice as many clusters of 8 run at once --
 // 8 images 0.60 ms (was 1.01), 28 images 1.06 (was 1.90).  One CTA per SM
 // and 128 registers; KM = 4 spills a little (160 x 160 px: 0.72 ms with
 // 4 CTAs, 0.48 with 8 and KM = 2).
@@ -657,7 +409,7 @@ __device__ __forceinline__ void st4(float *p, const F4 &a) {
 struct Tvc4Ctx {
     float *sm;
     const float *sl, *sr;
-    int N, nloc, nl, ix0, iz0, G, lc0;
+    int N, P, nloc, nl, ix0, iz0, G, lc0;  // P: N rounded up to 4, a column's stride
 };
 
 // a neighbour slab's float4: shared memory of the neighbour CTA, or (GM)
@@ -672,8 +424,9 @@ __device__ __forceinline__ F4 ld4n(const float *p) {
     }
 }
 
-// (I + B'B) in of the 4 pixels at (lc, iz0 .. iz0 + 3), element l = lc N + iz0
-template <class Halo>
+// (I + B'B) in of the 4 pixels at (lc, iz0 .. iz0 + 3), element l = lc P + iz0;
+// RAG: pixels beyond the column's N are kept 0
+template <bool RAG, class Halo>
 __device__ __forceinline__ F4 tvc4_M(const Tvc4Ctx &c, int oi, int lc, int l, Halo halo) {
     const float *in = c.sm + oi;
     const int ix = c.ix0 + lc;
@@ -684,8 +437,8 @@ __device__ __forceinline__ F4 tvc4_M(const Tvc4Ctx &c, int oi, int lc, int l, Ha
     for (int k = 0; k < 4; ++k) a[k + 1] = v.v[k];
     a[5] = c.iz0 + 4 < c.N ? in[l + 4] : 0.f;
     F4 L{}, R{};
-    if (ix >= 1) L = lc == 0 ? halo(c.sl, (c.nloc - 1) * c.N + c.iz0) : ld4(in + l - c.N);
-    if (ix + 1 < c.N) R = lc == c.nl - 1 ? halo(c.sr, c.iz0) : ld4(in + l + c.N);
+    if (ix >= 1) L = lc == 0 ? halo(c.sl, (c.nloc - 1) * c.P + c.iz0) : ld4(in + l - c.P);
+    if (ix + 1 < c.N) R = lc == c.nl - 1 ? halo(c.sr, c.iz0) : ld4(in + l + c.P);
     F4 o;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -695,24 +448,24 @@ __device__ __forceinline__ F4 tvc4_M(const Tvc4Ctx &c, int oi, int lc, int l, Ha
         const float g1n = iz + 1 < c.N ? a[k + 2] - x : 0.f;
         const float g2 = ix >= 1 ? x - L.v[k] : 0.f;
         const float g2n = ix + 1 < c.N ? R.v[k] - x : 0.f;
-        o.v[k] = x + (g1 - g1n) + (g2 - g2n);
+        o.v[k] = RAG && iz >= c.N ? 0.f : x + (g1 - g1n) + (g2 - g2n);
     }
     return o;
 }
 
 // loop over this thread's groups e (lc, l); KU copies of the body
 #define TVC4_FOR(c)                                                                        \
-    _Pragma("unroll KU") for (int e = 0, lc = (c).lc0, l = lc * (c).N + (c).iz0;           \
+    _Pragma("unroll KU") for (int e = 0, lc = (c).lc0, l = lc * (c).P + (c).iz0;           \
                               KM ? e < KM : lc < (c).nl;                                   \
-                              ++e, lc += (c).G, l += (c).G * (c).N) if (!KM || lc < (c).nl)
+                              ++e, lc += (c).G, l += (c).G * (c).P) if (!KM || lc < (c).nl)
 
-template <bool GM, int KM>
+template <bool GM, int KM, bool RAG>
 __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
     k_tv_prox_cl4(const float *__restrict__ g_all, const TvState *__restrict__ st,
                   double mu_const, int coupled, float *__restrict__ out_all, int N, int C,
                   int nloc, float *__restrict__ gwork) {
     namespace cg = cooperative_groups;
-    static_assert(!GM || KM == 0, "global vectors: none in registers");
+    static_assert(!GM || (KM == 0 && !RAG), "global vectors: none in registers, N % 4 == 0");
     constexpr int KU = KM ? KM : 1;
     extern __shared__ float4 tvc_smem[];
     __shared__ float wsum[64];
@@ -726,14 +479,15 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
     c.nloc = nloc;
     c.ix0 = rank * nloc;
     c.nl = max(0, min(nloc, N - c.ix0));
-    const int NG = N / 4;
+    const int P = RAG ? (N + 3) / 4 * 4 : N, NG = P / 4;
+    c.P = P;
     c.G = TVC_THREADS / NG;
     c.iz0 = 4 * ((int)threadIdx.x % NG);
     c.lc0 = (int)threadIdx.x / NG;
     if (c.lc0 >= c.G) c.lc0 = c.nl;  // idle thread
     if constexpr (GM) {
         // slabs of the cluster's CTAs are consecutive in the workspace
-        const size_t slab = (size_t)TVC_NV * nloc * N;
+        const size_t slab = (size_t)TVC_NV * nloc * P;
         c.sm = gwork + ((size_t)w * C + rank) * slab;
         c.sl = rank > 0 ? c.sm - slab : nullptr;
         c.sr = rank + 1 < C ? c.sm + slab : nullptr;
@@ -744,13 +498,13 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
     }
     const float mu = (float)(st ? st[gw].mu : mu_const);
     const float *g = g_all + (size_t)w * N * N + (size_t)c.ix0 * N;
-    const int V = nloc * N;
+    const int V = nloc * P;
     float *S = c.sm;
     int ou = V_U * V, ox = V_X * V;
     const int ob1 = V_B1 * V, ob2 = V_B2 * V, orr = V_R * V, oq = (KM ? 5 : V_Q) * V,
               ouc = (KM ? 6 : V_UC) * V, ovh = (KM ? 7 : V_VH) * V, oxm = (KM ? 8 : V_XMIN) * V;
     // rt, M q and M uc (no p, no uh here): in registers with KM
-    const int ort = V_RT * V, omq = V_P0 * V, omuc = V_P1 * V;
+    const int ort = V_RT * V, omq = V_MQ * V, omuc = V_MUC * V;
     F4 rrt[KU], rmq[KU], rmuc[KU];
     auto put = [&](F4 &reg, int o, const F4 &v) {
         if constexpr (KM > 0)
@@ -768,8 +522,19 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
     float A = 0.f, B = 0.f;
     float n2b = 0.f, rho = 0.f, rho1 = 1.f, normrmin = 0.f;
     const F4 zero4{{0.f, 0.f, 0.f, 0.f}};
+    auto image = [&](int lc, int l) {  // the input's four pixels
+        if constexpr (RAG) {
+            F4 v;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                v.v[k] = c.iz0 + k < N ? g[(size_t)lc * N + c.iz0 + k] : 0.f;
+            return v;
+        } else {
+            return ld4(g + l);
+        }
+    };
     TVC4_FOR(c) {
-        st4(S + ou + l, ld4(g + l));
+        st4(S + ou + l, image(lc, l));
         st4(S + ob1 + l, zero4);
         st4(S + ob2 + l, zero4);
     }
@@ -779,7 +544,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
         float n2 = 0.f;
         TVC4_FOR(c) {
             const int ix = c.ix0 + lc;
-            const F4 B1 = ld4(S + ob1 + l), B2 = ld4(S + ob2 + l), G4 = ld4(g + l);
+            const F4 B1 = ld4(S + ob1 + l), B2 = ld4(S + ob2 + l), G4 = image(lc, l);
             float c1[5], c2[4];
             for (int k = 0; k < 4; ++k) {
                 float b1, b2;
@@ -793,8 +558,8 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
             }
             float e2r[4] = {0.f, 0.f, 0.f, 0.f};
             if (ix + 1 < N) {
-                const F4 R1 = lc == c.nl - 1 ? ld4n<GM>(c.sr + ob1 + c.iz0) : ld4(S + ob1 + l + N);
-                const F4 R2 = lc == c.nl - 1 ? ld4n<GM>(c.sr + ob2 + c.iz0) : ld4(S + ob2 + l + N);
+                const F4 R1 = lc == c.nl - 1 ? ld4n<GM>(c.sr + ob1 + c.iz0) : ld4(S + ob1 + l + P);
+                const F4 R2 = lc == c.nl - 1 ? ld4n<GM>(c.sr + ob2 + c.iz0) : ld4(S + ob2 + l + P);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     float b1, b2, e1;
@@ -811,7 +576,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
                 float acc2 = 0.f;
                 if (ix >= 1) acc2 += c2[k];
                 if (ix + 1 < N) acc2 -= e2r[k];
-                rh.v[k] = G4.v[k] - (acc + acc2);
+                rh.v[k] = RAG && iz >= N ? 0.f : G4.v[k] - (acc + acc2);
                 n2 = fmaf(rh.v[k], rh.v[k], n2);
             }
             st4(S + orr + l, rh);
@@ -858,7 +623,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
                 };
                 float a_rtvh = 0.f;
                 TVC4_FOR(c) {
-                    const F4 muc = tvc4_M(c, ouc, lc, l, halo_uc);
+                    const F4 muc = tvc4_M<RAG>(c, ouc, lc, l, halo_uc);
                     put(rmuc[KM ? e : 0], omuc + l, muc);
                     F4 vh = muc;
                     if (!first) {
@@ -880,7 +645,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
                 auto halo_vh = [=](const float *b, int k) { return ld4n<GM>(b + ovh + k); };
                 float a_rr = 0.f, a_rtr = 0.f;
                 TVC4_FOR(c) {
-                    const F4 mv = tvc4_M(c, ovh, lc, l, halo_vh);
+                    const F4 mv = tvc4_M<RAG>(c, ovh, lc, l, halo_vh);
                     const F4 uv = ld4(S + ouc + l), vh = ld4(S + ovh + l);
                     const F4 muc = get(rmuc[KM ? e : 0], omuc + l);
                     const F4 xv = ld4(S + ox + l), rv = ld4(S + orr + l);
@@ -944,7 +709,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
             for (int k = 0; k < 4; ++k) xa[k + 1] = X.v[k];
             F4 Lx{};
             if (ix >= 1)
-                Lx = lc == 0 ? ld4n<GM>(c.sl + ox + (c.nloc - 1) * N + c.iz0) : ld4(S + ox + l - N);
+                Lx = lc == 0 ? ld4n<GM>(c.sl + ox + (c.nloc - 1) * P + c.iz0) : ld4(S + ox + l - P);
             F4 n1, n2v;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -953,6 +718,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
                 const float v = X.v[k];
                 n1.v[k] = (c.iz0 + k >= 1 ? v - xa[k] : 0.f) + b1;
                 n2v.v[k] = (ix >= 1 ? v - Lx.v[k] : 0.f) + b2;
+                if (RAG && c.iz0 + k >= N) n1.v[k] = n2v.v[k] = 0.f;
                 const float e = U.v[k] - v;
                 dif = fmaf(e, e, dif);
                 nrm = fmaf(v, v, nrm);
@@ -968,7 +734,16 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
         if (stop) break;
     }
     float *o = out_all + (size_t)w * N * N + (size_t)c.ix0 * N;
-    TVC4_FOR(c) st4(o + l, ld4(S + ou + l));
+    TVC4_FOR(c) {
+        const F4 v = ld4(S + ou + l);
+        if constexpr (RAG) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (c.iz0 + k < N) o[(size_t)lc * N + c.iz0 + k] = v.v[k];
+        } else {
+            st4(o + l, v);
+        }
+    }
     if (rank == 0 && threadIdx.x == 0) {
         atomicAdd(&g_tv_stats[0], (unsigned long long)n_sweeps);
         atomicAdd(&g_tv_stats[1], (unsigned long long)n_cg);
@@ -1227,11 +1002,11 @@ constexpr int TVC_KM = 4;                                     // most groups in 
 // the geometry with C CTAs per image, C = 0 in it if the image does not fit
 TvcGeom tvc_fit(int N, int C) {
     TvcGeom g;
-    const int nloc = (N + C - 1) / C;
-    size_t bytes = (size_t)TVC_NV * nloc * N * sizeof(float);
-    if (bytes > TVC_TWO && N % 4 == 0) {
-        const int G = TVC_THREADS / (N / 4), km = std::max(2, (nloc + G - 1) / G);
-        const size_t few = (size_t)TVC_NV_REG * nloc * N * sizeof(float);
+    const int nloc = (N + C - 1) / C, P = (N + 3) / 4 * 4;
+    size_t bytes = (size_t)TVC_NV * nloc * P * sizeof(float);
+    if (bytes > TVC_TWO) {
+        const int G = TVC_THREADS / (P / 4), km = std::max(2, (nloc + G - 1) / G);
+        const size_t few = (size_t)TVC_NV_REG * nloc * P * sizeof(float);
         if (km <= TVC_KM && few <= TVC_ONE) {
             g.KM = km;
             bytes = few;
@@ -1257,8 +1032,10 @@ TvcGeom tvc_geometry(int N, int W, int force = 0) {
     if (const int Cf = force ? force : g_tv_cluster.load())
         // negative: no shared-memory geometry, the global-memory form
         return Cf < 0 ? TvcGeom() : tvc_fit(N, Cf);
-    for (int C = 1; C <= 8; C *= 2)
-        if ((size_t)TVC_NV * ((N + C - 1) / C) * N * sizeof(float) <= TVC_TWO) return tvc_fit(N, C);
+    for (int C = 1; C <= 8; C *= 2) {
+        const TvcGeom g = tvc_fit(N, C);
+        if (g.C && g.KM == 0 && g.smem <= TVC_TWO) return g;
+    }
     TvcGeom best, smallest;
     double cost = 1e30;
     for (int C = 16; C >= 1; C /= 2) {
@@ -1276,8 +1053,9 @@ TvcGeom tvc_geometry(int N, int W, int force = 0) {
     return best.C ? best : smallest;
 }
 
-template <class K>
-static cudaError_t tvc_config(K kern, const TvcGeom &gm, int W, cudaStream_t st,
+using TvcKernel = void (*)(const float *, const TvState *, double, int, float *, int, int, int,
+                           float *);
+static cudaError_t tvc_config(TvcKernel kern, const TvcGeom &gm, int W, cudaStream_t st,
                               cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int &clusters) {
     clusters = 0;
     cudaError_t e = raise_max_dynamic_smem((const void *)kern, gm.smem);
@@ -1305,16 +1083,17 @@ static cudaError_t tvc_config(K kern, const TvcGeom &gm, int W, cudaStream_t st,
     return cudaSuccess;
 }
 
-// the kernel of a geometry for N % 4 == 0: 4 z-pixels per thread
-using TvcKernel4 = void (*)(const float *, const TvState *, double, int, float *, int, int, int,
-                            float *);
-TvcKernel4 tvc_kernel4(const TvcGeom &g) {
+template <bool RAG>
+TvcKernel tvc_kernel(const TvcGeom &g) {
     switch (g.KM) {
-    case 2: return k_tv_prox_cl4<false, 2>;
-    case 3: return k_tv_prox_cl4<false, 3>;
-    case 4: return k_tv_prox_cl4<false, 4>;
-    default: return k_tv_prox_cl4<false, 0>;
+    case 2: return k_tv_prox_cl4<false, 2, RAG>;
+    case 3: return k_tv_prox_cl4<false, 3, RAG>;
+    case 4: return k_tv_prox_cl4<false, 4, RAG>;
+    default: return k_tv_prox_cl4<false, 0, RAG>;
     }
+}
+TvcKernel tvc_kernel(const TvcGeom &g, int N) {
+    return N % 4 ? tvc_kernel<true>(g) : tvc_kernel<false>(g);
 }
 
 // clusters of a geometry that the GPU runs at once, 0 if it cannot run it
@@ -1322,10 +1101,7 @@ int tvc_active(const TvcGeom &g, int N) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[1];
     int n = 0;
-    const cudaError_t e =
-        N % 4 == 0 ? tvc_config(tvc_kernel4(g), g, 1, nullptr, cfg, at, n)
-                   : tvc_config(k_tv_prox_cl, g, 1, nullptr, cfg, at, n);
-    return e == cudaSuccess ? n : 0;
+    return tvc_config(tvc_kernel(g, N), g, 1, nullptr, cfg, at, n) == cudaSuccess ? n : 0;
 }
 
 cudaError_t tvc_launch(const TvcGeom &gm, const float *z, const TvState *sv, double mu,
@@ -1333,21 +1109,13 @@ cudaError_t tvc_launch(const TvcGeom &gm, const float *z, const TvState *sv, dou
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at[1];
     int clusters = 0;
-    // 4 z-pixels per thread where N allows (16-byte aligned groups)
-    if (N % 4 == 0 && N / 4 <= TVC_THREADS) {
-        const TvcKernel4 kern = tvc_kernel4(gm);
-        cudaError_t e = tvc_config(kern, gm, W, st, cfg, at, clusters);
-        fits = clusters > 0;
-        if (e != cudaSuccess || !fits) return e;
-        ++g_launch_count;
-        return cudaLaunchKernelEx(&cfg, kern, z, sv, mu, coupled, out, N, gm.C, gm.nloc,
-                                  (float *)nullptr);
-    }
-    cudaError_t e = tvc_config(k_tv_prox_cl, gm, W, st, cfg, at, clusters);
+    const TvcKernel kern = tvc_kernel(gm, N);
+    const cudaError_t e = tvc_config(kern, gm, W, st, cfg, at, clusters);
     fits = clusters > 0;
     if (e != cudaSuccess || !fits) return e;
     ++g_launch_count;
-    return cudaLaunchKernelEx(&cfg, k_tv_prox_cl, z, sv, mu, coupled, out, N, gm.C, gm.nloc);
+    return cudaLaunchKernelEx(&cfg, kern, z, sv, mu, coupled, out, N, gm.C, gm.nloc,
+                              (float *)nullptr);
 }
 
 // cluster of 16 CTAs per image with the work vectors in `work` (L2-resident)
@@ -1360,7 +1128,7 @@ cudaError_t tvc_launch_gm(const float *z, const TvState *sv, double mu, int coup
     // the slabs must fit the workspace of TV_NVEC vectors per image
     if (N % 4 != 0 || N / 4 > TVC_THREADS || (size_t)C * TVC_NV * nloc > (size_t)TV_NVEC * N)
         return cudaSuccess;
-    auto kern = k_tv_prox_cl4<true, 0>;
+    auto kern = k_tv_prox_cl4<true, 0, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};

@@ -1,6 +1,7 @@
-"""SB_ITV2 with part of its vectors in registers: clusters of 4, 8 and 16 CTAs
-with two to four groups of pixels per thread, slabs that end ragged, threads
-that own fewer groups than the others."""
+"""SB_ITV2 by thread-block clusters, with part of its vectors in registers
+(clusters of 4, 8 and 16 CTAs with two to four groups of pixels per thread) and
+without: slabs that end ragged, threads that own fewer groups than the others,
+columns that do not fill their last group of four pixels."""
 import numpy as np
 import pytest
 
@@ -16,7 +17,9 @@ pytestmark = pytest.mark.gpu
 # images of one call do not influence each other
 @pytest.mark.parametrize("n,W,C", [(132, 1, 4), (148, 2, 4), (160, 1, 4), (160, 1, 8),
                                    (172, 1, 8), (200, 1, 8), (200, 9, 0), (236, 1, 16),
-                                   (256, 1, 16), (160, 20, 0)])
+                                   (256, 1, 16), (160, 20, 0),
+                                   (3, 2, 0), (6, 1, 2), (97, 3, 0), (143, 1, 4), (161, 1, 8),
+                                   (199, 2, 0), (201, 10, 0), (235, 1, 16), (302, 1, 0)])
 def test_sb_itv2_with_vectors_in_registers(cuda, n, W, C):
     import torch
     from msot_gb300 import SB_ITV2, _lib

@@ -405,6 +405,9 @@ typedef struct msot_tuning {
     int adj_wt;                               /* instances per CTA of the DAS adjoint (4, 2, 1) */
     int fwd_staged;                           /* DAS forward: 1 staged, 2 per-detector buckets,
                                                  4 per-detector buckets, interleaved entries */
+    /* fwd_wt, adj_wt and fwd_staged name the best of the listed kernels; the plan
+     * takes them only where they beat the kernel it runs without tuning, which for
+     * batches is one with lanes over instances */
 } msot_tuning;
 int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tuning *out);
 

@@ -11,9 +11,9 @@
 //
 // The lanes of a pixel hold NI instances, four each, so a row read is
 // NI x 4 contiguous bytes: a 128-bit load of a warp takes 4 shared wavefronts
-// at NI = 32 and 6 at NI = 16 (two random rows per 8 lanes), where the table with one or two instances per
-// thread (k_das_adj4: lanes over pixels, random 16-byte rows) paid about 10 for
-// a quarter of the values.  (pixel, detector) pairs come as 4 bytes, knot row
+// at NI = 32 and 6 at NI = 16 (two random rows per 8 lanes), where the table
+// with one or two instances per thread (k_das_adj4: lanes over pixels, random
+// 16-byte rows) paid about 10 for a quarter of the values.  (pixel, detector) pairs come as 4 bytes, knot row
 // and g in fixed point, decoded once per 4 NI values.  Measured at batch 64,
 // 128 x 128 px, 256 detectors: 322 us (k_das_adj4) -> 211 us (NI = 32).
 //

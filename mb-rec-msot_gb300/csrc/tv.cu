@@ -281,9 +281,9 @@ __global__ void __launch_bounds__(TV_THREADS)
 
 // ---------------------------------------------------------------------------
 // Cluster-resident prox: one thread-block cluster of C CTAs per image, CTA
-// `rank` owning the column slab ix in [rank*nloc, rank*nloc + nl).  All
-// eleven work vectors of the split-Bregman + CGS iteration live in shared
-// memory (same layout in every CTA); the stencil's x-neighbours in the
+// `rank` owning the column slab ix in [rank*nloc, rank*nloc + nl).  The
+// work vectors of the split-Bregman + CGS iteration (TVC_NV, or TVC_NV_REG)
+// live in shared memory (same layout in every CTA); the stencil's x-neighbours in the
 // adjacent slabs are read through distributed shared memory.  Cluster-wide
 // sums: every CTA adds the C per-CTA partials in rank order, so all CTAs
 // see bitwise-identical scalars and take identical branches.

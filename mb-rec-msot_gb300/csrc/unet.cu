@@ -161,10 +161,10 @@ __global__ void __launch_bounds__(256) k_conv3_in(const float *__restrict__ in,
 // exact in TF32.  Every wait is bounded: on a timeout the CTA sets *err,
 // skips its stores and still frees its TMEM.
 // ---------------------------------------------------------------------------
-constexpr int TC_TY = 8, TC_TX = 16;              // pixel tile (M = 128)
+constexpr int TC_TY = 8, TC_TX = 16;              // the weight gradient's pixel tile
 constexpr int TC_CK = 32;                         // input channels per stage
-constexpr int TC_HY = TC_TY + 2;                  // halo rows
-constexpr int TC_THREADS = 256;                   // of the weight gradient
+constexpr int TC_HY = TC_TY + 2;                  // its halo rows
+constexpr int TC_THREADS = 256;                   // its threads
 constexpr int TC_H = 16, TC_W = 8;                // the convolution's pixel tile (M = 128)
 constexpr int TC_WY = TC_H + 2;                   // its window
 constexpr int TC_WX = TC_W + 2;

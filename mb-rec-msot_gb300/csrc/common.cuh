@@ -143,6 +143,7 @@ struct Plan {
     int sir_span_max = 0;
     int32_t *sir_off = nullptr;    // [D][sir_nj + 1] forward pairs per window start
     int sir_jmin = 0, sir_nj = 0, sir_maxlen = 0;
+    double sir_len_mean = 0.0;     // samples of a (pixel, detector)'s column on average
     // scratch for the operator chains
     int max_batch = 0;
     float *scr_img0 = nullptr, *scr_img1 = nullptr;  // [max_batch][P]

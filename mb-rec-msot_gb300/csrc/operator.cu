@@ -1407,12 +1407,26 @@ static int sir_adj_nt(const Plan &pl, const float *raw, float *x, float scale, d
     return MSOT_EINVAL;
 }
 
+// k_sir_adj2 instead of k_sir_adj for W instances.  k_sir_adj runs the tri taps
+// for every sample of a column, a pass per two instances (0.565 of one per
+// single instance when W is odd): 4 + 0.0445 x mean column length x taps ns
+// per pixel and pass, 256 detectors.  k_sir_adj2 reads a window in rounds of 16
+// taps, much the same for every column: 30.5 ns per pixel for up to four
+// instances, 36.5 per eight.  k_sir_adj / k_sir_adj2 measured, 128^2 px (columns
+// of 31 samples, 12 taps): 357 / 460 us for two images, 591 / 465 for three,
+// 1184 / 626 for eight; 160^2 (26, 10): 688 / 758 for three, 860 / 760 for four;
+// 200^2 (22, 8): 823 / 1139 for three, 1578 / 1471 for eight.
+static bool sir_adj_composite(const Plan &pl, int W) {
+    if (!pl.sir_tab) return false;
+    const double pass = 4.0 + 0.0445 * pl.sir_len_mean * (2 * pl.F + 2);
+    const double there = W <= 4 ? 30.5 : 36.5 * div_up(W, 8);
+    return there <= pass * (W % 2 ? 0.565 : 0.5) * W;
+}
+
 int launch_sir_adjoint(const Plan &pl, const float *raw, float *x, int W, float scale,
                        cudaStream_t st) {
     TimedScope ts_(KID_INTERP_ADJ, st);
-    // 128 x 128 px: 220 / 356 us here for one / two images against 450 / 460 us with
-    // a half warp per pixel, 591 against 465 for three
-    if (pl.sir_tab && W >= 3) return launch_sir_adjoint2(pl, raw, x, W, scale, st);
+    if (sir_adj_composite(pl, W)) return launch_sir_adjoint2(pl, raw, x, W, scale, st);
     const int wt = pick_wt(W, 1, 2);
     dim3 grid(pl.n_patch, W / wt);
     if (wt == 2) return sir_adj_nt<2>(pl, raw, x, scale, grid, st);

@@ -313,12 +313,15 @@ int sir_build(Plan &p, const int32_t *tfx, const int32_t *sidx, const std::vecto
     auto start = [&](int32_t tau, int s) { return (tau >> p.frac_bits) - half - F + se[s].x; };
     const size_t PD = (size_t)p.P * p.D;
     int jmin = INT_MAX, jmax = INT_MIN, maxlen = 0;
+    double sum = 0.0;
     for (size_t i = 0; i < PD; ++i) {
         const int s = sidx[i] - 1, j = start(tfx[i], s);
         jmin = std::min(jmin, j);
         jmax = std::max(jmax, j);
         maxlen = std::max(maxlen, se[s].y - se[s].x + 2 * F + 2);
+        sum += se[s].y - se[s].x + 1;
     }
+    p.sir_len_mean = sum / (double)PD;
     if (jmin < -32000 || jmax > 32000) return MSOT_OK;
     const int nj = jmax - jmin + 1;
     auto entry = [&](int32_t tau, int s, int pix) {
@@ -425,7 +428,7 @@ int launch_sir_adjoint2(const Plan &pl, const float *raw, float *x, int W, float
         if ((rc = set_smem(k_sir_adj2<NI>, smem)) != MSOT_OK) return rc;                   \
         KLAUNCH(k_sir_adj2<NI><<<grid, SA_THREADS, smem, st>>>(                            \
             pl.sir_aent, pl.sir_aspan, pl.sir_tab, raw, pl.scr_part, pl.P, pl.D, pl.T, W,  \
-            pl.sir_span_max, dpg, stride));                                                      \
+            pl.sir_span_max, dpg, stride));                                                \
     } while (0)
     if (ni == 8) SIRA(8);
     else SIRA(4);

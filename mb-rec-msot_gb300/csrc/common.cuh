@@ -115,13 +115,11 @@ struct Plan {
     // register pair m and lane, (re a, re b, im a, im b) of w^(lane k1) for
     // k1 = brev5(2m), brev5(2m + 1); conj w^(lane n) for n = 2m, 2m + 1; and
     // H[lane + 32 k2] for k2 = brev5(2m), brev5(2m + 1)  ([16][32] each)
-    // support of the interpolation per detector, [first, last + 1) samples over
-    // the taps of its pixels (SIR: the whole row), and the 1024-point
-    // convolution's tiles per column pair that it needs, forward and transpose
-    int2 *conv_rng = nullptr;
-    int conv_nt_f = 0, conv_nt_a = 0;
-    int conv_diff = 0;  // fft_hfb holds the spectrum of the taps' running sum
     float4 *fft_twb = nullptr, *fft_twn = nullptr, *fft_hfb = nullptr, *fft_hab = nullptr;
+    // support of the interpolation per detector, [first, last + 1) samples over
+    // the taps of its pixels and its neighbours' (SIR: the whole row), for the
+    // 1024-point convolution
+    int2 *conv_rng = nullptr;
     // prefilter
     int Kx = -1, Kz = -1;   // -1: no prefilter along that axis
     float *pre_x = nullptr, *pre_z = nullptr;

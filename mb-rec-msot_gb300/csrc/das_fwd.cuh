@@ -250,22 +250,15 @@ __global__ void __launch_bounds__(256, WT >= 16 ? 2 : 4) k_das_fwd3(const int32_
     for (int i = 0; i < WT; ++i) {
         const float *M0 = mom + (0 * WT + i) * NB + base;
         const float *M1 = mom + (1 * WT + i) * NB + base;
-        // four chains, the small outer taps first: the rounding of one chain
-        // over all 4F + 2 terms was the larger part of A's error (1.2e-6 of
-        // A x at 128 x 128 px, now 0.7e-6)
-        float u0 = mom[(2 * WT + i) * NB + base + F], u1 = mom[(3 * WT + i) * NB + base - F - 1];
-        float v0 = 0.f, v1 = 0.f;
+        // one chain in this order, here and in k_das_fwd6: the iterative solves
+        // amplify another rounding to 1e-3 of an image's rms at single pixels
+        float acc = mom[(2 * WT + i) * NB + base + F] + mom[(3 * WT + i) * NB + base - F - 1];
 #pragma unroll
-        for (int k = F - 1; k >= 0; --k) {
-            u0 = fmaf(1.f - (float)k * inv_r, M0[k], u0);
-            v0 += M1[k];
+        for (int k = -(F - 1); k <= F; ++k) {
+            const float a = 1.f - (float)(k < 0 ? -k : k) * inv_r;
+            acc = fmaf(a, M0[-k], acc);
+            acc = fmaf(k <= 0 ? -inv_r : inv_r, M1[-k], acc);
         }
-#pragma unroll
-        for (int k = F; k >= 1; --k) {
-            u1 = fmaf(1.f - (float)k * inv_r, M0[-k], u1);
-            v1 += M1[-k];
-        }
-        const float acc = fmaf(v1 - v0, inv_r, u0 + u1);
         if (w0 + i < W)
             raw[((size_t)(w0 + i) * D + d) * T + t] =
                 acc * (inv_s ? scale * __ldg(inv_s + w0 + i) : scale);

@@ -148,29 +148,23 @@ __global__ void __launch_bounds__(F6_THREADS, F <= 2 ? 2 : 3) k_das_fwd6(
         }
     }
     __syncthreads();
-    // the filter over the moments (four chains, the small outer taps first)
+    // the filter over the moments, the chain of k_das_fwd3
     const int d = d0 + di % DG, t = t0 + bi;
     if (bi >= TB || t >= T || d >= D) return;
     const int base = (di % DG) * F6_NB + bi + F + 1;  // bucket t
-#pragma unroll 2
+#pragma unroll 4
     for (int i = di / DG; i < NI; i += F6_THREADS / F6_NB / DG) {
         if (w0 + i >= W) break;
         const float *M0 = mom + (size_t)(0 * NI + i) * ROW + base;
         const float *M1 = mom + (size_t)(1 * NI + i) * ROW + base;
-        float u0 = mom[(size_t)(2 * NI + i) * ROW + base + F];
-        float u1 = mom[(size_t)(3 * NI + i) * ROW + base - F - 1];
-        float v0 = 0.f, v1 = 0.f;
+        float acc = mom[(size_t)(2 * NI + i) * ROW + base + F] +
+                    mom[(size_t)(3 * NI + i) * ROW + base - F - 1];
 #pragma unroll
-        for (int k = F - 1; k >= 0; --k) {
-            u0 = fmaf(1.f - (float)k * inv_r, M0[k], u0);
-            v0 += M1[k];
+        for (int k = -(F - 1); k <= F; ++k) {
+            acc = fmaf(1.f - (float)(k < 0 ? -k : k) * inv_r, M0[-k], acc);
+            acc = fmaf(k <= 0 ? -inv_r : inv_r, M1[-k], acc);
         }
-#pragma unroll
-        for (int k = F; k >= 1; --k) {
-            u1 = fmaf(1.f - (float)k * inv_r, M0[-k], u1);
-            v1 += M1[-k];
-        }
-        raw[((size_t)(w0 + i) * D + d) * T + t] = fmaf(v1 - v0, inv_r, u0 + u1) * scale;
+        raw[((size_t)(w0 + i) * D + d) * T + t] = acc * scale;
     }
 }
 

@@ -832,49 +832,13 @@ struct ConvEpi {
     double *part;
 };
 
-// per detector [first, last + 1) samples of the interpolation's support; grow:
-// how far the output reaches beyond it; fill: forward direction (see below)
+// rng: per detector [first, last + 1) samples of the interpolation's support, its
+// neighbours' included.  fwd: the input is zero outside it (and is not read
+// there); else (transpose) the output is read inside it only.
 struct ConvRange {
     const int2 *rng;
-    int D, grow, fill, ntile, diff;
+    int D, fwd;
 };
-
-// the row pair's samples outside [olo, ohi), where y = A x is zero
-template <int EPI>
-__device__ __forceinline__ void conv_outside(float *y1, float *y2, size_t row, int olo, int ohi,
-                                             int T, int lane, const ConvEpi &epi, float &acc) {
-    const int w = EPI ? (int)(row / T) / epi.D : 0;
-    float g = 0.f;
-    bool done = false;
-    if constexpr (EPI != 0) {
-        const Scal &q = epi.sc[epi.coupled ? 0 : w];
-        g = (float)q.gamma;
-        done = EPI == 2 && q.done;
-    }
-    const int out = olo + T - ohi;
-    for (int i0 = lane; i0 < out; i0 += 128) {
-        float v1[4], v2[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int i = i0 + 32 * j, t = i < olo ? i : i - olo + ohi;
-            v1[j] = v2[j] = 0.f;
-            if (EPI != 0 && i < out) {
-                v1[j] = EPI == 1 ? epi.b[row + t] : y1[t];
-                if (y2) v2[j] = EPI == 1 ? epi.b[row + T + t] : y2[t];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int i = i0 + 32 * j, t = i < olo ? i : i - olo + ohi;
-            if (i >= out) break;
-            const float f = EPI == 1 ? epi.sl : done ? 1.f : -g;
-            const float a = EPI ? f * v1[j] : 0.f, b = EPI ? f * v2[j] : 0.f;
-            y1[t] = a;
-            if (y2) y2[t] = b;
-            acc = fmaf(a, a, fmaf(b, b, acc));
-        }
-    }
-}
 
 // 1024-point overlap-save convolution by the four-step FFT 1024 = 32 x 32:
 // one warp per transform (two real columns as one complex sequence), the
@@ -886,22 +850,16 @@ __device__ __forceinline__ void conv_outside(float *y1, float *y2, size_t row, i
 // k1 = brev5(2m), brev5(2m + 1); twn = conj w1024^(lane n) for n = 2m,
 // 2m + 1; Hb = H[lane + 32 k2] for k2 = brev5(2m), brev5(2m + 1).
 //
-// Only the samples a detector can reach are transformed.  cr.rng holds each
-// detector's support of the interpolation, [first, last + 1) over its pixels'
-// taps: in the forward direction the input is zero outside it (and is not read
-// there) and the output outside the support grown by L / 2, which the CTAs of
-// blockIdx.x == cr.ntile fill (zeros, or the epilogue with y = 0); in the
-// transpose the output is read by the adjoint inside the support only.  At
-// 128 x 128 px / 256 x 2030 samples two tiles per column pair instead of
-// three, at 400 x 400 / 512 x 4096 two instead of six.  Measured per launch at
-// batch 64 (16384 columns): 98 -> 77 us forward, 62 us transpose.
-//
-// cr.diff: IRs without a DC part (any with the reference's high-pass) are
-// applied in the forward direction as their running sum to x[u] - x[u - 1].
-// The interpolated rows are smooth and positive, so the transform's rounding,
-// relative to the largest part of its input, no longer comes from a DC that
-// the IR removes: A's error at 128 x 128 px falls from 2.0e-6 to 1.1e-6 (with the four chains of
-// das_fwd.cuh); 7 % more instructions.
+// Only what a detector can reach is read, transformed and (transpose) written:
+// a tile without input is zero, a tile nobody reads is left out.  Forward and
+// transpose on average 76 -> 47 us for 13 images of 400 x 400 px / 512 x 4096 samples
+// (three of six tiles per column pair); 98 -> 95 and 87 us for 64 of 128 x 128 px / 256 x
+// 2030 samples.  The
+// tiles lie at multiples of V for every detector and the transform takes the
+// samples themselves: tiles that start at each detector's support (two per pair at
+// 2030 samples, 77 and 62 us), or the taps' running sum over differenced samples
+// (A's error 1.1e-6 for 2.0e-6), round differently, and the iterative solves
+// amplify a last bit to 1e-3 of an image's rms at single pixels.
 template <int FPC, int EPI = 0, int MINB = 1>
 __global__ void __launch_bounds__(32 * FPC, MINB) k_conv_fft1k(
     const float *__restrict__ in, float *__restrict__ out, const float4 *__restrict__ twb,
@@ -914,43 +872,35 @@ __global__ void __launch_bounds__(32 * FPC, MINB) k_conv_fft1k(
     const int c1 = 2 * pair, c2 = c1 + 1;
     if (c1 >= C) return;  // whole warp; no CTA-wide barriers below
     const bool has2 = c2 < C;
-    const int V = 1024 - L + 1;
+    const int V = 1024 - L + 1, t0 = blockIdx.x * V;
     const int2 ra = __ldg(cr.rng + c1 % cr.D), rb = has2 ? __ldg(cr.rng + c2 % cr.D) : ra;
-    const int olo = max(0, min(ra.x, rb.x) - cr.grow), ohi = min(T, max(ra.y, rb.y) + cr.grow);
+    const int lo = max(ra.x, rb.x), hi = min(ra.y, rb.y);  // holds both supports
+    // transpose: nobody reads the tile
+    if (EPI == 0 && !cr.fwd && (t0 >= hi || t0 + V <= lo)) return;
+    const int u0 = t0 + L / 2 - (L - 1);
+    const float *x1 = in + (size_t)c1 * T;
+    const float *x2 = in + (size_t)(has2 ? c2 : c1) * T;
     float *y1 = out + (size_t)c1 * T, *y2 = out + (size_t)c2 * T;
-    const int t0 = olo + blockIdx.x * V;
-    float acc = 0.f;
-    if (cr.fill && blockIdx.x == cr.ntile) {
-        // the samples outside [olo, ohi): A x is zero there
-        conv_outside<EPI>(y1, has2 ? y2 : nullptr, (size_t)c1 * T, olo, ohi, T, lane, epi, acc);
-    } else if (t0 < ohi) {
-        const int u0 = t0 + L / 2 - (L - 1);
-        const float *x1 = in + (size_t)c1 * T;
-        const float *x2 = in + (size_t)(has2 ? c2 : c1) * T;
-        // forward (grow > 0 or not, fill set): the input counts inside its support
-        const int a1 = cr.fill ? ra.x : 0, e1 = cr.fill ? ra.y : T;
-        const int a2 = cr.fill ? rb.x : 0, e2 = cr.fill ? rb.y : T;
-        float2 R[16], I[16];
+    const int a = cr.fwd ? lo : 0, e = cr.fwd ? hi : T;  // the input counts here
+    float2 R[16], I[16];
+    if (u0 >= e || u0 + 1024 <= a) {  // uniform in the warp
 #pragma unroll
-        for (int n1 = 0; n1 < 32; ++n1) {
-            const int u = u0 + 32 * n1 + lane;
-            ev(R, n1) = u >= a1 && u < e1 ? __ldg(x1 + u) : 0.f;
-            ev(I, n1) = (has2 && u >= a2 && u < e2) ? __ldg(x2 + u) : 0.f;
-        }
-        if (cr.diff) {
-            // x[u] - x[u - 1]: the left neighbour is the lane below, for lane 0
-            // the last lane of the row before
-            const int u = u0 - 1;
-            float pr = u >= a1 && u < e1 ? __ldg(x1 + u) : 0.f;
-            float pi = (has2 && u >= a2 && u < e2) ? __ldg(x2 + u) : 0.f;
+        for (int m = 0; m < 16; ++m) R[m] = I[m] = make_float2(0.f, 0.f);
+    } else {
+        if (u0 >= a && u0 + 1024 <= e) {
 #pragma unroll
             for (int n1 = 0; n1 < 32; ++n1) {
-                const float r = __shfl_sync(0xffffffffu, ev(R, n1), (lane + 31) & 31);
-                const float i = __shfl_sync(0xffffffffu, ev(I, n1), (lane + 31) & 31);
-                ev(R, n1) -= lane ? r : pr;
-                ev(I, n1) -= lane ? i : pi;
-                pr = r;
-                pi = i;
+                const int u = u0 + 32 * n1 + lane;
+                ev(R, n1) = __ldg(x1 + u);
+                ev(I, n1) = has2 ? __ldg(x2 + u) : 0.f;
+            }
+        } else {
+#pragma unroll
+            for (int n1 = 0; n1 < 32; ++n1) {
+                const int u = u0 + 32 * n1 + lane;
+                const bool ok = (unsigned)(u - a) < (unsigned)(e - a);
+                ev(R, n1) = ok ? __ldg(x1 + u) : 0.f;
+                ev(I, n1) = (ok && has2) ? __ldg(x2 + u) : 0.f;
             }
         }
         fft32_dif2<-1>(R, I);  // over n1 (this lane is n2); register e holds k1 = brev5(e)
@@ -988,63 +938,61 @@ __global__ void __launch_bounds__(32 * FPC, MINB) k_conv_fft1k(
             I[m] = *reinterpret_cast<const float2 *>(&Si[lane][2 * m]);
         }
         fft32_dif2<1>(R, I);  // inverse over k1: register e holds y[n1' + 32 n2'], n2' = brev5(e)
-        if constexpr (EPI == 0) {
+    }
+    if constexpr (EPI == 0) {
 #pragma unroll
-            for (int e = 0; e < 32; ++e) {
-                const int n = lane + 32 * brev5(e);
-                const int t = t0 + n - (L - 1);
-                if (n >= L - 1 && t < ohi) {
-                    y1[t] = ev(R, e);
-                    if (has2) y2[t] = ev(I, e);
-                }
+        for (int e = 0; e < 32; ++e) {
+            const int n = lane + 32 * brev5(e);
+            const int t = t0 + n - (L - 1);
+            if (n >= L - 1 && t < T) {
+                y1[t] = ev(R, e);
+                if (has2) y2[t] = ev(I, e);
             }
-        } else {
-            const int w = c1 / epi.D;
-            const Scal &q = epi.sc[epi.coupled ? 0 : w];
-            const float g = (float)q.gamma, sl = epi.sl;
-            const bool done = EPI == 2 && q.done;
-            const float *b1 = epi.b + (size_t)c1 * T, *b2 = epi.b + (size_t)c2 * T;
-            // chunks of 8 outputs: all loads of a chunk are issued before its
-            // stores (the stores could alias the loads of later iterations)
-            constexpr int CH = 8;
+        }
+    } else {
+        const int w = c1 / epi.D;
+        const Scal &q = epi.sc[epi.coupled ? 0 : w];
+        const float g = (float)q.gamma, sl = epi.sl;
+        const bool done = EPI == 2 && q.done;
+        const float *b1 = epi.b + (size_t)c1 * T, *b2 = epi.b + (size_t)c2 * T;
+        float acc = 0.f;
+        // chunks of 8 outputs: all loads of a chunk are issued before its
+        // stores (the stores could alias the loads of later iterations)
+        constexpr int CH = 8;
 #pragma unroll
-            for (int c0 = 0; c0 < 32; c0 += CH) {
-                float l1[CH], l2[CH];
+        for (int c0 = 0; c0 < 32; c0 += CH) {
+            float l1[CH], l2[CH];
 #pragma unroll
-                for (int j = 0; j < CH; ++j) {
-                    const int n = lane + 32 * (c0 + j);
-                    const int t = t0 + n - (L - 1);
-                    const bool ok = n >= L - 1 && t < ohi;
-                    const float *s1 = EPI == 1 ? b1 : y1, *s2 = EPI == 1 ? b2 : y2;
-                    l1[j] = ok ? s1[t] : 0.f;
-                    l2[j] = (ok && has2) ? s2[t] : 0.f;
-                }
+            for (int j = 0; j < CH; ++j) {
+                const int n = lane + 32 * (c0 + j);
+                const int t = t0 + n - (L - 1);
+                const bool ok = n >= L - 1 && t < T;
+                const float *s1 = EPI == 1 ? b1 : y1, *s2 = EPI == 1 ? b2 : y2;
+                l1[j] = ok ? s1[t] : 0.f;
+                l2[j] = (ok && has2) ? s2[t] : 0.f;
+            }
 #pragma unroll
-                for (int j = 0; j < CH; ++j) {
-                    const int n2 = c0 + j, e = brev5(n2);
-                    const int n = lane + 32 * n2;
-                    const int t = t0 + n - (L - 1);
-                    if (n >= L - 1 && t < ohi) {
-                        const float vr = ev(R, e), vi = ev(I, e);
-                        float a, bb;
-                        if (EPI == 1) {
-                            a = fmaf(sl, l1[j], -sl * vr);
-                            bb = has2 ? fmaf(sl, l2[j], -sl * vi) : 0.f;
-                        } else {
-                            a = done ? l1[j] : fmaf(sl, vr, -g * l1[j]);
-                            bb = done ? l2[j] : fmaf(sl, vi, -g * l2[j]);
-                        }
-                        y1[t] = a;
-                        if (has2) y2[t] = bb;
-                        acc = fmaf(a, a, acc);
-                        acc = fmaf(bb, bb, acc);
+            for (int j = 0; j < CH; ++j) {
+                const int n2 = c0 + j, e = brev5(n2);
+                const int n = lane + 32 * n2;
+                const int t = t0 + n - (L - 1);
+                if (n >= L - 1 && t < T) {
+                    const float vr = ev(R, e), vi = ev(I, e);
+                    float a, bb;
+                    if (EPI == 1) {
+                        a = fmaf(sl, l1[j], -sl * vr);
+                        bb = has2 ? fmaf(sl, l2[j], -sl * vi) : 0.f;
+                    } else {
+                        a = done ? l1[j] : fmaf(sl, vr, -g * l1[j]);
+                        bb = done ? l2[j] : fmaf(sl, vi, -g * l2[j]);
                     }
+                    y1[t] = a;
+                    if (has2) y2[t] = bb;
+                    acc = fmaf(a, a, acc);
+                    acc = fmaf(bb, bb, acc);
                 }
             }
         }
-    }
-    if constexpr (EPI != 0) {
-        const int w = c1 / epi.D;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
         __shared__ float wacc[FPC];
@@ -1443,13 +1391,8 @@ static int conv_min_blocks(const Plan &pl) {
     return pl.tune_conv_mb ? pl.tune_conv_mb : g_conv_min_blocks.load();
 }
 
-static ConvRange conv_range(const Plan &pl, bool transpose) {
-    return {pl.conv_rng, pl.D, transpose ? 0 : pl.L / 2, transpose ? 0 : 1,
-            transpose ? pl.conv_nt_a : pl.conv_nt_f, transpose ? 0 : pl.conv_diff};
-}
-
 // forward: `in` counts inside each detector's support only; transpose: `out` is
-// written inside it only (1024-point path; the others cover whole rows)
+// written in the tiles that meet it (1024-point path; the others cover whole rows)
 int launch_conv(const Plan &pl, const float *in, float *out, int W, bool transpose,
                 cudaStream_t st) {
     TimedScope ts_(KID_CONV, st);
@@ -1462,8 +1405,8 @@ int launch_conv(const Plan &pl, const float *in, float *out, int W, bool transpo
         int rc;
         if (pl.fft_log4n == 5) {
             constexpr int FPC = CONV_FPC;
-            const ConvRange cr = conv_range(pl, transpose);
-            dim3 g1(cr.ntile + cr.fill, div_up(div_up(C, 2), FPC));
+            const ConvRange cr{pl.conv_rng, pl.D, transpose ? 0 : 1};
+            dim3 g1(div_up(pl.T, V), div_up(div_up(C, 2), FPC));
             const float4 *Hb = transpose ? pl.fft_hab : pl.fft_hfb;
             switch (conv_min_blocks(pl)) {
             case 3:
@@ -1502,7 +1445,8 @@ int launch_conv(const Plan &pl, const float *in, float *out, int W, bool transpo
 
 bool forward_update_fusable(const Plan &pl, int W) {
     if (pl.L <= 0 || pl.fft_log4n != 5 || pl.D % (2 * CONV_FPC) != 0) return false;
-    const int nparts = (pl.D / (2 * CONV_FPC)) * (pl.conv_nt_f + 1);
+    const int V = 1024 - pl.L + 1;
+    const int nparts = (pl.D / (2 * CONV_FPC)) * div_up(pl.T, V);
     return nparts <= 256 && W >= 1;
 }
 
@@ -1587,9 +1531,9 @@ int apply_forward_update(const Plan &pl, const float *img, float *u, const float
     int rc;
     if ((rc = forward_to_raw(pl, img, W, st))) return rc;
     TimedScope ts_(KID_CONV, st);
-    const int C = W * pl.D;
-    const ConvRange cr = conv_range(pl, false);
-    const dim3 g1(cr.ntile + 1, div_up(div_up(C, 2), CONV_FPC));
+    const int C = W * pl.D, V = 1024 - pl.L + 1;
+    const ConvRange cr{pl.conv_rng, pl.D, 1};
+    const dim3 g1(div_up(pl.T, V), div_up(div_up(C, 2), CONV_FPC));
     ConvEpi e;
     e.b = b;
     e.sc = sc;

@@ -252,13 +252,19 @@ static int build(const msot_plan_desc *d, Plan &p) {
     }
 
     // --- support of the interpolation per detector: taps floor(tau) - F ..
-    // floor(tau) + F + 1 of its pixels; SIR responses may reach the whole row
-    std::vector<int2> rng(p.D, make_int2(0, p.T));
+    // floor(tau) + F + 1 of its pixels; SIR responses may reach the whole row.
+    // Together with the neighbours' (the convolution transforms two detectors at
+    // once, the last one with the first where D is odd)
+    std::vector<int2> own(p.D, make_int2(0, p.T)), rng(p.D);
     for (int det = 0; det < p.D && !has_sir; ++det) {
         const int32_t *tf = tfx.data() + (size_t)det * p.P;
         const auto mm = std::minmax_element(tf, tf + p.P);
-        rng[det] = make_int2(std::max(0, (*mm.first >> fb) - p.F),
+        own[det] = make_int2(std::max(0, (*mm.first >> fb) - p.F),
                              std::min(p.T, (*mm.second >> fb) + p.F + 2));
+    }
+    for (int det = 0; det < p.D; ++det) {
+        const int2 a = own[(det + p.D - 1) % p.D], b = own[det], c = own[(det + 1) % p.D];
+        rng[det] = make_int2(std::min({a.x, b.x, c.x}), std::max({a.y, b.y, c.y}));
     }
 
     // --- adjoint blocks: 64x64 pixels, travel times and bucket span per detector --------
@@ -396,24 +402,13 @@ static int build(const msot_plan_desc *d, Plan &p) {
         const double two_pi = 6.283185307179586476925286766559;
         for (int t = 0; t < N; ++t)
             ftw[t] = make_float2((float)std::cos(two_pi * t / N), (float)-std::sin(two_pi * t / N));
-        // taps that sum to zero: the forward direction of the 1024-point path
-        // takes differenced input and the taps' running sum (operator.cu)
-        std::vector<double> hf0(d->ir, d->ir + p.L);
-        double sum = 0.0, mag = 0.0;
-        for (double v : hf0) sum += v, mag += std::fabs(v);
-        if (p.fft_log4n == 5 && std::fabs(sum) <= 1e-11 * mag) {
-            p.conv_diff = 1;
-            double run = 0.0;
-            for (int k = 0; k < p.L; ++k) hf0[k] = run += d->ir[k];
-            hf0[p.L - 1] = 0.0;
-        }
         // direct DFT of the short tap vectors: H[f] = sum_k h[k] e^{-2 pi i f k / N} / N
         for (int f = 0; f < N; ++f) {
             double fr = 0, fi = 0, ar = 0, ai = 0;
             for (int k = 0; k < p.L; ++k) {
                 const double ang = -two_pi * (double)(((long)f * k) % N) / N;
                 const double c = std::cos(ang), sn = std::sin(ang);
-                const double hf = hf0[k] / p.norm, ha = d->ir[p.L - 1 - k] / p.norm;
+                const double hf = d->ir[k] / p.norm, ha = d->ir[p.L - 1 - k] / p.norm;
                 fr += hf * c; fi += hf * sn;
                 ar += ha * c; ai += ha * sn;
             }
@@ -423,16 +418,6 @@ static int build(const msot_plan_desc *d, Plan &p) {
     }
     std::vector<float4> ftwb, ftwn, fhfb, fhab;
     if (p.fft_log4n == 5) {
-        // tiles that the widest column pair (neighbouring detectors, or the
-        // last and the first of two instances) needs
-        const int V = 1024 - p.L + 1, h = p.L / 2;
-        for (int det = 0; det < p.D; ++det) {
-            const int2 a = rng[det], b = rng[(det + 1) % p.D];
-            const int lo = std::min(a.x, b.x), hi = std::max(a.y, b.y);
-            p.conv_nt_a = std::max(p.conv_nt_a, div_up(hi - lo, V));
-            p.conv_nt_f = std::max(p.conv_nt_f,
-                                   div_up(std::min(p.T, hi + h) - std::max(0, lo - h), V));
-        }
         auto brev5 = [](int i) {
             return ((i & 1) << 4) | ((i & 2) << 2) | (i & 4) | ((i & 8) >> 2) | ((i & 16) >> 4);
         };

@@ -265,7 +265,7 @@ int launch_permute(const Plan &pl, const float *in, float *out, int W, cudaStrea
 int launch_das_forward(const Plan &pl, const float *x_pi, float *raw, int W, float scale,
                        cudaStream_t st, bool to_conv);
 int launch_das_adjoint(const Plan &pl, const float *raw, float *x, int W, float scale,
-                       cudaStream_t st);
+                       cudaStream_t st, bool batched);
 int launch_conv(const Plan &pl, const float *in, float *out, int W, bool transpose,
                 cudaStream_t st);
 int launch_sir_forward(const Plan &pl, const float *x_pi, float *raw, int W, float scale,
@@ -276,8 +276,10 @@ int launch_sir_adjoint(const Plan &pl, const float *raw, float *x, int W, float 
 // detector's support (Plan::conv_rng), so tiles outside it are not written
 int interp_forward(const Plan &pl, const float *x_pi, float *raw, int W, float scale,
                    cudaStream_t st, bool to_conv = false);
+// batched: a call of the operator itself, which may take the batched kernel; the
+// iterative solves keep k_das_adj4's order of the sums (das_adj.cu)
 int interp_adjoint(const Plan &pl, const float *raw, float *x, int W, float scale,
-                   cudaStream_t st);
+                   cudaStream_t st, bool batched = false);
 int apply_forward(const Plan &pl, const float *img, float *sino, int W, cudaStream_t st);
 
 // Per-group scalars of the Krylov solvers (one group = one instance, or the
@@ -301,7 +303,8 @@ bool forward_update_fusable(const Plan &pl, int W);
 void solver_cache_free(Plan &pl);  // solver.cu
 void solver_cache_invalidate(Plan &pl);  // drops the captured solver graphs (solver.cu)
 bool profiling_enabled();          // timing.cu
-int apply_transpose(const Plan &pl, const float *sino, float *img, int W, cudaStream_t st);
+int apply_transpose(const Plan &pl, const float *sino, float *img, int W, cudaStream_t st,
+                    bool batched = false);
 
 inline int div_up(int a, int b) { return (a + b - 1) / b; }
 

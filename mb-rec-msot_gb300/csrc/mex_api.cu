@@ -93,7 +93,8 @@ int run_mex(bool forward, const double *in, int W, int P, int D, int T, const do
                     h[((size_t)w * D + det) * T + t] = (float)in[((size_t)det * T + t) * W + w];
         MSOT_CUDA_TRY(
             cudaMemcpy(dsino.p, h.data(), NS_ * sizeof(float), cudaMemcpyHostToDevice));
-        if ((rc = interp_adjoint(pl, (float *)dsino.p, (float *)dimg.p, W, 1.f, st))) return rc;
+        if ((rc = interp_adjoint(pl, (float *)dsino.p, (float *)dimg.p, W, 1.f, st, true)))
+            return rc;
         std::vector<float> o(NI);
         MSOT_CUDA_TRY(cudaMemcpy(o.data(), dimg.p, NI * sizeof(float), cudaMemcpyDeviceToHost));
         for (int p = 0; p < P; ++p)

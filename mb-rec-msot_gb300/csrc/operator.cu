@@ -148,6 +148,9 @@ __global__ void k_prefilter(const float *__restrict__ in, float *__restrict__ ou
 // of 128 x 128 px (18 -> 7 us), and any grid size (400 x 400 px took one
 // launch per axis with every tap from global memory: 13 images 133 -> 28
 // us); batch 64 at 128 x 128 px 23 -> 14 to 16 us, the stores were the bound.
+//
+// XF: x first, then z (IPC = 1, out_mode 0).  The transpose takes the axes in the
+// order that launch_prefilter2d names, so that its sums round as they did.
 // ---------------------------------------------------------------------------
 constexpr int PF_T = 32, PF_RZ = 8, PF_RX = 4, PF_THREADS = 256;
 
@@ -156,7 +159,7 @@ __device__ __forceinline__ int wrap_mod(int a, int n) {
     return a < 0 ? a + n : a;
 }
 
-template <int KM, int IPC>
+template <int KM, int IPC, bool XF = false>
 __global__ void __launch_bounds__(PF_THREADS) k_prefilter2d(
     const float *__restrict__ in, float *__restrict__ out, const float *__restrict__ taps_x,
     const float *__restrict__ taps_z, int Kx, int Kz, int nx, int nz, int W, int transpose,
@@ -193,6 +196,7 @@ __global__ void __launch_bounds__(PF_THREADS) k_prefilter2d(
                 if (lane + 32 * j < NC) A[c * LA + lane + 32 * j] = __ldg(scol + row[j]);
         }
         __syncthreads();
+        if constexpr (XF) break;
         // z pass, lanes over columns: B[c][z] = sum_k hz[k] A[c][z + KM - k]
         constexpr int NCG = (NC + 31) / 32;
         for (int it = warp; it < NCG * (PF_T / PF_RZ); it += NW) {
@@ -215,6 +219,53 @@ __global__ void __launch_bounds__(PF_THREADS) k_prefilter2d(
                 for (int j = 0; j < PF_RZ; ++j) B[(i * NC + c) * LB + z0 + j] = acc[j];
             }
         }
+    }
+    if constexpr (XF) {
+        static_assert(!XF || IPC == 1, "one image per CTA");
+        // x pass, lanes along the staged rows: B[x][r] = sum_k hx[k] A[x + KM - k][r]
+        constexpr int NRG = (NC + 31) / 32;
+        for (int it = warp; it < NRG * (PF_T / PF_RZ); it += NW) {
+            const int r = (it % NRG) * 32 + lane, c0 = (it / NRG) * PF_RZ;
+            if (r < NC) {
+                float win[PF_RZ + 2 * KM];
+#pragma unroll
+                for (int j = 0; j < PF_RZ + 2 * KM; ++j) win[j] = A[(c0 + j) * LA + r];
+                float acc[PF_RZ];
+#pragma unroll
+                for (int j = 0; j < PF_RZ; ++j) acc[j] = 0.f;
+#pragma unroll
+                for (int k = -KM; k <= KM; ++k) {
+                    const float h = hx[k + KM];
+#pragma unroll
+                    for (int j = 0; j < PF_RZ; ++j) acc[j] = fmaf(h, win[j - k + KM], acc[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < PF_RZ; ++j) B[(c0 + j) * LA + r] = acc[j];
+            }
+        }
+        __syncthreads();
+        // z pass, lanes over columns, back into A [column][LB]
+        for (int z0 = warp * PF_RX; z0 < PF_T; z0 += NW * PF_RX) {
+            float win[PF_RX + 2 * KM], acc[PF_RX];
+#pragma unroll
+            for (int j = 0; j < PF_RX + 2 * KM; ++j) win[j] = B[lane * LA + z0 + j];
+#pragma unroll
+            for (int j = 0; j < PF_RX; ++j) acc[j] = 0.f;
+#pragma unroll
+            for (int k = -KM; k <= KM; ++k) {
+                const float h = hz[k + KM];
+#pragma unroll
+                for (int j = 0; j < PF_RX; ++j) acc[j] = fmaf(h, win[j - k + KM], acc[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < PF_RX; ++j) A[lane * LB + z0 + j] = acc[j];
+        }
+        __syncthreads();
+        const int z = iz0 + lane;
+        for (int c = warp; c < PF_T && z < nz; c += NW)
+            if (ix0 + c < nx)
+                out[((size_t)w0 * nx + ix0 + c) * nz + z] = A[c * LB + lane];
+        return;
     }
     __syncthreads();
     // x pass, lanes along z: out[ix0 + c][z] = sum_k hx[k] B[c + KM - k][z]
@@ -1095,17 +1146,18 @@ int launch_prefilter(const Plan &pl, const float *in, float *out, int W, bool tr
     return MSOT_OK;
 }
 
-template <int KM, int IPC>
+template <int KM, int IPC, bool XF = false>
 static int prefilter2d_run(const Plan &pl, const float *in, float *out, int W, bool transpose,
                            int out_mode, int wt, int fmt, cudaStream_t st) {
     constexpr int NC = PF_T + 2 * KM;
     constexpr size_t smem =
         (size_t)(NC * (NC | 1) + IPC * NC * (PF_T + 1) + 2 * (2 * KM + 1)) * sizeof(float);
-    int rc = set_smem(k_prefilter2d<KM, IPC>, smem);
+    static_assert(!XF || PF_T * (NC | 1) <= NC * (PF_T + 1), "B holds the x pass");
+    int rc = set_smem(k_prefilter2d<KM, IPC, XF>, smem);
     if (rc) return rc;
     const dim3 grid((unsigned)div_up(pl.nx, PF_T), (unsigned)div_up(pl.nz, PF_T),
                     (unsigned)div_up(W, IPC));
-    KLAUNCH(k_prefilter2d<KM, IPC><<<grid, PF_THREADS, smem, st>>>(
+    KLAUNCH(k_prefilter2d<KM, IPC, XF><<<grid, PF_THREADS, smem, st>>>(
         in, out, pl.pre_x, pl.pre_z, pl.Kx, pl.Kz, pl.nx, pl.nz, W, transpose ? 1 : 0, out_mode,
         wt, fmt, pl.h16_sc));
     MSOT_LAUNCH_CHECK();
@@ -1122,6 +1174,12 @@ static int prefilter2d_km(const Plan &pl, const float *in, float *out, int W, bo
                                                pl.h16_sc, pl.max_batch));
     if (out_mode == 2 && fmt == 0 && wt % 4 == 0)
         return prefilter2d_run<KM, 4>(pl, in, out, W, transpose, out_mode, wt, fmt, st);
+    // the transpose of longer columns filters x first: the order of its sums, which
+    // the solves' bits depend on, is that of the per-axis kernels that longer columns had
+    constexpr int NC = PF_T + 2 * KM;
+    const bool z_first = (size_t)(2 * NC * (pl.nz | 1) + 2 * (2 * KM + 1)) * 4 <= 200 * 1024;
+    if (transpose && !z_first && out_mode == 0)
+        return prefilter2d_run<KM, 1, true>(pl, in, out, W, transpose, out_mode, wt, fmt, st);
     return prefilter2d_run<KM, 1>(pl, in, out, W, transpose, out_mode, wt, fmt, st);
 }
 
@@ -1243,6 +1301,8 @@ static int das_adj_launch(const Plan &pl, const float *raw, float *x, int W, flo
     const int base = pl.n_blk * (W / WT);
     int groups = std::max(1, std::min(pl.D, div_up(2 * sm_count(), base)));
     groups = std::min(groups, std::max(1, pl.adj_groups_max * pl.max_batch / W));
+    // no more than one partial image in 512: the groups are the order of the sums
+    groups = std::min({groups, 32, std::max(1, 512 / pl.max_batch)});
     const int dpg = div_up(pl.D, groups);
     groups = div_up(pl.D, dpg);
     const size_t stride = (size_t)W * pl.P;
@@ -1288,14 +1348,11 @@ static int das_adj_f(const Plan &pl, const float *raw, float *x, int W, float sc
 }
 
 int launch_das_adjoint(const Plan &pl, const float *raw, float *x, int W, float scale,
-                       cudaStream_t st) {
+                       cudaStream_t st, bool batched) {
     TimedScope ts_(KID_INTERP_ADJ, st);
-    // the batched kernel unless the autotuner found a wt of k_das_adj4 faster
+    if (batched && adj5_usable(pl, W)) return launch_das_adjoint5(pl, raw, x, W, scale, st);
     int wt = pick_wt(W, 1, 2);
-    if (pl.tune_adj_wt && W % pl.tune_adj_wt == 0)
-        wt = pl.tune_adj_wt;
-    else if (adj5_usable(pl, W))
-        return launch_das_adjoint5(pl, raw, x, W, scale, st);
+    if (pl.tune_adj_wt && W % pl.tune_adj_wt == 0) wt = pl.tune_adj_wt;
     if (wt == 4) return das_adj_f<4>(pl, raw, x, W, scale, st);
     if (wt == 2) return das_adj_f<2>(pl, raw, x, W, scale, st);
     return das_adj_f<1>(pl, raw, x, W, scale, st);
@@ -1460,9 +1517,9 @@ int interp_forward(const Plan &pl, const float *x_pi, float *raw, int W, float s
 }
 
 int interp_adjoint(const Plan &pl, const float *raw, float *x, int W, float scale,
-                   cudaStream_t st) {
+                   cudaStream_t st, bool batched) {
     return pl.S ? launch_sir_adjoint(pl, raw, x, W, scale, st)
-                : launch_das_adjoint(pl, raw, x, W, scale, st);
+                : launch_das_adjoint(pl, raw, x, W, scale, st, batched);
 }
 
 // the image order the interpolation takes: perm[] (k_sir_fwd) or pixel-major
@@ -1561,7 +1618,8 @@ int apply_forward_update(const Plan &pl, const float *img, float *u, const float
     return MSOT_OK;
 }
 
-int apply_transpose(const Plan &pl, const float *sino, float *img, int W, cudaStream_t st) {
+int apply_transpose(const Plan &pl, const float *sino, float *img, int W, cudaStream_t st,
+                    bool batched) {
     int rc;
     const float *src = sino;
     float scale = pl.scale;
@@ -1572,7 +1630,7 @@ int apply_transpose(const Plan &pl, const float *sino, float *img, int W, cudaSt
     }
     const bool pre = pl.Kx >= 0 || pl.Kz >= 0;
     float *x = pre ? pl.scr_img0 : img;
-    if ((rc = interp_adjoint(pl, src, x, W, scale, st))) return rc;
+    if ((rc = interp_adjoint(pl, src, x, W, scale, st, batched))) return rc;
     if ((rc = launch_prefilter2d(pl, pl.scr_img0, img, W, true, 0, st)) <= 0) return rc;
     if (pl.Kx >= 0 && pl.Kz >= 0) {
         if ((rc = launch_prefilter(pl, pl.scr_img0, pl.scr_img1, W, true, true, 1.f, 0, st)))
@@ -1705,7 +1763,7 @@ int msot_transpose(msot_plan_t plan, const float *d_sino, float *d_img, int batc
                    void *stream) {
     int rc = check_batch(plan, batch, d_sino, d_img);
     if (rc) return rc;
-    return apply_transpose(plan->p, d_sino, d_img, batch, (cudaStream_t)stream);
+    return apply_transpose(plan->p, d_sino, d_img, batch, (cudaStream_t)stream, true);
 }
 
 int msot_interp_forward(msot_plan_t plan, const float *d_coeffs, float *d_raw, int batch,
@@ -1725,7 +1783,7 @@ int msot_interp_transpose(msot_plan_t plan, const float *d_raw, float *d_coeffs,
                           void *stream) {
     int rc = check_batch(plan, batch, d_raw, d_coeffs);
     if (rc) return rc;
-    return interp_adjoint(plan->p, d_raw, d_coeffs, batch, 1.f, (cudaStream_t)stream);
+    return interp_adjoint(plan->p, d_raw, d_coeffs, batch, 1.f, (cudaStream_t)stream, true);
 }
 
 int msot_plan_set_storage(msot_plan_t plan, int image_format, int refine_every) {

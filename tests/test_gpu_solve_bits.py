@@ -53,6 +53,10 @@ CASES = [
     ("forward", 70, 37, 1300, 3),      # odd D: column pairs across images
     ("forward", 70, 16, 4096, 9),      # most tiles without input; lanes over instances
     ("forward", 31, 8, 1300, 33),      # r = 8.9; tiles of 32 images and of one
+    ("transpose", 400, 8, 1300, 2),    # prefilter of long columns
+    ("l2", 64, 64, 1300, 9),
+    ("l2", 90, 40, 1300, 2),           # D no multiple of 8 pairs: the unfused update
+    ("l1", 64, 64, 1300, 6),
 ]
 
 

@@ -8,12 +8,12 @@
 //                 sweeps).  One CTA per image runs the whole prox on the
 //                 device (bounded loops, no host round trips), vectors in
 //                 global memory.
-//   k_tv_prox_cl4  the same prox by one thread-block cluster per image, the
-//                 image split into column slabs held in shared memory
-//                 (neighbours over distributed shared memory), 4 z-pixels per
-//                 thread; its GM form keeps the vectors in an L2-resident
-//                 workspace for images too large for shared memory.
-//                 k_tv_prox is the fallback.
+//   k_tv_prox_cl / k_tv_prox_cl4  the same prox by one thread-block cluster
+//                 per image, the image split into column slabs held in shared
+//                 memory (neighbours over distributed shared memory); cl4
+//                 handles 4 z-pixels per thread, and its GM form keeps the
+//                 vectors in an L2-resident workspace for images too large
+//                 for shared memory.  k_tv_prox is the fallback.
 //   k_itv      <- ITV.m:5-6 (isotropic TV with MATLAB's gradient: central
 //                 differences inside, one-sided at the borders).
 //   msot_rec_nn_with_TV_reg <- rec_nn_with_TV_reg.m:20-54 and
@@ -302,6 +302,20 @@ constexpr int TVC_MAXC = 16;  // largest cluster
 constexpr int TVC_NV = 12;
 constexpr int TVC_NV_REG = 9;  // without rt, M uc, M q: in registers
 enum TvcVec { V_U = 0, V_X, V_B1, V_B2, V_R, V_RT, V_MQ, V_MUC, V_Q, V_UC, V_VH, V_XMIN };
+// the kernel of a pixel per thread: p in two buffers and uh instead of M q, M uc
+constexpr int TVC_NV1 = 13;
+enum Tvc1Vec { S_U = 0, S_X, S_B1, S_B2, S_R, S_RT, S_P0, S_P1, S_Q, S_UC, S_UH, S_VH, S_XMIN };
+
+// Thread mapping inside a slab: thread t owns row iz = t % N of the columns
+// lc = t / N, t / N + G, ... (G = TVC_THREADS / N column groups; N <= 512).
+struct TvcCtx {
+    float *sm;        // this CTA's vectors
+    const float *sl;  // left neighbour's vectors (rank - 1), or null
+    const float *sr;  // right neighbour's vectors (rank + 1), or null
+    int N, nloc, nl, ix0, iz, G, lc0;
+    bool zlo, zhi;
+};
+
 
 // the Bregman quantities b = Bub - d and b - d of one pixel from its Bub pair
 __device__ __forceinline__ void tvc_bd(float a1, float a2, float mu, float &b1, float &b2,
@@ -315,33 +329,66 @@ __device__ __forceinline__ void tvc_bd(float a1, float a2, float mu, float &b1, 
     c2 = b2 - d2;
 }
 
+// value of vector o at the left / right x-neighbour of (lc, iz), element l
+__device__ __forceinline__ float tvc_left(const TvcCtx &c, int o, int lc, int l) {
+    return lc == 0 ? c.sl[o + (c.nloc - 1) * c.N + c.iz] : c.sm[o + l - c.N];
+}
+__device__ __forceinline__ float tvc_right(const TvcCtx &c, int o, int lc, int l) {
+    return lc == c.nl - 1 ? c.sr[o + c.iz] : c.sm[o + l + c.N];
+}
+
+// (I + B'B) of vector oi at (lc, iz) (same stencil as tv_apply_M).  The
+// x-neighbours in the adjacent slabs are not read from oi there: halo(base,
+// k) recomputes them from that CTA's vectors (base = its shared memory, k =
+// the element), with the same float operations the owner used.
+template <class Halo>
+__device__ __forceinline__ float tvc_M(const TvcCtx &c, int oi, int lc, int l, Halo halo) {
+    const float *in = c.sm + oi;
+    const int ix = c.ix0 + lc;
+    const float v = in[l];
+    const float g1 = c.zlo ? v - in[l - 1] : 0.f;
+    const float g1n = c.zhi ? in[l + 1] - v : 0.f;
+    float g2 = 0.f, g2n = 0.f;
+    if (ix >= 1) g2 = v - (lc == 0 ? halo(c.sl, (c.nloc - 1) * c.N + c.iz) : in[l - c.N]);
+    if (ix + 1 < c.N) g2n = (lc == c.nl - 1 ? halo(c.sr, c.iz) : in[l + c.N]) - v;
+    return v + (g1 - g1n) + (g2 - g2n);
+}
+
 // Cluster-wide sums of two per-thread values, returned to every thread.
-// Each CTA pushes its two block sums into slot [par][rank] of every CTA of
-// the cluster (remote stores, then the barrier), and every thread adds the C
-// slots of its own CTA in rank order: bitwise-identical results in all
+// Each CTA pushes its block sums into slot [par][slab] of every CTA of
+// the cluster (remote stores, then the barrier), and every thread adds the
+// slots of its own CTA in slab order: bitwise-identical results in all
 // threads of all CTAs, so every thread evaluates the scalar recurrences
 // itself and all take the same branches (no broadcast barrier).  Sums and
 // scalars are FP32 like the vectors: they lie on every CGS step's critical
-// path, and FP64 latency on GB300 is long.
-__device__ __forceinline__ void tvc_reduce(float a, float b, float &A, float &B, float *wsum,
-                                           float *red, int &par, int C, int rank) {
+// path, and FP64 latency on GB300 is long.  VR: slabs per CTA, each with
+// sums of its own (a[v], b[v]), so that a cluster of half the CTAs adds as
+// the whole one does.
+template <int VR>
+__device__ __forceinline__ void tvc_reduce(const float (&a_)[VR], const float (&b_)[VR], float &A,
+                                           float &B, float *wsum, float *red, int &par, int C,
+                                           int rank) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-    }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        wsum[wid] = a;
-        wsum[32 + wid] = b;
+#pragma unroll
+    for (int v = 0; v < VR; ++v) {
+        float a = a_[v], b = b_[v];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_down_sync(0xffffffffu, a, o);
+            b += __shfl_down_sync(0xffffffffu, b, o);
+        }
+        if (lane == 0) {
+            wsum[64 * v + wid] = a;
+            wsum[64 * v + 32 + wid] = b;
+        }
     }
     __syncthreads();
-    if (wid == 0) {
+    if (wid < VR) {
         constexpr int NW = TVC_THREADS / 32;
-        float da = lane < NW ? wsum[lane] : 0.f;
-        float db = lane < NW ? wsum[32 + lane] : 0.f;
+        float da = lane < NW ? wsum[64 * wid + lane] : 0.f;
+        float db = lane < NW ? wsum[64 * wid + 32 + lane] : 0.f;
 #pragma unroll
         for (int o = NW / 2; o > 0; o >>= 1) {
             da += __shfl_down_sync(0xffffffffu, da, o);
@@ -350,7 +397,8 @@ __device__ __forceinline__ void tvc_reduce(float a, float b, float &A, float &B,
         da = __shfl_sync(0xffffffffu, da, 0);
         db = __shfl_sync(0xffffffffu, db, 0);
         if (lane < C) {
-            float *dst = cl.map_shared_rank(red, lane) + (par * TVC_MAXC + rank) * 2;
+            float *dst =
+                cl.map_shared_rank(red, lane) + (par * TVC_MAXC + rank * VR + wid) * 2;
             dst[0] = da;
             dst[1] = db;
         }
@@ -359,21 +407,237 @@ __device__ __forceinline__ void tvc_reduce(float a, float b, float &A, float &B,
     const float *src = red + par * TVC_MAXC * 2;
     A = 0.f;
     B = 0.f;
-    for (int r = 0; r < C; ++r) {
+    for (int r = 0; r < C * VR; ++r) {
         A += src[2 * r];
         B += src[2 * r + 1];
     }
     par ^= 1;
 }
+__device__ __forceinline__ void tvc_reduce(float a, float b, float &A, float &B, float *wsum,
+                                           float *red, int &par, int C, int rank) {
+    const float a_[1] = {a}, b_[1] = {b};
+    tvc_reduce<1>(a_, b_, A, B, wsum, red, par, C, rank);
+}
+
+// loop over this thread's elements (lc, l) of the slab
+#define TVC_FOR(c) for (int lc = (c).lc0, l = lc * (c).N + (c).iz; lc < (c).nl; lc += (c).G, l += (c).G * (c).N)
+
+// CGS step structure (per step two cluster barriers, both inside the sums):
+//   uc = r + beta q ; p_new = uc + beta (q + beta p_old)     (local)
+//   __syncthreads ; vh = M p_new, halo p_new from the neighbour's r, q, p_old
+//   sum rt'vh -> alpha
+//   q = uc - alpha vh ; uh = uc + q ; x += alpha uh         (local)
+//   __syncthreads ; r -= alpha M uh, halo uh from the neighbour's uc, vh
+//   sum r'r, rt'r -> convergence, beta
+// p alternates between two buffers so that a neighbour can still read p_old
+// while this CTA writes p_new; every vector read remotely in a phase was
+// written before the barrier that opened the phase.
+__global__ void __launch_bounds__(TVC_THREADS, 2)
+    k_tv_prox_cl(const float *__restrict__ g_all, const TvState *__restrict__ st, double mu_const,
+                 int coupled, float *__restrict__ out_all, int N, int C, int nloc, float *) {
+    namespace cg = cooperative_groups;
+    extern __shared__ float4 tvc_smem[];
+    __shared__ float wsum[64];
+    __shared__ float red[2 * TVC_MAXC * 2];
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank();
+    const int w = blockIdx.x / C, gw = coupled ? 0 : w;
+    if (st && st[gw].done) return;  // uniform over the cluster
+    TvcCtx c;
+    c.sm = reinterpret_cast<float *>(tvc_smem);
+    c.N = N;
+    c.nloc = nloc;
+    c.ix0 = rank * nloc;
+    c.nl = max(0, min(nloc, N - c.ix0));
+    c.G = TVC_THREADS / N;
+    c.iz = threadIdx.x % N;
+    c.lc0 = (int)threadIdx.x / N;
+    if (c.lc0 >= c.G) c.lc0 = c.nl;  // idle thread: empty loops
+    c.zlo = c.iz >= 1;
+    c.zhi = c.iz + 1 < N;
+    c.sl = rank > 0 ? cl.map_shared_rank(c.sm, rank - 1) : nullptr;
+    c.sr = rank + 1 < C ? cl.map_shared_rank(c.sm, rank + 1) : nullptr;
+    const float mu = (float)(st ? st[gw].mu : mu_const);
+    const float *g = g_all + (size_t)w * N * N + (size_t)c.ix0 * N;
+    const int V = nloc * N;
+    float *S = c.sm;
+    int ou = S_U * V, ox = S_X * V;  // swapped after every sweep
+    const int ob1 = S_B1 * V, ob2 = S_B2 * V, orr = S_R * V, ort = S_RT * V, oq = S_Q * V,
+              ouc = S_UC * V, ouh = S_UH * V, ovh = S_VH * V, oxm = S_XMIN * V;
+    int op = S_P0 * V, opo = S_P1 * V;  // p_new, p_old
+    int par = 0, n_sweeps = 0, n_cg = 0;
+    float A = 0.f, B = 0.f;
+    float n2b = 0.f, rho = 0.f, rho1 = 1.f, normrmin = 0.f;
+    TVC_FOR(c) {
+        S[ou + l] = g[l];
+        S[ob1 + l] = 0.f;
+        S[ob2 + l] = 0.f;
+    }
+    cl.sync();
+    for (int it = 0; it < TV_SB_MAX; ++it) {
+        ++n_sweeps;
+        // rhs = g - B'(b - d); r = rt = rhs; x = xmin = 0
+        float n2 = 0.f;
+        TVC_FOR(c) {
+            const int ix = c.ix0 + lc;
+            float b1, b2, c1, c2, t1, t2, e1, e2;
+            tvc_bd(S[ob1 + l], S[ob2 + l], mu, b1, b2, c1, c2);
+            float acc = 0.f;
+            if (c.zlo) acc += c1;
+            if (c.zhi) {
+                tvc_bd(S[ob1 + l + 1], S[ob2 + l + 1], mu, t1, t2, e1, e2);
+                acc -= e1;
+            }
+            float acc2 = 0.f;
+            if (ix >= 1) acc2 += c2;
+            if (ix + 1 < N) {
+                tvc_bd(tvc_right(c, ob1, lc, l), tvc_right(c, ob2, lc, l), mu, t1, t2, e1, e2);
+                acc2 -= e2;
+            }
+            const float rhs = g[l] - (acc + acc2);
+            S[orr + l] = rhs;
+            S[ort + l] = rhs;
+            S[ox + l] = 0.f;
+            S[oxm + l] = 0.f;
+            n2 = fmaf(rhs, rhs, n2);
+        }
+        tvc_reduce(n2, 0.f, A, B, wsum, red, par, C, rank);
+        n2b = sqrtf(A);
+        rho = A;  // rt' r of the first step (rt = r = rhs)
+        rho1 = 1.f;
+        normrmin = n2b;
+        float beta_next = 0.f;
+        bool converged = false;
+        if (n2b > 0.f) {
+            for (int cit = 0; cit < TV_CG_MAX; ++cit) {
+                ++n_cg;
+                const float beta = beta_next;
+                {
+                    const int t = op;
+                    op = opo;
+                    opo = t;
+                }
+                if (cit == 0) {
+                    TVC_FOR(c) {
+                        const float rv = S[orr + l];
+                        S[ouc + l] = rv;
+                        S[op + l] = rv;
+                    }
+                } else {
+                    TVC_FOR(c) {
+                        const float qv = S[oq + l];
+                        const float uv = fmaf(beta, qv, S[orr + l]);
+                        S[ouc + l] = uv;
+                        S[op + l] = fmaf(beta, fmaf(beta, S[opo + l], qv), uv);
+                    }
+                }
+                __syncthreads();  // p_new complete in this slab
+                const bool first = cit == 0;
+                const int opo_ = opo;
+                auto halo_p = [=](const float *b, int k) {
+                    const float rv = b[orr + k];
+                    if (first) return rv;
+                    const float qv = b[oq + k];
+                    const float uv = fmaf(beta, qv, rv);
+                    return fmaf(beta, fmaf(beta, b[opo_ + k], qv), uv);
+                };
+                float a_rtvh = 0.f;
+                TVC_FOR(c) {
+                    const float vhv = tvc_M(c, op, lc, l, halo_p);
+                    S[ovh + l] = vhv;
+                    a_rtvh = fmaf(S[ort + l], vhv, a_rtvh);
+                }
+                tvc_reduce(a_rtvh, 0.f, A, B, wsum, red, par, C, rank);
+                if (A == 0.f || !isfinite(A)) break;
+                const float alpha = rho / A;
+                TVC_FOR(c) {
+                    const float uv = S[ouc + l];
+                    const float qq = fmaf(-alpha, S[ovh + l], uv);
+                    S[oq + l] = qq;
+                    const float uh = uv + qq;
+                    S[ouh + l] = uh;
+                    S[ox + l] = fmaf(alpha, uh, S[ox + l]);
+                }
+                __syncthreads();  // uh complete in this slab
+                auto halo_uh = [=](const float *b, int k) {
+                    const float uv = b[ouc + k];
+                    return uv + fmaf(-alpha, b[ovh + k], uv);
+                };
+                float a_rr = 0.f, a_rtr = 0.f;
+                TVC_FOR(c) {
+                    const float rv = fmaf(-alpha, tvc_M(c, ouh, lc, l, halo_uh), S[orr + l]);
+                    S[orr + l] = rv;
+                    a_rr = fmaf(rv, rv, a_rr);
+                    a_rtr = fmaf(S[ort + l], rv, a_rtr);
+                }
+                tvc_reduce(a_rr, a_rtr, A, B, wsum, red, par, C, rank);
+                int f = 0;
+                {
+                    const float normr = sqrtf(A);
+                    if (normr <= 1e-5f * n2b) {
+                        f = TVB_CONVERGED;
+                    } else {
+                        if (normr < normrmin) {
+                            normrmin = normr;
+                            f |= TVB_IMPROVED;
+                        }
+                        rho1 = rho;
+                        rho = B;  // rt' r of the next step
+                        if (rho == 0.f || !isfinite(rho))
+                            f |= TVB_BREAK;
+                        else
+                            beta_next = rho / rho1;
+                    }
+                }
+                if (f & TVB_CONVERGED) {
+                    converged = true;
+                    break;
+                }
+                if (f & TVB_IMPROVED) {
+                    TVC_FOR(c) S[oxm + l] = S[ox + l];
+                }
+                if (f & TVB_BREAK) break;
+            }
+        }
+        if (!converged) {
+            TVC_FOR(c) S[ox + l] = S[oxm + l];
+        }
+        cl.sync();  // new u (in x) complete in every slab
+        // Bub = B u + b ; change of u
+        float dif = 0.f, nrm = 0.f;
+        TVC_FOR(c) {
+            float b1, b2, c1, c2;
+            tvc_bd(S[ob1 + l], S[ob2 + l], mu, b1, b2, c1, c2);
+            const float v = S[ox + l];
+            S[ob1 + l] = (c.zlo ? v - S[ox + l - 1] : 0.f) + b1;
+            S[ob2 + l] = (c.ix0 + lc >= 1 ? v - tvc_left(c, ox, lc, l) : 0.f) + b2;
+            const float e = S[ou + l] - v;
+            dif = fmaf(e, e, dif);
+            nrm = fmaf(v, v, nrm);
+        }
+        tvc_reduce(dif, nrm, A, B, wsum, red, par, C, rank);
+        const bool stop = !(B > 0.f) || sqrtf(A / B) <= 1e-3f;
+        const int t = ou;
+        ou = ox;
+        ox = t;
+        if (stop) break;
+    }
+    float *o = out_all + (size_t)w * N * N + (size_t)c.ix0 * N;
+    TVC_FOR(c) o[l] = S[ou + l];
+    if (rank == 0 && threadIdx.x == 0) {
+        atomicAdd(&g_tv_stats[0], (unsigned long long)n_sweeps);
+        atomicAdd(&g_tv_stats[1], (unsigned long long)n_cg);
+    }
+    cl.sync();  // no CTA leaves while a neighbour may still read its shared memory
+}
+#undef TVC_FOR
 
 // The cluster prox: 4 consecutive z-pixels per thread, columns padded to P =
 // N rounded up to 4 (the pad pixels stay 0), 128-bit shared-memory accesses;
 // thread t owns group jz = t % (P/4) (pixels 4 jz .. 4 jz + 3) of the columns
 // lc = t / (P/4), ... + G.  Its CGS step carries M p and M q instead of p and
 // uh (M = I + B'B is linear, so M p_new = M uc + beta (M q + beta M p_old) and
-// M uh = M uc + M q, M q = M uc - alpha M vh), which saves a CTA barrier.
-// Sides that are no multiple of 4 had a kernel of a pixel per thread: 28 images
-// of 199 x 199 2.77 ms, now 1.13; 81 x 81 0.57, now 0.45:
+// M uh = M uc + M q, M q = M uc - alpha M vh), which saves a CTA barrier:
 //   A  uc = r + beta q                                        (local)
 //      __syncthreads
 //   B  Muc = M uc (halo uc from the neighbour's r, q); vh = Muc + beta (Mq +
@@ -388,12 +652,16 @@ __device__ __forceinline__ void tvc_reduce(float a, float b, float &A, float &B,
 // KM > 0: a thread owns at most KM groups and keeps the vectors that no other
 // thread reads (rt, M uc, M q) in registers: nine vectors of shared memory
 // instead of twelve, so that larger images fit a smaller cluster, which
-// matters because the barriers and not the pixels bound a step: an image of
-// 200 x 200 takes 0.53 ms with 16 CTAs and 0.58 with 8 (with thirteen vectors
-// in shared memory it needed the 16: 0.57), and twice as many clusters of 8 run at once --
-// 8 images 0.60 ms (was 1.01), 28 images 1.06 (was 1.90).  One CTA per SM
-// and 128 registers; KM = 4 spills a little (160 x 160 px: 0.72 ms with
-// 4 CTAs, 0.48 with 8 and KM = 2).
+// matters because the barriers and not the pixels bound a step and because
+// twice as many clusters of half the CTAs run at once.  One CTA per SM and 128
+// registers; KM = 4 spills a little.
+//
+// VR = 2: a CTA owns two slabs of the split that the sums follow (tvc_slabs),
+// with partial sums of their own, so a cluster of 8 gives the bits of one of 16:
+// 28 images of 200 x 200 px 3.14 ms (all vectors in shared memory, 16 CTAs) ->
+// 2.08 ms, 8 images 1.66 -> 1.15.  A slab per CTA without regard to the former
+// split would save a group of four per thread (about 25 %), but other sums are
+// other images: the TV solve amplifies a last bit.
 // ---------------------------------------------------------------------------
 struct F4 {
     float v[4];
@@ -409,7 +677,7 @@ __device__ __forceinline__ void st4(float *p, const F4 &a) {
 struct Tvc4Ctx {
     float *sm;
     const float *sl, *sr;
-    int N, P, nloc, nl, ix0, iz0, G, lc0;  // P: N rounded up to 4, a column's stride
+    int N, P, nloc, nv, nl, ix0, iz0, G, lc0;  // P: N rounded up to 4, a column's stride
 };
 
 // a neighbour slab's float4: shared memory of the neighbour CTA, or (GM)
@@ -453,22 +721,27 @@ __device__ __forceinline__ F4 tvc4_M(const Tvc4Ctx &c, int oi, int lc, int l, Ha
     return o;
 }
 
-// loop over this thread's groups e (lc, l); KU copies of the body
+// loop over this thread's groups (lc, l).  KM: groups e, KM / VR in each slab v
 #define TVC4_FOR(c)                                                                        \
     _Pragma("unroll KU") for (int e = 0, lc = (c).lc0, l = lc * (c).P + (c).iz0;           \
                               KM ? e < KM : lc < (c).nl;                                   \
-                              ++e, lc += (c).G, l += (c).G * (c).P) if (!KM || lc < (c).nl)
+                              ++e, lc = KM ? e / KV * (c).nv + (c).lc0 + e % KV * (c).G    \
+                                           : lc + (c).G,                                   \
+                                   l = lc * (c).P + (c).iz0)                               \
+        if (const int vs = KM ? e / KV : 0;                                                \
+            !KM || ((c).lc0 + e % KV * (c).G < (c).nv && lc < (c).nl))
 
-template <bool GM, int KM, bool RAG>
+template <bool GM, int KM, bool RAG, int VR = 1>
 __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
     k_tv_prox_cl4(const float *__restrict__ g_all, const TvState *__restrict__ st,
                   double mu_const, int coupled, float *__restrict__ out_all, int N, int C,
                   int nloc, float *__restrict__ gwork) {
     namespace cg = cooperative_groups;
     static_assert(!GM || (KM == 0 && !RAG), "global vectors: none in registers, N % 4 == 0");
-    constexpr int KU = KM ? KM : 1;
+    static_assert(VR == 1 || (KM > 0 && KM % VR == 0), "slabs of a CTA: whole groups each");
+    constexpr int KU = KM ? KM : 1, KV = KM ? KM / VR : 1;
     extern __shared__ float4 tvc_smem[];
-    __shared__ float wsum[64];
+    __shared__ float wsum[64 * VR];
     __shared__ float red[2 * TVC_MAXC * 2];
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
@@ -477,6 +750,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
     Tvc4Ctx c;
     c.N = N;
     c.nloc = nloc;
+    c.nv = nloc / VR;
     c.ix0 = rank * nloc;
     c.nl = max(0, min(nloc, N - c.ix0));
     const int P = RAG ? (N + 3) / 4 * 4 : N, NG = P / 4;
@@ -484,7 +758,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
     c.G = TVC_THREADS / NG;
     c.iz0 = 4 * ((int)threadIdx.x % NG);
     c.lc0 = (int)threadIdx.x / NG;
-    if (c.lc0 >= c.G) c.lc0 = c.nl;  // idle thread
+    if (c.lc0 >= c.G) c.lc0 = nloc;  // idle thread
     if constexpr (GM) {
         // slabs of the cluster's CTAs are consecutive in the workspace
         const size_t slab = (size_t)TVC_NV * nloc * P;
@@ -541,7 +815,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
     cl.sync();
     for (int it = 0; it < TV_SB_MAX; ++it) {
         ++n_sweeps;
-        float n2 = 0.f;
+        float n2[VR] = {}, zero[VR] = {};
         TVC4_FOR(c) {
             const int ix = c.ix0 + lc;
             const F4 B1 = ld4(S + ob1 + l), B2 = ld4(S + ob2 + l), G4 = image(lc, l);
@@ -577,14 +851,14 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
                 if (ix >= 1) acc2 += c2[k];
                 if (ix + 1 < N) acc2 -= e2r[k];
                 rh.v[k] = RAG && iz >= N ? 0.f : G4.v[k] - (acc + acc2);
-                n2 = fmaf(rh.v[k], rh.v[k], n2);
+                n2[vs] = fmaf(rh.v[k], rh.v[k], n2[vs]);
             }
             st4(S + orr + l, rh);
             put(rrt[KM ? e : 0], ort + l, rh);
             st4(S + ox + l, zero4);
             st4(S + oxm + l, zero4);
         }
-        tvc_reduce(n2, 0.f, A, B, wsum, red, par, C, rank);
+        tvc_reduce<VR>(n2, zero, A, B, wsum, red, par, C, rank);
         n2b = sqrtf(A);
         rho = A;
         rho1 = 1.f;
@@ -621,7 +895,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
                     for (int m = 0; m < 4; ++m) o.v[m] = fmaf(beta, qv.v[m], rv.v[m]);
                     return o;
                 };
-                float a_rtvh = 0.f;
+                float a_rtvh[VR] = {};
                 TVC4_FOR(c) {
                     const F4 muc = tvc4_M<RAG>(c, ouc, lc, l, halo_uc);
                     put(rmuc[KM ? e : 0], omuc + l, muc);
@@ -635,15 +909,15 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
                     st4(S + ovh + l, vh);
                     const F4 rt = get(rrt[KM ? e : 0], ort + l);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) a_rtvh = fmaf(rt.v[k], vh.v[k], a_rtvh);
+                    for (int k = 0; k < 4; ++k) a_rtvh[vs] = fmaf(rt.v[k], vh.v[k], a_rtvh[vs]);
                 }
-                tvc_reduce(a_rtvh, 0.f, A, B, wsum, red, par, C, rank);
+                tvc_reduce<VR>(a_rtvh, zero, A, B, wsum, red, par, C, rank);
                 if (A == 0.f || !isfinite(A)) break;
                 const float alpha = rho / A;
                 // C: Mvh = M vh (halo vh read from the neighbour); q = uc - alpha vh,
                 //    Mq = Muc - alpha Mvh, x += alpha (uc + q), r -= alpha (Muc + Mq)
                 auto halo_vh = [=](const float *b, int k) { return ld4n<GM>(b + ovh + k); };
-                float a_rr = 0.f, a_rtr = 0.f;
+                float a_rr[VR] = {}, a_rtr[VR] = {};
                 TVC4_FOR(c) {
                     const F4 mv = tvc4_M<RAG>(c, ovh, lc, l, halo_vh);
                     const F4 uv = ld4(S + ouc + l), vh = ld4(S + ovh + l);
@@ -657,15 +931,15 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
                         mq.v[k] = fmaf(-alpha, mv.v[k], muc.v[k]);
                         xn.v[k] = fmaf(alpha, uv.v[k] + q.v[k], xv.v[k]);
                         rn.v[k] = fmaf(-alpha, muc.v[k] + mq.v[k], rv.v[k]);
-                        a_rr = fmaf(rn.v[k], rn.v[k], a_rr);
-                        a_rtr = fmaf(rt.v[k], rn.v[k], a_rtr);
+                        a_rr[vs] = fmaf(rn.v[k], rn.v[k], a_rr[vs]);
+                        a_rtr[vs] = fmaf(rt.v[k], rn.v[k], a_rtr[vs]);
                     }
                     st4(S + oq + l, q);
                     put(rmq[KM ? e : 0], omq + l, mq);
                     st4(S + ox + l, xn);
                     st4(S + orr + l, rn);
                 }
-                tvc_reduce(a_rr, a_rtr, A, B, wsum, red, par, C, rank);
+                tvc_reduce<VR>(a_rr, a_rtr, A, B, wsum, red, par, C, rank);
                 int f = 0;
                 {
                     const float normr = sqrtf(A);
@@ -698,7 +972,7 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
             TVC4_FOR(c) st4(S + ox + l, ld4(S + oxm + l));
         }
         cl.sync();
-        float dif = 0.f, nrm = 0.f;
+        float dif[VR] = {}, nrm[VR] = {};
         TVC4_FOR(c) {
             const int ix = c.ix0 + lc;
             const F4 B1 = ld4(S + ob1 + l), B2 = ld4(S + ob2 + l), X = ld4(S + ox + l),
@@ -715,18 +989,18 @@ __global__ void __launch_bounds__(TVC_THREADS, KM ? 1 : 2)
             for (int k = 0; k < 4; ++k) {
                 float b1, b2, cc1, cc2;
                 tvc_bd(B1.v[k], B2.v[k], mu, b1, b2, cc1, cc2);
-                const float v = X.v[k];
-                n1.v[k] = (c.iz0 + k >= 1 ? v - xa[k] : 0.f) + b1;
-                n2v.v[k] = (ix >= 1 ? v - Lx.v[k] : 0.f) + b2;
+                const float xk = X.v[k];
+                n1.v[k] = (c.iz0 + k >= 1 ? xk - xa[k] : 0.f) + b1;
+                n2v.v[k] = (ix >= 1 ? xk - Lx.v[k] : 0.f) + b2;
                 if (RAG && c.iz0 + k >= N) n1.v[k] = n2v.v[k] = 0.f;
-                const float e = U.v[k] - v;
-                dif = fmaf(e, e, dif);
-                nrm = fmaf(v, v, nrm);
+                const float ch = U.v[k] - xk;
+                dif[vs] = fmaf(ch, ch, dif[vs]);
+                nrm[vs] = fmaf(xk, xk, nrm[vs]);
             }
             st4(S + ob1 + l, n1);
             st4(S + ob2 + l, n2v);
         }
-        tvc_reduce(dif, nrm, A, B, wsum, red, par, C, rank);
+        tvc_reduce<VR>(dif, nrm, A, B, wsum, red, par, C, rank);
         const bool stop = !(B > 0.f) || sqrtf(A / B) <= 1e-3f;
         const int t = ou;
         ou = ox;
@@ -875,45 +1149,60 @@ __global__ void __launch_bounds__(TV_RED)
     tv_store(a_as, part, TS_AS, W, sh);
 }
 
-// sum of the partials of group g, by the whole warp (every lane returns it): a
-// coupled stack of 28 has 616 of them per sum, which one thread added in 60 us
+// sum of the partials of group g in their order, by a warp whose lanes load 32
+// at a time (every lane returns it): a coupled stack of 28 has 616 of them per
+// sum, which one thread loaded and added in 60 us.  In order, because the step
+// size follows from the sums and the solve amplifies a last bit.
 __device__ double tv_group(const double *part, int q, int g, int W, int G, int coupled) {
     const double *p = part + ((size_t)q * W + (coupled ? 0 : g)) * G;
-    const int n = coupled ? W * G : G;
-    double s = 0.0;
-    for (int k = threadIdx.x & 31; k < n; k += 32) s += p[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const int n = coupled ? W * G : G, lane = threadIdx.x & 31;
+    double s = 0.0, next = lane < n ? p[lane] : 0.0;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const double v = next;
+        next = k0 + 32 + lane < n ? p[k0 + 32 + lane] : 0.0;
+        const int m = min(32, n - k0);
+        for (int i = 0; i < m; ++i) s += __shfl_sync(0xffffffffu, v, i);
+    }
     return s;
 }
 
 // stage 0: objective of the start point, alpha = 1.
 // stage 1: after a step: new objective, BB alpha, stop test (StopCriterion 1).
-__global__ void k_tv_scalar(int stage, const double *part, int G, int W, int coupled, double tau,
-                            double lambda, double beta, double tol, TvState *st) {
+// A warp per (group, sum), then a thread per group.
+constexpr int TV_SC_THREADS = 1024, TV_SC_GROUPS = 64;  // groups whose sums are held at once
+__global__ void __launch_bounds__(TV_SC_THREADS) k_tv_scalar(int stage, const double *part, int G,
+                                                             int W, int coupled, double tau,
+                                                             double lambda, double beta,
+                                                             double tol, TvState *st) {
+    __shared__ double sums[TV_SC_GROUPS][TS_N];
     const int n = coupled ? 1 : W;
-    for (int g = threadIdx.x >> 5; g < n; g += blockDim.x >> 5) {
-        TvState &s = st[g];
-        if (stage == 1 && s.done) continue;  // uniform in the warp
-        const double f = 0.5 * (tv_group(part, TS_RS, g, W, G, coupled) +
-                                tv_group(part, TS_RI, g, W, G, coupled)) +
-                         tau * tv_group(part, TS_PHI, g, W, G, coupled);
-        const double dd = stage ? tv_group(part, TS_DX, g, W, G, coupled) : 0.0;
-        const double as = stage ? tv_group(part, TS_AS, g, W, G, coupled) : 0.0;
-        if ((threadIdx.x & 31) != 0) continue;
-        if (stage == 0) {
-            s.f = f;
-            s.alpha = 1.0;
-            s.done = 0;
-        } else {
-            const double prev = s.f;
-            s.f = f;
-            const double dgd = lambda * as + beta * dd;
-            const double a = dgd / (2.2250738585072014e-308 + dd);  // realmin guard
-            s.alpha = fmin(1e30, fmax(1e-30, a));
-            if (dd == 0.0 || fabs(f - prev) <= tol * fabs(prev)) s.done = 1;
+    for (int g0 = 0; g0 < n; g0 += TV_SC_GROUPS) {
+        const int m = min(TV_SC_GROUPS, n - g0);
+        for (int i = threadIdx.x >> 5; i < TS_N * m; i += TV_SC_THREADS / 32) {
+            const double v = tv_group(part, i % TS_N, g0 + i / TS_N, W, G, coupled);
+            if ((threadIdx.x & 31) == 0) sums[i / TS_N][i % TS_N] = v;
         }
-        s.mu = tau / s.alpha;
+        __syncthreads();
+        TvState &s = st[g0 + min((int)threadIdx.x, m - 1)];
+        if ((int)threadIdx.x < m && !(stage == 1 && s.done)) {
+            const double *v = sums[threadIdx.x];
+            const double f = 0.5 * (v[TS_RS] + v[TS_RI]) + tau * v[TS_PHI];
+            if (stage == 0) {
+                s.f = f;
+                s.alpha = 1.0;
+                s.done = 0;
+            } else {
+                const double prev = s.f;
+                s.f = f;
+                const double dd = v[TS_DX];
+                const double dgd = lambda * v[TS_AS] + beta * dd;
+                const double a = dgd / (2.2250738585072014e-308 + dd);  // realmin guard
+                s.alpha = fmin(1e30, fmax(1e-30, a));
+                if (dd == 0.0 || fabs(f - prev) <= tol * fabs(prev)) s.done = 1;
+            }
+            s.mu = tau / s.alpha;
+        }
+        __syncthreads();
     }
 }
 
@@ -986,9 +1275,11 @@ int blocks_per_instance(int W) {
 std::atomic<int> g_prox_path{0};
 
 // cluster geometry of the shared-memory-resident prox for W images of N x N:
-// C CTAs per image, KM groups per thread with vectors in registers (0: none).
+// C CTAs per image with VR slabs each, KM groups per thread with vectors in
+// registers (0: none); one: the kernel of a pixel per thread.
 struct TvcGeom {
-    int C = 0, nloc = 0, KM = 0;
+    int C = 0, nloc = 0, KM = 0, VR = 1;
+    bool one = false;
     size_t smem = 0;
 };
 
@@ -999,21 +1290,35 @@ std::atomic<int> g_tv_cluster{0};
 constexpr size_t TVC_TWO = 113 * 1024, TVC_ONE = 225 * 1024;  // two CTAs per SM, one
 constexpr int TVC_KM = 4;                                     // most groups in registers
 
-// the geometry with C CTAs per image, C = 0 in it if the image does not fit
-TvcGeom tvc_fit(int N, int C) {
+// The slabs that an image's sums are added in, TVC_NV1 vectors each: as few as
+// fit two CTAs per SM (up to 8), else one (up to 16).  They are what the
+// bits of a result depend on, and the TV solve amplifies a last bit to 1e-3
+// of an image's rms at single pixels: whatever cluster runs, the slabs stay.
+// 0: more than 16.
+int tvc_slabs(int N) {
+    for (size_t most : {TVC_TWO, TVC_ONE})
+        for (int C = 1; C <= (most == TVC_ONE ? 16 : 8); C *= 2)
+            if ((size_t)TVC_NV1 * ((N + C - 1) / C) * N * sizeof(float) <= most) return C;
+    return 0;
+}
+
+// the geometry of C slabs, VR per CTA; C = 0 in it if the image does not fit
+TvcGeom tvc_fit(int N, int C, int VR = 1) {
     TvcGeom g;
-    const int nloc = (N + C - 1) / C, P = (N + 3) / 4 * 4;
+    const int nv = (N + C - 1) / C, P = (N + 3) / 4 * 4, nloc = VR * nv;
     size_t bytes = (size_t)TVC_NV * nloc * P * sizeof(float);
-    if (bytes > TVC_TWO) {
-        const int G = TVC_THREADS / (P / 4), km = std::max(2, (nloc + G - 1) / G);
+    if (bytes > TVC_TWO || VR > 1) {
+        const int G = TVC_THREADS / (P / 4);
+        const int km = VR > 1 ? VR * ((nv + G - 1) / G) : std::max(2, (nv + G - 1) / G);
         const size_t few = (size_t)TVC_NV_REG * nloc * P * sizeof(float);
-        if (km <= TVC_KM && few <= TVC_ONE) {
-            g.KM = km;
-            bytes = few;
-        }
+        if (km <= TVC_KM && few <= TVC_ONE)
+            g.KM = km, bytes = few;
+        else if (VR > 1)
+            return g;
     }
-    if (bytes > TVC_ONE) return TvcGeom();
-    g.C = C;
+    if (bytes > TVC_ONE) return g;
+    g.C = C / VR;
+    g.VR = VR;
     g.nloc = nloc;
     g.smem = bytes;
     return g;
@@ -1021,36 +1326,38 @@ TvcGeom tvc_fit(int N, int C) {
 
 int tvc_active(const TvcGeom &g, int N);
 
-// The smallest cluster whose slab fits two CTAs per SM (portable sizes up to
-// 8); else, one CTA per SM, the register form whose rounds of clusters cost
-// least: rounds x (1 + 2e-4 x pixels of a CTA), the slope fitted to one round
-// of 2600, 3200, 5000 and 6400 pixels (0.53, 0.48, 0.58, 0.72 ms).  So one
-// image of 200 x 200 has 16 CTAs and eight images have 8 each; 28 images of
-// 160 x 160 have 4 CTAs each (0.74 ms; with 8: 0.83).
+// Two CTAs per SM where the slabs fit; else the register form, one or two slabs
+// per CTA, whichever's rounds of clusters cost less: rounds x (1 + 2e-4 x pixels
+// of a CTA).  SB_ITV2 in ms with one / two slabs per CTA: 200 x 200 px, 1, 6, 8,
+// 16, 28 images: 0.88 / 1.14, 0.89 / 1.14, 1.55 / 1.14, 2.21 / 2.06, 2.88 / 2.08;
+// 160 x 160 px, 1, 12, 16, 28: 0.77 / 1.10, 0.79 / 1.12, 1.34 / 1.13, 1.34 / 1.13.
+// Sides that are no multiple of 4 take the kernel of a pixel per thread (g.one)
+// where its slabs fit, and above that (265 px) the padded columns instead of
+// k_tv_prox (one image of 302 x 302 px 31 -> 1.25 ms).
 TvcGeom tvc_geometry(int N, int W, int force = 0) {
     if (N > TVC_THREADS) return TvcGeom();
     if (const int Cf = force ? force : g_tv_cluster.load())
         // negative: no shared-memory geometry, the global-memory form
         return Cf < 0 ? TvcGeom() : tvc_fit(N, Cf);
-    for (int C = 1; C <= 8; C *= 2) {
-        const TvcGeom g = tvc_fit(N, C);
-        if (g.C && g.KM == 0 && g.smem <= TVC_TWO) return g;
+    const int slabs = tvc_slabs(N);
+    if (N % 4 && slabs) {
+        TvcGeom g;
+        g.one = true;
+        g.C = slabs;
+        g.nloc = (N + slabs - 1) / slabs;
+        g.smem = (size_t)TVC_NV1 * g.nloc * N * sizeof(float);
+        return g;
     }
-    TvcGeom best, smallest;
-    double cost = 1e30;
-    for (int C = 16; C >= 1; C /= 2) {
-        const TvcGeom g = tvc_fit(N, C);
-        if (!g.C) break;
-        smallest = g;
-        const int act = g.KM ? tvc_active(g, N) : 0;
-        if (act < 1) continue;
-        const double t = (double)((W + act - 1) / act) * (1.0 + 2e-4 * g.nloc * N);
-        if (t < cost) {
-            cost = t;
-            best = g;
-        }
-    }
-    return best.C ? best : smallest;
+    const TvcGeom g1 = tvc_fit(N, slabs ? slabs : 16);
+    if (!g1.KM || g1.C == 1) return g1;
+    const TvcGeom g2 = tvc_fit(N, g1.C, 2);
+    if (!g2.C || N % 4) return g1;
+    const int a1 = tvc_active(g1, N), a2 = tvc_active(g2, N);
+    if (a2 < 1) return g1;
+    auto cost = [&](const TvcGeom &g, int act) {
+        return (double)((W + act - 1) / act) * (1.0 + 2e-4 * g.nloc * N);
+    };
+    return a1 < 1 || cost(g2, a2) < cost(g1, a1) ? g2 : g1;
 }
 
 using TvcKernel = void (*)(const float *, const TvState *, double, int, float *, int, int, int,
@@ -1085,6 +1392,9 @@ static cudaError_t tvc_config(TvcKernel kern, const TvcGeom &gm, int W, cudaStre
 
 template <bool RAG>
 TvcKernel tvc_kernel(const TvcGeom &g) {
+    if constexpr (!RAG)
+        if (g.VR == 2)
+            return g.KM == 2 ? k_tv_prox_cl4<false, 2, false, 2> : k_tv_prox_cl4<false, 4, false, 2>;
     switch (g.KM) {
     case 2: return k_tv_prox_cl4<false, 2, RAG>;
     case 3: return k_tv_prox_cl4<false, 3, RAG>;
@@ -1093,6 +1403,7 @@ TvcKernel tvc_kernel(const TvcGeom &g) {
     }
 }
 TvcKernel tvc_kernel(const TvcGeom &g, int N) {
+    if (g.one) return k_tv_prox_cl;
     return N % 4 ? tvc_kernel<true>(g) : tvc_kernel<false>(g);
 }
 
@@ -1388,7 +1699,7 @@ int msot_rec_nn_with_TV_reg(msot_plan_t plan, const float *d_b, float *d_rec, in
         MSOT_LAUNCH_CHECK();
         if ((r = apply_forward(pl, x, As, W, s))) return r;
         KLAUNCH(k_tv_rs0<<<grid, TV_RED, 0, s>>>(d_b, As, rs, ns, sl, W, part));
-        KLAUNCH(k_tv_scalar<<<1, 512, 0, s>>>(0, part, G, W, coupled, reg, 1.0, TV_BETA, 1e-8, sv));
+        KLAUNCH(k_tv_scalar<<<1, TV_SC_THREADS, 0, s>>>(0, part, G, W, coupled, reg, 1.0, TV_BETA, 1e-8, sv));
         MSOT_LAUNCH_CHECK();
         for (int k = 0; k < sparsa_iter; ++k) {
             if ((r = apply_transpose(pl, rs, atr, W, s))) return r;
@@ -1399,7 +1710,7 @@ int msot_rec_nn_with_TV_reg(msot_plan_t plan, const float *d_b, float *d_rec, in
             MSOT_LAUNCH_CHECK();
             if ((r = apply_forward(pl, dx, As, W, s))) return r;
             KLAUNCH(k_tv_rs<<<grid, TV_RED, 0, s>>>(rs, As, ns, sl, W, part));
-            KLAUNCH(k_tv_scalar<<<1, 512, 0, s>>>(1, part, G, W, coupled, reg, 1.0, TV_BETA, 1e-8,
+            KLAUNCH(k_tv_scalar<<<1, TV_SC_THREADS, 0, s>>>(1, part, G, W, coupled, reg, 1.0, TV_BETA, 1e-8,
                                                  sv));
             MSOT_LAUNCH_CHECK();
         }

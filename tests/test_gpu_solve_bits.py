@@ -58,6 +58,15 @@ CASES = [
     ("l2", 90, 40, 1300, 2),           # D no multiple of 8 pairs: the unfused update
     ("l1", 64, 64, 1300, 6),
 ]
+TV_CASES = [
+    ("tv", 48, 32, 1300, 5),           # coupled sums of five images
+    ("tv", 77, 32, 1300, 2),           # a side that is no multiple of four
+    ("prox", 136, 0, 0, 2),            # slabs of one CTA per SM
+    ("prox", 200, 0, 0, 1),
+    ("prox", 200, 0, 0, 12),           # two slabs per CTA
+    ("prox", 141, 0, 0, 3),
+    ("prox", 280, 0, 0, 1),            # beyond the slabs: vectors in registers or in L2
+]
 
 
 def digest(what, n, D, T, W):
@@ -95,8 +104,13 @@ def test_operator_and_solves_keep_their_bits(cuda, case):
     _check(case)
 
 
+@pytest.mark.parametrize("case", TV_CASES, ids=lambda c: "-".join(map(str, c)))
+def test_tv_keeps_its_bits(cuda, case):
+    _check(case)
+
+
 if __name__ == "__main__":
     import sys
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     sys.path[:0] = [root, os.path.join(root, "mb-rec-msot_gb300")]
-    print(json.dumps({"-".join(map(str, c)): digest(*c) for c in CASES}, indent=1))
+    print(json.dumps({"-".join(map(str, c)): digest(*c) for c in CASES + TV_CASES}, indent=1))

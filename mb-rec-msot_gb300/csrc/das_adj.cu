@@ -15,11 +15,17 @@
 // with one or two instances per thread (k_das_adj4: lanes over pixels, random
 // 16-byte rows) paid about 10 for a quarter of the values.  (pixel, detector) pairs come as 4 bytes, knot row
 // and g in fixed point, decoded once per 4 NI values.  Measured at batch 64,
-// 128 x 128 px, 256 detectors: 322 us (k_das_adj4) -> 211 us (NI = 32).
+// 128 x 128 px, 256 detectors: 329 us (k_das_adj4) -> 271 us (NI = 32).
 //
 // Bound: shared-memory wavefronts of the row reads, then the issue slots of
-// the decode and of the knot table (U and V run along the samples: 12
-// operations per knot triple instead of 4F).
+// the decode and of the knot table.  Every knot comes from its own window of
+// samples, as in k_das_adj4: sums that run along the samples (12 operations per
+// knot triple instead of 4F, 211 us) carry a NaN or a
+// spike's rounding to pixels whose taps do not meet it.
+//
+// For calls of the operator itself.  The iterative solves keep k_das_adj4
+// (apply_transpose): they amplify a last bit to 1e-3 of an image's rms at
+// single pixels, so their A^T keeps one order of its sums.
 #include <algorithm>
 
 #include "common.cuh"
@@ -32,6 +38,7 @@ template <int NI> constexpr int a5_threads = NI == 32 ? 512 : 256;
 // seg rows of NI + 2 words: even, for the knots' 8-byte loads, and staging
 // stores along t meet each bank twice only
 constexpr int A5_PAD = 2;
+constexpr int A5_RUN = 4;  // buckets that a thread tabulates from one window
 
 struct Adj5Const {
     float inv_r, ce1;       // 1 / r, (r - F) / r
@@ -172,42 +179,38 @@ __global__ void __launch_bounds__(a5_threads<NI>, NI == 32 ? 1 : 2) k_das_adj5(
         if (nb <= 0) continue;
         {
             // knots of buckets 0 .. nb (the last one's first row closes the
-            // table), in runs of `per` per thread: U and V from their sums at
-            // the run's start, then along the samples
-            const int per = (nb + NRUN) / NRUN;
-            const int b0 = run * per, b1 = min(nb + 1, b0 + per);
-            const float *g = seg0 + (size_t)buf * seg_rows * RS + inst + (size_t)(b0 + F) * RS;
-            if (b0 < b1) {
-                // two instances side by side in packed arithmetic
-                auto ld = [&](int k) { return *reinterpret_cast<const float2 *>(g + k * RS); };
-                auto two = [](float v) { return make_float2(v, v); };
-                const float2 m1 = two(-1.f);
-                float2 U = two(0.f), V0 = U, V1 = U;
+            // table), two instances side by side in packed arithmetic
+            constexpr int NWIN = 2 * F + 1 + A5_RUN;
+            auto two = [](float v) { return make_float2(v, v); };
+            for (int b0 = run * A5_RUN; b0 <= nb; b0 += NRUN * A5_RUN) {
+                const float *g = seg0 + (size_t)buf * seg_rows * RS + inst + (size_t)b0 * RS;
+                float2 win[NWIN];  // win[F + j]: sample b0 + j
 #pragma unroll
-                for (int k = F - 1; k >= 0; --k) {
-                    const float2 v = ld(-k);
-                    U = ffma2(two(1.f - (float)k * cst.inv_r), v, U);
-                    V0 = fadd2(V0, v);
-                }
-#pragma unroll
-                for (int k = F; k >= 1; --k) {
-                    const float2 v = ld(k);
-                    U = ffma2(two(1.f - (float)k * cst.inv_r), v, U);
-                    V1 = fadd2(V1, v);
-                }
-                float2 V = ffma2(V0, m1, V1), sl = ld(-F);
+                for (int j = 0; j < NWIN; ++j)
+                    win[j] = *reinterpret_cast<const float2 *>(g + j * RS);
                 float *row = K + (size_t)3 * b0 * NI + inst;
-                for (int b = b0; b < b1; ++b) {
-                    const float2 sh = ld(F + 1), s1 = ld(1), sn = ld(1 - F);
+#pragma unroll
+                for (int r = 0; r < A5_RUN; ++r, row += 3 * NI) {
+                    if (b0 + r > nb) break;
+                    float2 U = two(0.f), V0 = U, V1 = U;
+#pragma unroll
+                    for (int k = F - 1; k >= 0; --k) {
+                        const float2 v = win[r + F - k];
+                        U = ffma2(two(1.f - (float)k * cst.inv_r), v, U);
+                        V0 = fadd2(V0, v);
+                    }
+#pragma unroll
+                    for (int k = F; k >= 1; --k) {
+                        const float2 v = win[r + F + k];
+                        U = ffma2(two(1.f - (float)k * cst.inv_r), v, U);
+                        V1 = fadd2(V1, v);
+                    }
+                    const float2 V = ffma2(V0, two(-1.f), V1), sl = win[r],
+                                 sh = win[r + 2 * F + 1];
                     float2 *o = reinterpret_cast<float2 *>(row);
                     o[0] = ffma2(two(cst.ce1), sl, U);
                     o[NP] = ffma2(two(cst.q1), V, ffma2(two(cst.cl), sl, U));
                     o[2 * NP] = ffma2(two(cst.q2), V, ffma2(two(cst.ch), sh, U));
-                    row += 3 * NI;
-                    U = ffma2(two(cst.ce1), ffma2(sn, m1, sh), ffma2(V, two(cst.inv_r), U));
-                    V = fadd2(V, fadd2(ffma2(s1, m1, sh), ffma2(s1, m1, sn)));
-                    sl = sn;
-                    g += RS;
                 }
             }
         }
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(a5_threads<NI>, NI == 32 ? 1 : 2) k_das_adj5(
 
 static size_t adj5_smem(const Plan &pl, int ni) {
     return ((size_t)(3 * pl.adj5_span_max + 4) * ni +
-            (size_t)2 * (pl.adj5_span_max + 2 * pl.F + 3) * (ni + A5_PAD)) *
+            (size_t)2 * (pl.adj5_span_max + 2 * pl.F + 2 + A5_RUN) * (ni + A5_PAD)) *
            sizeof(float);
 }
 
@@ -298,7 +301,7 @@ static int adj5_launch(const Plan &pl, const float *raw, float *part, int W, int
     const dim3 grid(4 * pl.n_blk, div_up(W, NI), groups);
     KLAUNCH(k_das_adj5<NI, F><<<grid, a5_threads<NI>, smem, st>>>(
         pl.adj5_ent, pl.adj5_span, raw, part, pl.nx, pl.nz, pl.n_blk_x, pl.D, pl.T, W,
-        adj5_const(pl), pl.adj5_span_max + 2 * pl.F + 3, 3 * pl.adj5_span_max + 4, dpg, stride));
+        adj5_const(pl), pl.adj5_span_max + 2 * pl.F + 2 + A5_RUN, 3 * pl.adj5_span_max + 4, dpg, stride));
     MSOT_LAUNCH_CHECK();
     return MSOT_OK;
 }
@@ -327,17 +330,22 @@ static int adj5_ni(const Plan &pl, int W) {
     return ni >= 8 ? ni : 0;
 }
 
+// whether k_das_adj5 beats k_das_adj4 for W instances: odd batches (one instance
+// per CTA there) from 5 up, others where three quarters of the instance tiles
+// are filled.  k_das_adj4 / k_das_adj5 in us for 6, 8, 12, 18, 24, 64 images of
+// 128 x 128 px: 49 / 55, 50 / 54, 84 / 80, 100 / 128, 148 / 133, 329 / 271; 200 x 200 px,
+// 6, 8, 10, 16, 28: 123 / 128, 166 / 126, 214 / 206, 276 / 207, 403 / 366; 400 x 400 px,
+// 512 detectors, 5, 6, 8, 13: 1083 / 665, 523 / 668, 721 / 660, 2277 / 950
 bool adj5_usable(const Plan &pl, int W) {
-    // up to four instances k_das_adj4 is as fast or faster (W = 4: 63 us each at
-    // 128 x 128 px, 0.51 against 0.39 ms at 400 x 400 px, 512 detectors)
-    return pl.adj5_ent && W >= 5 && adj5_ni(pl, W);
+    const int ni = pl.adj5_ent && W >= 5 ? adj5_ni(pl, W) : 0;
+    return ni && (W % 2 || (W >= 8 && 4 * W >= 3 * ni * div_up(W, ni)));
 }
 
 int launch_das_adjoint5(const Plan &pl, const float *raw, float *x, int W, float scale,
                         cudaStream_t st) {
     const int ni = adj5_ni(pl, W);
     // detector groups: the fewest that come close to filling whole waves of two
-    // CTAs per SM (each group writes a partial image)
+    // CTAs per SM, one at NI = 32 (each group writes a partial image)
     const int base = 4 * pl.n_blk * div_up(W, ni), slots = (ni == 32 ? 1 : 2) * sm_count();
     const int most = std::max(1, std::min({pl.adj_groups_max * pl.max_batch / W, pl.D, 32}));
     int groups = 1;

@@ -1412,19 +1412,28 @@ static int sir_adj_nt(const Plan &pl, const float *raw, float *x, float scale, d
     return MSOT_EINVAL;
 }
 
-// k_sir_adj2 instead of k_sir_adj for W instances.  k_sir_adj runs the tri taps
-// for every sample of a column, a pass per two instances (0.565 of one per
-// single instance when W is odd): 4 + 0.0445 x mean column length x taps ns
-// per pixel and pass, 256 detectors.  k_sir_adj2 reads a window in rounds of 16
-// taps, much the same for every column: 30.5 ns per pixel for up to four
-// instances, 36.5 per eight.  k_sir_adj / k_sir_adj2 measured, 128^2 px (columns
-// of 31 samples, 12 taps): 357 / 460 us for two images, 591 / 465 for three,
-// 1184 / 626 for eight; 160^2 (26, 10): 688 / 758 for three, 860 / 760 for four;
-// 200^2 (22, 8): 823 / 1139 for three, 1578 / 1471 for eight.
+// k_sir_adj2 instead of k_sir_adj for W instances.
+//
+// Below seven samples of radius it is the more exact one too.  Error of A^T, arc of 256,
+// k_sir_adj / k_sir_adj2, on recordings of absorbers: 50 x 50 px 5.2e-6 / 7.4e-6, 60
+// 1.9e-6 / 2.5e-6, 78 (r = 8.8) 7.6e-7 / 7.5e-7, 92 6.4e-7 / 4.0e-7, 128 6.4e-7 / 2.9e-7;
+// on noise in the EIR's band with responses as wide as the pixel: 80 (8.6)
+// 3.5e-6 / 4.2e-6, 90 (7.6) 1.7e-6 / 1.9e-6, 95 (7.2) 1.34e-6 / 1.33e-6, 100 (6.8)
+// 1.10e-6 / 0.98e-6, 120 7.8e-7 / 5.3e-7.  A wider tri filter takes more of the
+// recording away, and k_sir_adj rounds after it, the composite rows before.
+//
+// The price: k_sir_adj runs the tri taps for every sample of a column, a pass per
+// two instances (0.565 of one per single instance when W is odd): 4 + 0.0445 x mean
+// column length x taps ns per pixel and pass, 256 detectors.  k_sir_adj2 reads a
+// window in rounds of 16 taps, much the same for every column: 30.5 ns per pixel
+// for up to four instances, 48 per eight.  k_sir_adj / k_sir_adj2 measured, 128^2 px
+// (columns of 31 samples, 12 taps): 358 / 505 us for two images, 592 / 508 for three,
+// 1187 / 740 for eight; 160^2 (26, 10): 689 / 814 for three, 862 / 814 for four, 1166 /
+// 1113 for five; 200^2 (22, 8): 823 / 1217 for three, 1579 / 1669 for eight.
 static bool sir_adj_composite(const Plan &pl, int W) {
-    if (!pl.sir_tab) return false;
+    if (!pl.sir_tab || pl.F > 6) return false;
     const double pass = 4.0 + 0.0445 * pl.sir_len_mean * (2 * pl.F + 2);
-    const double there = W <= 4 ? 30.5 : 36.5 * div_up(W, 8);
+    const double there = W <= 4 ? 30.5 : 48.0 * div_up(W, 8);
     return there <= pass * (W % 2 ? 0.565 : 0.5) * W;
 }
 

@@ -371,7 +371,7 @@ static int build(const msot_plan_desc *d, Plan &p) {
         (void)maxlen;
         const int rc = sir_build(p, tfx.data(), d->sir_idx, se, p.device_bytes);
         if (rc != MSOT_OK) return rc;
-        if (p.sir_tab) {  // k_sir_fwd's tables stay behind (k_sir_adj serves 1 and 2 images)
+        if (p.sir_tab) {  // k_sir_fwd's tables stay behind (k_sir_adj keeps its own: operator.cu)
             tpi.clear();
             spi.clear();
         }

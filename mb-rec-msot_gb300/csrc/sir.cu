@@ -14,12 +14,12 @@
 //               warps share the list and are summed at the end.  No atomics:
 //               deterministic, where the column in shared memory took one
 //               atomic (a compare-and-swap loop for FP32) per tap and instance.
-//   k_sir_adj2  half warp = pixel: lanes over the window's taps, per detector
+//   k_sir_adj2  half warp = two pixels: lanes over the window's taps, per detector
 //               one e[m] for all instances against the block's samples in
-//               shared memory, lanes reduced once per pixel.
+//               shared memory, the taps added before the next detector's.
 //
 // 128 x 128 px, 256 x 2030 samples, 8 instances, columns of 31 samples on
-// average: forward 2398 -> 515 us, adjoint 1214 -> 644 us.  Bound:
+// average: forward 2398 -> 515 us, adjoint 1187 -> 740 us.  Bound:
 // issue slots (address and window arithmetic per pair, one packed FMA per tap
 // and two instances) and the table rows' L1 lines.
 #include <algorithm>
@@ -173,8 +173,17 @@ __global__ void __launch_bounds__(32 * SF_WARPS) k_sir_fwd2(
 
 // CTA = (SA_PIX pixels, NI instances).  Per detector the samples that the
 // block's windows span (aspan) lie in shared memory, [sample][instance]; a
-// half warp takes a pixel, lanes over taps, the next detector's samples are
+// half warp takes two pixels, lanes over taps, the next detector's samples are
 // loaded into registers meanwhile.
+//
+// A detector's taps are added to one value before they enter the pixel's sum.
+// The composite row is smooth and the recordings oscillate, so taps cancel within
+// one detector and not tap by tap over the detectors: lanes that each kept a
+// tap's sum over all detectors lost a factor of 4 at 80 x 80 px and of 40 at 60 x
+// 60.  The half warp reduces and scatters: lane bits 3, 2, 1, 0 take the pixel, the
+// group of four instances and the instance in it, and each lane ends with one
+// (pixel, instance).  Pixels and groups sit in the lanes' registers in the order
+// that lets a lane send its second half as it is; no selection there.
 template <int NI>
 __global__ void __launch_bounds__(SA_THREADS) k_sir_adj2(
     const int4 *__restrict__ ent, const int2 *__restrict__ aspan, const float2 *__restrict__ tab,
@@ -182,17 +191,18 @@ __global__ void __launch_bounds__(SA_THREADS) k_sir_adj2(
     int span_max, int det_per_group, size_t part_stride) {
     constexpr int QN = NI / 4;                       // 16-byte groups per sample
     constexpr int PPH = SA_PIX / (SA_THREADS / 16);  // pixels per half warp
+    static_assert(PPH == 2 && (NI == 4 || NI == 8), "lane bits of the reduction");
     constexpr int NPRE = 3;                          // groups in flight per thread
     extern __shared__ float4 ys[];  // [2][QN][span_max]
     const int l = threadIdx.x & 15, half = threadIdx.x >> 4;
+    const int b3 = l >> 3, b2 = l >> 2 & 1, b1 = l >> 1 & 1, b0 = l & 1;
     const int blk = blockIdx.x, w0 = blockIdx.y * NI;
     const int4 *e = ent + (size_t)blk * D * SA_PIX;
     const size_t DT = (size_t)D * T;
-    float2 acc[PPH][NI / 2];
-#pragma unroll
-    for (int k = 0; k < PPH; ++k)
-#pragma unroll
-        for (int i = 0; i < NI / 2; ++i) acc[k][i] = make_float2(0.f, 0.f);
+    // slot k of a lane holds pixel k ^ b3 of its half warp, slot g (NI = 8) the
+    // instances 4 (g ^ b2) ..
+    const int pix[PPH] = {b3 * (SA_THREADS / 16) + half, (b3 ^ 1) * (SA_THREADS / 16) + half};
+    float sum = 0.f;
     float4 pre[NPRE];
     // group g of the staging: sample g / QN, instances 4 (g % QN) ..; zero outside
     // the row, instances past W repeat the last one and are not stored
@@ -218,7 +228,7 @@ __global__ void __launch_bounds__(SA_THREADS) k_sir_adj2(
             *slot(0, g) = load(d0, g, sp);
 #pragma unroll
         for (int k = 0; k < PPH; ++k)
-            qn[k] = __ldg(e + (size_t)d0 * SA_PIX + k * (SA_THREADS / 16) + half);
+            qn[k] = __ldg(e + (size_t)d0 * SA_PIX + pix[k]);
     }
     for (int d = d0; d < d1; ++d) {
         const int buf = (d - d0) & 1;
@@ -241,8 +251,13 @@ __global__ void __launch_bounds__(SA_THREADS) k_sir_adj2(
             const int last = max(se_len(qc[k].y) - 1, 0);
 #pragma unroll
             for (int h = 0; h < 3; ++h) tv[k][h] = __ldg(tab + qc[k].x + min(16 * h + l, last));
-            qn[k] = __ldg(e + (size_t)min(d + 1, D - 1) * SA_PIX + k * (SA_THREADS / 16) + half);
+            qn[k] = __ldg(e + (size_t)min(d + 1, D - 1) * SA_PIX + pix[k]);
         }
+        float2 acc[PPH][NI / 2];
+#pragma unroll
+        for (int k = 0; k < PPH; ++k)
+#pragma unroll
+            for (int i = 0; i < NI / 2; ++i) acc[k][i] = make_float2(0.f, 0.f);
 #pragma unroll
         for (int k = 0; k < PPH; ++k) {
             const int4 q = qc[k];
@@ -262,7 +277,7 @@ __global__ void __launch_bounds__(SA_THREADS) k_sir_adj2(
                     const int s = min(max(at + min(m, last), 0), span_max - 1);
 #pragma unroll
                     for (int g = 0; g < QN; ++g) {
-                        const float4 v = y[g * span_max + s];
+                        const float4 v = y[(QN == 2 ? g ^ b2 : g) * span_max + s];
                         if (m < len) {
                             acc[k][2 * g] = ffma2(e2, make_float2(v.x, v.y), acc[k][2 * g]);
                             acc[k][2 * g + 1] = ffma2(e2, make_float2(v.z, v.w), acc[k][2 * g + 1]);
@@ -271,6 +286,28 @@ __global__ void __launch_bounds__(SA_THREADS) k_sir_adj2(
                 }
             }
         }
+        // taps of this detector: the other lanes' parts of what this lane keeps
+        float2 v[NI / 2];
+#pragma unroll
+        for (int i = 0; i < NI / 2; ++i) {
+            v[i].x = acc[0][i].x + __shfl_xor_sync(0xffffffffu, acc[1][i].x, 8);
+            v[i].y = acc[0][i].y + __shfl_xor_sync(0xffffffffu, acc[1][i].y, 8);
+        }
+        if constexpr (NI == 8) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                v[i].x += __shfl_xor_sync(0xffffffffu, v[2 + i].x, 4);
+                v[i].y += __shfl_xor_sync(0xffffffffu, v[2 + i].y, 4);
+            }
+        }
+        const int hi = NI == 8 ? b1 : b2, lo = NI == 8 ? b0 : b1;
+        float2 u = hi ? v[1] : v[0];
+        const float2 o = hi ? v[0] : v[1];
+        u.x += __shfl_xor_sync(0xffffffffu, o.x, NI == 8 ? 2 : 4);
+        u.y += __shfl_xor_sync(0xffffffffu, o.y, NI == 8 ? 2 : 4);
+        float t = (lo ? u.y : u.x) + __shfl_xor_sync(0xffffffffu, lo ? u.x : u.y, NI == 8 ? 1 : 2);
+        if constexpr (NI == 4) t += __shfl_xor_sync(0xffffffffu, t, 1);
+        sum += t;
         if (d + 1 < d1) {
             const int n = QN * (sn.y - sn.x);
 #pragma unroll
@@ -281,17 +318,9 @@ __global__ void __launch_bounds__(SA_THREADS) k_sir_adj2(
                 *slot(buf ^ 1, g) = load(d + 1, g, sn);
         }
     }
-#pragma unroll
-    for (int k = 0; k < PPH; ++k) {
-        const int p = blk * SA_PIX + k * (SA_THREADS / 16) + half;
-#pragma unroll
-        for (int i = 0; i < NI; ++i) {
-            float v = i & 1 ? acc[k][i / 2].y : acc[k][i / 2].x;
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (l == 0 && p < P && w0 + i < W) out[blockIdx.z * part_stride + (size_t)(w0 + i) * P + p] = v;
-        }
-    }
+    const int p = blk * SA_PIX + pix[0], i = NI == 8 ? 4 * b2 + 2 * b1 + b0 : 2 * b2 + b1;
+    if ((NI == 8 || !b0) && p < P && w0 + i < W)
+        out[blockIdx.z * part_stride + (size_t)(w0 + i) * P + p] = sum;
 }
 
 // Tables of the two kernels from the travel times tfx [D][P], the 0-based
@@ -360,6 +389,7 @@ int sir_build(Plan &p, const int32_t *tfx, const int32_t *sidx, const std::vecto
     }
     int span = 1;
     for (const int2 &v : asp) span = std::max(span, v.y - v.x);
+    span = (span + 7) / 8 * 8;  // lanes of two groups of instances meet other banks
     if ((size_t)span * 2 * 32 > 100 * 1024) return MSOT_OK;  // two buffers of 8 instances
     p.sir_span_max = span;
     MSOT_CUDA_TRY(cudaMalloc(&p.sir_aspan, asp.size() * sizeof(int2)));

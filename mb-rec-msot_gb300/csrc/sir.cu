@@ -19,7 +19,7 @@
 //               shared memory, the taps added before the next detector's.
 //
 // 128 x 128 px, 256 x 2030 samples, 8 instances, columns of 31 samples on
-// average: forward 2398 -> 515 us, adjoint 1187 -> 740 us.  Bound:
+// average: forward 2398 -> 590 us, adjoint 1187 -> 740 us.  Bound:
 // issue slots (address and window arithmetic per pair, one packed FMA per tap
 // and two instances) and the table rows' L1 lines.
 #include <algorithm>
@@ -34,6 +34,10 @@
 namespace msot {
 
 constexpr int SF_T = 64, SF_WARPS = 4;      // forward: samples per CTA, warps sharing a list
+// chains of a sample's sum in each warp: a few hundred terms cancel to a tenth of them,
+// and one chain was less exact than the former kernel's atomics (128 x 128 px, one
+// image: 3.1e-6 of A x, there 2.2e-6, now 2.0e-6; 8 images 550 -> 624 us)
+constexpr int SF_CH = 2;
 constexpr int SA_THREADS = 256, SA_PIX = 32;  // adjoint: pixels per CTA, a half warp each
 
 // (A, B)[m] of every (column, piece), m = j + F + k over tri taps j = -F ..
@@ -88,9 +92,11 @@ __global__ void __launch_bounds__(32 * SF_WARPS) k_sir_fwd2(
     __shared__ float red[SF_WARPS - 1][NI][SF_T];
     const int d = blockIdx.y, w0 = blockIdx.z * NI, t0 = blockIdx.x * SF_T;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float2 acc[2][NP];  // samples t0 + lane and t0 + 32 + lane
+    // samples t0 + lane and t0 + 32 + lane, SF_CH chains each
+    float2 part[SF_CH][2][NP];
 #pragma unroll
-    for (int i = 0; i < NP; ++i) acc[0][i] = acc[1][i] = make_float2(0.f, 0.f);
+    for (int i = 0; i < SF_CH * 2 * NP; ++i)
+        part[i / (2 * NP)][i / NP % 2][i % NP] = make_float2(0.f, 0.f);
     // pairs whose window starts in (t0 - maxlen, t0 + 64)
     const int32_t *o = off + (size_t)d * (nj + 1);
     const int ja = min(max(t0 - maxlen + 1 - jmin, 0), nj), jb = min(max(t0 + SF_T - jmin, 0), nj);
@@ -145,11 +151,21 @@ __global__ void __launch_bounds__(32 * SF_WARPS) k_sir_fwd2(
                 const float2 e2 = make_float2(ev, ev);
                 if (m + 32u * h < len) {  // a NaN pixel reaches its own window only
 #pragma unroll
-                    for (int i = 0; i < NP; ++i) acc[h][i] = ffma2(e2, xv[u][i], acc[h][i]);
+                    for (int i = 0; i < NP; ++i)
+                        part[u % SF_CH][h][i] = ffma2(e2, xv[u][i], part[u % SF_CH][h][i]);
                 }
             }
         }
     }
+    float2 acc[2][NP];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            acc[h][i] = part[0][h][i];
+#pragma unroll
+            for (int c = 1; c < SF_CH; ++c) acc[h][i] = fadd2(acc[h][i], part[c][h][i]);
+        }
 #pragma unroll
     for (int i = 0; i < NI && warp > 0; ++i)
 #pragma unroll

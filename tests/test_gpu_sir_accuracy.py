@@ -49,3 +49,19 @@ def test_transpose_is_as_exact_in_a_batch(cuda, n, W):
     batch = rel(pm.transpose(torch.tensor(y)).cpu().numpy()[W - 1], ref)
     print(f"n {n} W {W}: alone {alone:.2e} batch {batch:.2e}")
     assert batch <= 1.1 * alone
+
+
+# the bars are the errors of k_sir_fwd (a column in shared memory, atomics) on these images
+@pytest.mark.parametrize("n,W,bar", [(78, 4, 7.9e-6), (100, 2, 3.8e-6), (128, 1, 2.2e-6),
+                                     (128, 8, 2.6e-6)])
+def test_forward_is_as_exact_as_with_atomics(cuda, n, W, bar):
+    import torch
+    pm, om = _pair(n, W)
+    x = np.linspace(-1, 1, n)
+    img = np.zeros((W, n, n), dtype=np.float32)
+    for cx, cz, r in ((-0.3, 0.2, 0.4), (0.5, 0.5, 0.15), (0.1, -0.6, 0.25), (-0.7, -0.7, 0.05)):
+        img += ((x[:, None] - cx) ** 2 + (x[None] - cz) ** 2 <= r * r).astype(np.float32)
+    ref = om.forward(img[:1].astype(np.float64))[0]
+    err = rel(pm.forward(torch.tensor(img)).cpu().numpy()[W - 1], ref)
+    print(f"n {n} W {W}: forward {err:.2e}")
+    assert err <= bar

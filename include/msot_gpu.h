@@ -390,24 +390,24 @@ int msot_butter_response(int order, int type, double wn1, double wn2, int n, int
 /* Autotuner (no reference counterpart): times the variants of the plan's
  * hot kernels on its own geometry at `batch` instances -- the DAS forward's
  * kernel (image values staged in shared memory per time tile and detector
- * group, or gathered per detector) and instances per CTA (8, 4, 2), the DAS
- * adjoint's instances per CTA (4, 2, 1), the register cap of the
- * IR convolution (1, 3, 4 resident CTAs per SM) and, for square grids, the
- * CTAs per image of the
- * SB_ITV2 cluster kernel (automatic, 1 .. 16, or -1: 16 CTAs with the
- * vectors in a global-memory workspace) -- and keeps the fastest in
- * the plan (they change results only in float summation order).  Drops the
- * plan's captured solver graphs.  Not concurrent with other calls on the
- * plan.  out (may be NULL) receives the choices and their times. */
+ * group, or gathered per detector) and instances per CTA (16, 8, 4, 2), the
+ * instances per CTA of the DAS adjoint that the solves run (4, 2, 1), the
+ * register cap of the IR convolution (1, 3, 4 resident CTAs per SM) and, for
+ * square grids, the CTAs per image of the SB_ITV2 cluster kernel (automatic,
+ * 1 .. 16, or -1: 16 CTAs with the vectors in a global-memory workspace) --
+ * and keeps, for batches of this size, those that beat the built-in choice by
+ * more than 3 per cent (they change results only in float summation order).
+ * Other batch sizes run the built-in choice.  Drops the plan's captured solver
+ * graphs.  Not concurrent with other calls on the plan.  out (may be NULL)
+ * receives what batches of this size run from now on, and the times. */
 typedef struct msot_tuning {
-    int fwd_wt, conv_min_blocks, tv_cluster;  /* 0 = the built-in choice */
+    int fwd_wt, conv_min_blocks, tv_cluster;  /* fwd_wt 0: the batched kernel, tv_cluster 0:
+                                                 automatic */
     double fwd_ms, transpose_ms, tv_prox_ms;  /* per apply of the chosen variant */
     int adj_wt;                               /* instances per CTA of the DAS adjoint (4, 2, 1) */
-    int fwd_staged;                           /* DAS forward: 1 staged, 2 per-detector buckets,
-                                                 4 per-detector buckets, interleaved entries */
-    /* fwd_wt, adj_wt and fwd_staged name the best of the listed kernels; the plan
-     * takes them only where they beat the kernel it runs without tuning, which for
-     * batches is one with lanes over instances */
+    int fwd_staged;                           /* DAS forward: 0 lanes over instances, 1 staged,
+                                                 2 per-detector buckets, 4 per-detector
+                                                 buckets, interleaved entries */
 } msot_tuning;
 int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tuning *out);
 

@@ -87,7 +87,10 @@ struct Plan {
     int adj_groups_max = 0;        // detector groups the partial buffer is sized for
     float *scr_part = nullptr;     // [adj_groups_max][max_batch][P] adjoint partial sums
     struct SolverCache *solver = nullptr;  // solver workspace and captured CUDA graphs
-    // variants chosen by msot_autotune for this plan (0 = the built-in choice)
+    // variants chosen by msot_autotune for this plan (0 = the built-in choice), for
+    // batches of tune_batch instances: at others other kernels are faster
+    int tune_batch = 0;
+    bool tuned(int W) const { return W == tune_batch; }
     int tune_fwd_wt = 0;      // instances per CTA of the DAS forward (8, 4, 2)
     int tune_adj_wt = 0;      // instances per CTA of the DAS adjoint (2, 1)
     int tune_conv_mb = 0;     // register cap of the IR convolution (1, 3, 4)
@@ -342,6 +345,7 @@ extern std::atomic<int> g_fwd_staged;
 // instances per CTA of the DAS forward at batch W: the interpolation input is
 // laid out [W/wt][P][wt] (pixel-major within an instance tile).  operator.cu
 int das_fwd_wt(const Plan &pl, int W);
+void das_fwd_choice(const Plan &pl, int W, int &kernel, int &wt);  // 0: lanes, 1, 2, 4
 bool scatter_order(const Plan &pl);  // k_sir_fwd's image order instead; operator.cu
 
 // C (M x N) = alpha A (M x K) B (K x N), column-major FP32, on the tensor

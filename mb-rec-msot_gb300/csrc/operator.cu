@@ -1225,35 +1225,35 @@ int launch_to_pixmajor(const Plan &pl, const float *in, float *out, int W, cudaS
 std::atomic<int> g_fwd_staged{1};
 std::atomic<int> g_fwd_ell{1};
 
-// the DAS forward kernel: the autotuner's pick, else 4 (the interleaved
-// entry table, the fastest on GB300) when msot_tune_set("fwd_ell") is on
-// (default) and the plan has the table, else 1 (staged) or 2 (k_das_fwd3 on
+// the DAS forward kernel: the autotuner's pick for this batch, else 4 (the
+// interleaved entry table, the fastest on GB300) when msot_tune_set("fwd_ell") is
+// on (default) and the plan has the table, else 1 (staged) or 2 (k_das_fwd3 on
 // the CSR table) by msot_tune_set("fwd_staged"); all give the same sums
-static int fwd_kernel(const Plan &pl) {
-    if (pl.tune_fwd_staged) return pl.tune_fwd_staged;
+static int fwd_kernel(const Plan &pl, int W) {
+    if (pl.tuned(W) && pl.tune_fwd_staged) return pl.tune_fwd_staged;
     if (g_fwd_ell.load() && pl.fwd_ell_off) return 4;
     return g_fwd_staged.load() ? 1 : 2;
 }
 
 // the staged kernel (das_fwd_staged.cu) where the plan has its tables and
 // they fit shared memory at this instance tile, else k_das_fwd3
-static bool use_staged(const Plan &pl, int wt) {
+static bool use_staged(const Plan &pl, int W, int wt) {
     if (pl.image_fmt) return false;  // 16-bit storage is read by k_das_fwd3 only
-    return fwd_kernel(pl) == 1 && fwd_staged_fits(pl, wt);
+    return fwd_kernel(pl, W) == 1 && fwd_staged_fits(pl, wt);
 }
 
 // the lanes-over-instances kernel (das_fwd_lanes.cu) serves batches above 8 of
 // the FP32 input unless the autotuner or a knob chose another kernel
-static bool fwd_lanes(const Plan &pl) {
-    return !pl.tune_fwd_staged && g_fwd_ell.load() && !pl.image_fmt && !pl.S;
+static bool fwd_lanes(const Plan &pl, int W) {
+    return !(pl.tuned(W) && pl.tune_fwd_staged) && g_fwd_ell.load() && !pl.image_fmt && !pl.S;
 }
 
 // instances per CTA of the DAS forward, the last tile part-filled: the
-// autotuner's pick (16, 8, 4, 2), else 32 or 16 for the lanes kernel, else the
+// autotuner's pick for this batch (16, 8, 4, 2), else 32 or 16 for the lanes kernel, else the
 // next power of two up to 8
 int das_fwd_wt(const Plan &pl, int W) {
-    if (pl.tune_fwd_wt && W % pl.tune_fwd_wt == 0 && !pl.S) return pl.tune_fwd_wt;
-    if (!fwd_lanes(pl)) {
+    if (pl.tuned(W) && pl.tune_fwd_wt && !pl.S) return pl.tune_fwd_wt;
+    if (!fwd_lanes(pl, W)) {
         int wt = 1;  // a part-filled tile of 8 costs less than W narrow ones
         while (wt < W && wt < 8) wt *= 2;
         return wt;
@@ -1264,17 +1264,30 @@ int das_fwd_wt(const Plan &pl, int W) {
     return wt;
 }
 
+// the DAS forward that a plan runs for W instances: kernel (0: lanes over instances)
+// and tile
+void das_fwd_choice(const Plan &pl, int W, int &kernel, int &wt) {
+    wt = das_fwd_wt(pl, W);
+    if (wt > 8 && fwd_lanes(pl, W))
+        kernel = 0;
+    else if (use_staged(pl, W, wt) && W % wt == 0)
+        kernel = 1;
+    else
+        kernel = fwd_kernel(pl, W) == 4 && pl.fwd_ell_off ? 4 : 2;
+}
+
 int launch_das_forward(const Plan &pl, const float *xpm, float *raw, int W, float scale,
                        cudaStream_t st, bool to_conv) {
     TimedScope ts_(KID_INTERP_FWD, st);
     const int wt = das_fwd_wt(pl, W);
-    if (wt > 8 && fwd_lanes(pl))
+    if (wt > 8 && fwd_lanes(pl, W))
         return launch_das_forward_lanes(pl, xpm, raw, W, wt, scale,
                                         to_conv ? pl.conv_rng : nullptr, st);
-    if (use_staged(pl, wt) && W % wt == 0) return launch_das_forward_staged(pl, xpm, raw, W, wt, scale, st);
+    if (use_staged(pl, W, wt) && W % wt == 0)
+        return launch_das_forward_staged(pl, xpm, raw, W, wt, scale, st);
     // k_das_fwd3 in the plan's storage format (das_fwd_f32.cu, das_fwd_bf16.cu,
     // das_fwd_f16.cu), on the interleaved entry table where chosen
-    const bool ell = fwd_kernel(pl) == 4 && pl.fwd_ell_off;
+    const bool ell = fwd_kernel(pl, W) == 4 && pl.fwd_ell_off;
     const int2 *skip = to_conv ? pl.conv_rng : nullptr;
     if (pl.image_fmt == 1)
         return das_fwd_run_bf16(pl, xpm, raw, W, scale, nullptr, ell, wt, skip, st);
@@ -1352,7 +1365,7 @@ int launch_das_adjoint(const Plan &pl, const float *raw, float *x, int W, float 
     TimedScope ts_(KID_INTERP_ADJ, st);
     if (batched && adj5_usable(pl, W)) return launch_das_adjoint5(pl, raw, x, W, scale, st);
     int wt = pick_wt(W, 1, 2);
-    if (pl.tune_adj_wt && W % pl.tune_adj_wt == 0) wt = pl.tune_adj_wt;
+    if (pl.tuned(W) && pl.tune_adj_wt) wt = pl.tune_adj_wt;
     if (wt == 4) return das_adj_f<4>(pl, raw, x, W, scale, st);
     if (wt == 2) return das_adj_f<2>(pl, raw, x, W, scale, st);
     return das_adj_f<1>(pl, raw, x, W, scale, st);
@@ -1453,8 +1466,8 @@ constexpr int CONV_FPC = 4;
 // 4 (128 registers, no spills; the fastest on GB300);
 // msot_tune_set("conv_min_blocks")
 std::atomic<int> g_conv_min_blocks{4};
-static int conv_min_blocks(const Plan &pl) {
-    return pl.tune_conv_mb ? pl.tune_conv_mb : g_conv_min_blocks.load();
+static int conv_min_blocks(const Plan &pl, int W) {
+    return pl.tuned(W) && pl.tune_conv_mb ? pl.tune_conv_mb : g_conv_min_blocks.load();
 }
 
 // forward: `in` counts inside each detector's support only; transpose: `out` is
@@ -1474,7 +1487,7 @@ int launch_conv(const Plan &pl, const float *in, float *out, int W, bool transpo
             const ConvRange cr{pl.conv_rng, pl.D, transpose ? 0 : 1};
             dim3 g1(div_up(pl.T, V), div_up(div_up(C, 2), FPC));
             const float4 *Hb = transpose ? pl.fft_hab : pl.fft_hfb;
-            switch (conv_min_blocks(pl)) {
+            switch (conv_min_blocks(pl, W)) {
             case 3:
                 KLAUNCH(k_conv_fft1k<FPC, 0, 3><<<g1, 32 * FPC, 0, st>>>(
                     in, out, pl.fft_twb, pl.fft_twn, Hb, C, pl.T, pl.L, cr));
@@ -1609,7 +1622,7 @@ int apply_forward_update(const Plan &pl, const float *img, float *u, const float
     e.nparts = (pl.D / (2 * CONV_FPC)) * (int)g1.x;
     e.part = part;
     *nparts = e.nparts;
-    const int mb = conv_min_blocks(pl);
+    const int mb = conv_min_blocks(pl, W);
 #define CONV_EPI_LAUNCH(EPI, MB)                                                           \
     KLAUNCH(k_conv_fft1k<CONV_FPC, EPI, MB><<<g1, 32 * CONV_FPC, 0, st>>>(                \
         pl.scr_sino, u, pl.fft_twb, pl.fft_twn, pl.fft_hfb, C, pl.T, pl.L, cr, e))

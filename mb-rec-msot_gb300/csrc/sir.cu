@@ -38,7 +38,7 @@ constexpr int SF_T = 64, SF_WARPS = 4;      // forward: samples per CTA, warps s
 // and one chain was less exact than the former kernel's atomics (128 x 128 px, one
 // image: 3.1e-6 of A x, there 2.2e-6, now 2.0e-6; 8 images 550 -> 624 us)
 constexpr int SF_CH = 2;
-constexpr int SA_THREADS = 256, SA_PIX = 32;  // adjoint: pixels per CTA, a half warp each
+constexpr int SA_THREADS = 256, SA_PIX = 32;  // adjoint: pixels per CTA, two per half warp
 
 // (A, B)[m] of every (column, piece), m = j + F + k over tri taps j = -F ..
 // F + 1 and column samples k; row length S + 2F + 1

@@ -1704,7 +1704,8 @@ int msot_rec_nn_with_TV_reg(msot_plan_t plan, const float *d_b, float *d_rec, in
         for (int k = 0; k < sparsa_iter; ++k) {
             if ((r = apply_transpose(pl, rs, atr, W, s))) return r;
             KLAUNCH(k_tv_z<<<grid, TV_RED, 0, s>>>(x, atr, ri, sv, coupled, z, P, sl, sb));
-            if ((r = tv_prox(z, sv, 0.0, coupled, xn, work, W, N, s, pl.tune_tv_cluster)))
+            if ((r = tv_prox(z, sv, 0.0, coupled, xn, work, W, N, s,
+                             pl.tuned(W) ? pl.tune_tv_cluster : 0)))
                 return r;
             KLAUNCH(k_tv_step<<<grid, TV_RED, 0, s>>>(x, xn, ri, dx, sv, coupled, N, sb, W, part));
             MSOT_LAUNCH_CHECK();
@@ -1852,23 +1853,38 @@ extern "C" int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tun
     MSOT_LAUNCH_CHECK();
     int rc;
     msot_tuning res{};
+    // A variant replaces the built-in choice where it beats it by more than two
+    // timings of one kernel differ; the built-in kernel itself is no candidate.
+    constexpr double GAIN = 0.97;
+    struct Tuned {  // a call that fails leaves the built-in choice
+        Plan &p;
+        bool keep = false;
+        void clear(int batch) {
+            p.tune_batch = batch;
+            p.tune_fwd_wt = p.tune_fwd_staged = p.tune_adj_wt = p.tune_conv_mb = 0;
+            p.tune_tv_cluster = 0;
+        }
+        ~Tuned() {
+            if (!keep) clear(0);
+        }
+    } tuned{pl};
+    tuned.clear(batch);
     // DAS forward: kernel (1 staged, 2 per-detector buckets on the CSR table,
     // 4 the same on the interleaved table) and instances per CTA
     // (apply_forward: prefilter, forward, conv)
     {
-        // fwd_wt and fwd_staged report the best of these; the plan takes it only
-        // where it beats the built-in choice (0)
-        double best = 1e30, builtin = 0.0;
-        int pick = 0, pick_kernel = 0;
-        pl.tune_fwd_wt = pl.tune_fwd_staged = 0;
+        double builtin, best;
+        int pick = 0, pick_kernel = 0, own_kernel, own_wt;
+        das_fwd_choice(pl, batch, own_kernel, own_wt);
         if ((rc = tune_time(st, 3, builtin,
                             [&] { return apply_forward(pl, img, sino, batch, st); })))
             return rc;
+        best = GAIN * builtin;
         for (int kernel : {1, 2, 4}) {
             if (kernel == 1 && !pl.st_tt) continue;
             if (kernel == 4 && !pl.fwd_ell_off) continue;
             for (int wt : {16, 8, 4, 2}) {
-                if (batch % wt) continue;
+                if (batch % wt || (kernel == own_kernel && wt == own_wt)) continue;
                 if (kernel == 1 && !fwd_staged_fits(pl, wt)) continue;
                 pl.tune_fwd_wt = wt;
                 pl.tune_fwd_staged = kernel;
@@ -1879,24 +1895,23 @@ extern "C" int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tun
                 if (ms < best) best = ms, pick = wt, pick_kernel = kernel;
             }
         }
-        pl.tune_fwd_wt = best < builtin ? pick : 0;
-        pl.tune_fwd_staged = best < builtin ? pick_kernel : 0;
-        res.fwd_wt = pick;
-        res.fwd_staged = pick_kernel;
-        res.fwd_ms = std::min(best, builtin);
+        pl.tune_fwd_wt = pick;
+        pl.tune_fwd_staged = pick_kernel;
+        res.fwd_wt = pick ? pick : own_kernel ? own_wt : 0;
+        res.fwd_staged = pick ? pick_kernel : own_kernel;
+        res.fwd_ms = pick ? best : builtin;
     }
-    // DAS adjoint: instances per CTA (apply_transpose)
+    // k_das_adj4: instances per CTA (apply_transpose as the solves call it)
     {
-        // adj_wt reports the best k_das_adj4 tile; the plan takes it only where it
-        // beats the built-in choice (0: the batched kernel from 3 instances up)
-        double best = 1e30, builtin = 0.0;
+        double builtin, best;
         int pick = 0;
-        pl.tune_adj_wt = 0;
+        const int own = batch % 2 ? 1 : 2;
         if ((rc = tune_time(st, 3, builtin,
                             [&] { return apply_transpose(pl, sino, img2, batch, st); })))
             return rc;
+        best = GAIN * builtin;
         for (int wt : {4, 2, 1}) {
-            if (batch % wt) continue;
+            if (batch % wt || wt == own) continue;
             pl.tune_adj_wt = wt;
             double ms;
             if ((rc = tune_time(st, 3, ms,
@@ -1904,14 +1919,20 @@ extern "C" int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tun
                 return rc;
             if (ms < best) best = ms, pick = wt;
         }
-        pl.tune_adj_wt = best < builtin ? pick : 0;
-        res.adj_wt = pick;
+        pl.tune_adj_wt = pick;
+        res.adj_wt = pick ? pick : own;
     }
     // IR convolution register cap (apply_transpose: conv, adjoint, prefilter)
     {
-        double best = 1e30;
-        int pick = 3;
+        double builtin, best;
+        int pick = 0;
+        const int own = g_conv_min_blocks.load();
+        if ((rc = tune_time(st, 3, builtin,
+                            [&] { return apply_transpose(pl, sino, img2, batch, st); })))
+            return rc;
+        best = GAIN * builtin;
         for (int mb : {1, 3, 4}) {
+            if (mb == own) continue;
             pl.tune_conv_mb = mb;
             double ms;
             if ((rc = tune_time(st, 3, ms,
@@ -1920,16 +1941,15 @@ extern "C" int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tun
             if (ms < best) best = ms, pick = mb;
         }
         pl.tune_conv_mb = pick;
-        res.conv_min_blocks = pick;
-        res.transpose_ms = best;
+        res.conv_min_blocks = pick ? pick : own;
+        res.transpose_ms = pick ? best : builtin;
     }
     // SB_ITV2 cluster size (square grids): the automatic choice, every forced
     // size whose vectors fit in shared memory, and (-1) the 16-CTA cluster on
     // the global-memory workspace, which holds more images at once than
     // 16-CTA clusters of one CTA per SM (a cluster stays inside one GPC)
-    res.tv_cluster = 0;
     if (tv_ok) {
-        double best = 1e30;
+        double builtin, best;
         int pick = 0;
         for (int C : {0, 1, 2, 4, 8, 16, -1}) {
             if (C > 0 && !tvc_geometry(pl.nx, batch, C).C) continue;
@@ -1939,12 +1959,16 @@ extern "C" int msot_autotune(msot_plan_t plan, int batch, void *stream, msot_tun
                      return tv_prox(img, nullptr, 0.05, 1, img2, work, batch, pl.nx, st, C);
                  })))
                 return rc;
-            if (ms < best) best = ms, pick = C;
+            if (C == 0)
+                builtin = ms, best = GAIN * ms;
+            else if (ms < best)
+                best = ms, pick = C;
         }
         pl.tune_tv_cluster = pick;
         res.tv_cluster = pick;
-        res.tv_prox_ms = best;
+        res.tv_prox_ms = pick ? best : builtin;
     }
+    tuned.keep = true;
     // the solvers' captured graphs hold the old kernels
     solver_cache_invalidate(pl);
     if (out) *out = res;

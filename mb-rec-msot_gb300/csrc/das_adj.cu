@@ -38,6 +38,7 @@ template <int NI> constexpr int a5_threads = NI == 32 ? 512 : 256;
 // seg rows of NI + 2 words: even, for the knots' 8-byte loads, and staging
 // stores along t meet each bank twice only
 constexpr int A5_PAD = 2;
+constexpr int A5_MIN_BATCH = 5;
 constexpr int A5_RUN = 4;  // buckets that a thread tabulates from one window
 
 struct Adj5Const {
@@ -262,9 +263,18 @@ static size_t adj5_smem(const Plan &pl, int ni) {
            sizeof(float);
 }
 
+// instances per tile: the widest that W fills to more than half and whose
+// tables leave two CTAs per SM (one of twice the threads at 32); 0: none does
+static int adj5_ni(const Plan &pl, int W) {
+    int ni = W > 16 && (W + 31) / 32 * 32 - W < 16 ? 32 : W > 8 ? 16 : 8;
+    while (ni >= 8 && adj5_smem(pl, ni) > (ni == 32 ? 222 : 110) * 1024) ni /= 2;
+    return ni >= 8 ? ni : 0;
+}
+
 int adj5_build(Plan &p, size_t &bytes) {
     const int subs = 4 * p.n_blk;
-    if (p.D > 65535 * 8 || subs > 65535) return MSOT_OK;  // k_das_adj4 serves such plans
+    // k_das_adj4 serves such plans: smaller batches never take the kernel
+    if (p.max_batch < A5_MIN_BATCH || subs > 65535) return MSOT_OK;
     MSOT_CUDA_TRY(cudaMalloc(&p.adj5_span, sizeof(int2) * (size_t)subs * p.D));
     bytes += sizeof(int2) * (size_t)subs * p.D;
     int *most = nullptr;
@@ -282,6 +292,7 @@ int adj5_build(Plan &p, size_t &bytes) {
     if (bits > 11) return MSOT_OK;
     p.adj5_rowbits = bits;
     p.adj5_span_max = span;
+    if (!adj5_ni(p, A5_MIN_BATCH)) return MSOT_OK;  // no tile's tables fit shared memory
     const size_t n = (size_t)subs * p.D * A5_PIX;
     MSOT_CUDA_TRY(cudaMalloc(&p.adj5_ent, sizeof(uint32_t) * n));
     bytes += sizeof(uint32_t) * n;
@@ -322,14 +333,6 @@ static int adj5_f(const Plan &pl, const float *raw, float *part, int W, int grou
     }
 }
 
-// instances per tile: the widest that W fills to more than half and whose
-// tables leave two CTAs per SM (one of twice the threads at 32); 0: none does
-static int adj5_ni(const Plan &pl, int W) {
-    int ni = W > 16 && (W + 31) / 32 * 32 - W < 16 ? 32 : W > 8 ? 16 : 8;
-    while (ni >= 8 && adj5_smem(pl, ni) > (ni == 32 ? 222 : 110) * 1024) ni /= 2;
-    return ni >= 8 ? ni : 0;
-}
-
 // whether k_das_adj5 beats k_das_adj4 for W instances: odd batches (one instance
 // per CTA there) from 5 up, others where three quarters of the instance tiles
 // are filled.  k_das_adj4 / k_das_adj5 in us for 6, 8, 12, 18, 24, 64 images of
@@ -337,7 +340,7 @@ static int adj5_ni(const Plan &pl, int W) {
 // 6, 8, 10, 16, 28: 123 / 128, 166 / 126, 214 / 206, 276 / 207, 403 / 366; 400 x 400 px,
 // 512 detectors, 5, 6, 8, 13: 1083 / 665, 523 / 668, 721 / 660, 2277 / 950
 bool adj5_usable(const Plan &pl, int W) {
-    const int ni = pl.adj5_ent && W >= 5 ? adj5_ni(pl, W) : 0;
+    const int ni = pl.adj5_ent && W >= A5_MIN_BATCH ? adj5_ni(pl, W) : 0;
     return ni && (W % 2 || (W >= 8 && 4 * W >= 3 * ni * div_up(W, ni)));
 }
 

@@ -509,10 +509,13 @@ static int build(const msot_plan_desc *d, Plan &p) {
 #undef UP
     const size_t W = (size_t)p.max_batch;
     if ((rc = alloc(&p.scr_img0, W * p.P, B)) != MSOT_OK) return rc;
-    // the forward's input is padded to whole instance tiles (at most 32); the
-    // padding is read, never used
-    if ((rc = alloc(&p.scr_img1, (W + 31) / 32 * 32 * p.P, B)) != MSOT_OK) return rc;
-    MSOT_CUDA_TRY(cudaMemset(p.scr_img1, 0, (W + 31) / 32 * 32 * p.P * sizeof(float)));
+    // the forward's input is padded to whole instance tiles (das_fwd_wt: the next
+    // power of two up to 16 images, then 16 or 32); the padding is read, never used
+    size_t padded = 1;
+    while (padded < W && padded < 32) padded *= 2;
+    padded = (W + padded - 1) / padded * padded;
+    if ((rc = alloc(&p.scr_img1, padded * p.P, B)) != MSOT_OK) return rc;
+    MSOT_CUDA_TRY(cudaMemset(p.scr_img1, 0, padded * p.P * sizeof(float)));
     if ((rc = alloc(&p.scr_sino, W * p.D * p.T, B)) != MSOT_OK) return rc;
     if ((rc = alloc(&p.h16_sc, 2 * W, B)) != MSOT_OK) return rc;
     p.pre_gain_x = p.pre_gain_z = 1.f;  // bounds of |prefiltered| / max |input|

@@ -240,6 +240,16 @@ class TimedScope {
         }                                                                              \
     } while (0)
 
+// device memory for a table; MSOT_ENOMEM where there is none left
+#define MSOT_MALLOC_TRY(call)                                                          \
+    do {                                                                               \
+        if (cudaError_t e_ = (call)) {                                                 \
+            (void)cudaGetLastError();                                                  \
+            ::msot::set_error("%s: %s", #call, cudaGetErrorString(e_));                \
+            return MSOT_ENOMEM;                                                        \
+        }                                                                              \
+    } while (0)
+
 // interpolation with SIR columns (sir.cu)
 int sir_build(Plan &p, const int32_t *tfx, const int32_t *sidx, const std::vector<int2> &se,
               size_t &bytes);

@@ -275,10 +275,10 @@ int adj5_build(Plan &p, size_t &bytes) {
     const int subs = 4 * p.n_blk;
     // k_das_adj4 serves such plans: smaller batches never take the kernel
     if (p.max_batch < A5_MIN_BATCH || subs > 65535) return MSOT_OK;
-    MSOT_CUDA_TRY(cudaMalloc(&p.adj5_span, sizeof(int2) * (size_t)subs * p.D));
+    MSOT_MALLOC_TRY(cudaMalloc(&p.adj5_span, sizeof(int2) * (size_t)subs * p.D));
     bytes += sizeof(int2) * (size_t)subs * p.D;
     int *most = nullptr;
-    MSOT_CUDA_TRY(cudaMalloc(&most, sizeof(int)));
+    MSOT_MALLOC_TRY(cudaMalloc(&most, sizeof(int)));
     cudaMemset(most, 0, sizeof(int));
     const dim3 grid(p.D, subs);
     KLAUNCH(k_adj5_span<<<grid, 256>>>(p.blk_tau, p.D, p.frac_bits, p.adj5_span, most));
@@ -294,7 +294,7 @@ int adj5_build(Plan &p, size_t &bytes) {
     p.adj5_span_max = span;
     if (!adj5_ni(p, A5_MIN_BATCH)) return MSOT_OK;  // no tile's tables fit shared memory
     const size_t n = (size_t)subs * p.D * A5_PIX;
-    MSOT_CUDA_TRY(cudaMalloc(&p.adj5_ent, sizeof(uint32_t) * n));
+    MSOT_MALLOC_TRY(cudaMalloc(&p.adj5_ent, sizeof(uint32_t) * n));
     bytes += sizeof(uint32_t) * n;
     const double a = p.radius - p.F, b = p.F + 1 - p.radius;
     KLAUNCH(k_adj5_entries<<<grid, 256>>>(p.blk_tau, p.D, p.frac_bits, std::min(a, b),

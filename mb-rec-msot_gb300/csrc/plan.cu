@@ -78,6 +78,7 @@ static int upload(T **dst, const T *src, size_t n, size_t &bytes) {
     }
     cudaError_t e = cudaMalloc((void **)dst, n * sizeof(T));
     if (e != cudaSuccess) {
+        (void)cudaGetLastError();  // reported here, not by the next launch check
         set_error("cudaMalloc(%zu): %s", n * sizeof(T), cudaGetErrorString(e));
         return MSOT_ENOMEM;
     }
@@ -112,7 +113,8 @@ static inline int32_t to_fx(double v, int fb) { return (int32_t)std::nearbyint(s
 static inline int tap_lo(int32_t tau, int32_t r, int fb) { return -((r - tau) >> fb); }
 static inline int tap_hi(int32_t tau, int32_t r, int fb) { return (tau + r) >> fb; }
 
-static int build(const msot_plan_desc *d, Plan &p) {
+// tables: those of the batched kernels too (k_das_adj5, k_sir_fwd2, k_sir_adj2)
+static int build(const msot_plan_desc *d, Plan &p, bool tables) {
     if (!d || d->nx <= 0 || d->nz <= 0 || d->n_det <= 0 || d->n_t <= 1 || !d->travel) {
         set_error("plan: bad grid / detector / sample counts or missing travel table");
         return MSOT_EINVAL;
@@ -369,8 +371,8 @@ static int build(const msot_plan_desc *d, Plan &p) {
         sirf.resize((size_t)p.NS * p.S);
         for (size_t i = 0; i < sirf.size(); ++i) sirf[i] = (float)d->sir[i];
         (void)maxlen;
-        const int rc = sir_build(p, tfx.data(), d->sir_idx, se, p.device_bytes);
-        if (rc != MSOT_OK) return rc;
+        if (tables)
+            if (int rc = sir_build(p, tfx.data(), d->sir_idx, se, p.device_bytes)) return rc;
         if (p.sir_tab) {  // k_sir_fwd's tables stay behind (k_sir_adj keeps its own: operator.cu)
             tpi.clear();
             spi.clear();
@@ -473,7 +475,7 @@ static int build(const msot_plan_desc *d, Plan &p) {
         UP(p.fwd_ell_off, felloff);
         UP(p.blk_tau, btau);
         UP(p.blk_span, bspan);
-        if ((rc = adj5_build(p, B)) != MSOT_OK) return rc;
+        if (tables && (rc = adj5_build(p, B)) != MSOT_OK) return rc;
     }
     if (has_sir) {
         UP(p.sir, sirf);
@@ -567,9 +569,22 @@ int msot_plan_create(const msot_plan_desc *desc, msot_plan_t *out) {
     *out = nullptr;
     msot_plan *h = new (std::nothrow) msot_plan;
     if (!h) return MSOT_ENOMEM;
-    int rc = build(desc, h->p);
-    if (rc != MSOT_OK) {
+    // a plan that does not fit with the batched kernels' tables (32 more bytes per
+    // pixel and detector with SIR, 4 without, and on the host as much) runs the
+    // kernels that need none
+    int rc = MSOT_ENOMEM;
+    for (bool tables : {true, false}) {
+        try {
+            rc = build(desc, h->p, tables);
+        } catch (const std::bad_alloc &) {
+            set_error("plan: out of host memory");
+            rc = MSOT_ENOMEM;
+        }
+        if (rc == MSOT_OK) break;
         free_plan(h->p);
+        if (rc != MSOT_ENOMEM) break;
+    }
+    if (rc != MSOT_OK) {
         delete h;
         return rc;
     }

@@ -408,17 +408,17 @@ int sir_build(Plan &p, const int32_t *tfx, const int32_t *sidx, const std::vecto
     span = (span + 7) / 8 * 8;  // lanes of two groups of instances meet other banks
     if ((size_t)span * 2 * 32 > 100 * 1024) return MSOT_OK;  // two buffers of 8 instances
     p.sir_span_max = span;
-    MSOT_CUDA_TRY(cudaMalloc(&p.sir_aspan, asp.size() * sizeof(int2)));
+    MSOT_MALLOC_TRY(cudaMalloc(&p.sir_aspan, asp.size() * sizeof(int2)));
     MSOT_CUDA_TRY(cudaMemcpy(p.sir_aspan, asp.data(), asp.size() * sizeof(int2),
                              cudaMemcpyHostToDevice));
-    MSOT_CUDA_TRY(cudaMalloc(&p.sir_fent, PD * sizeof(int4)));
-    MSOT_CUDA_TRY(cudaMalloc(&p.sir_aent, na * sizeof(int4)));
-    MSOT_CUDA_TRY(cudaMalloc(&p.sir_off, off.size() * sizeof(int32_t)));
+    MSOT_MALLOC_TRY(cudaMalloc(&p.sir_fent, PD * sizeof(int4)));
+    MSOT_MALLOC_TRY(cudaMalloc(&p.sir_aent, na * sizeof(int4)));
+    MSOT_MALLOC_TRY(cudaMalloc(&p.sir_off, off.size() * sizeof(int32_t)));
     MSOT_CUDA_TRY(cudaMemcpy(p.sir_fent, fe.data(), PD * sizeof(int4), cudaMemcpyHostToDevice));
     MSOT_CUDA_TRY(cudaMemcpy(p.sir_aent, ae.data(), na * sizeof(int4), cudaMemcpyHostToDevice));
     MSOT_CUDA_TRY(cudaMemcpy(p.sir_off, off.data(), off.size() * sizeof(int32_t),
                              cudaMemcpyHostToDevice));
-    MSOT_CUDA_TRY(cudaMalloc(&p.sir_tab, tab * sizeof(float2)));
+    MSOT_MALLOC_TRY(cudaMalloc(&p.sir_tab, tab * sizeof(float2)));
     bytes += (PD + na) * sizeof(int4) + asp.size() * sizeof(int2) + off.size() * sizeof(int32_t) + tab * sizeof(float2);
     p.sir_jmin = jmin;
     p.sir_nj = nj;

@@ -30,3 +30,34 @@ def test_a_plan_holds_what_its_batches_use(cuda):
     assert b[4] - b[1] == per_batch(4) - per_batch(1)
     # the batched adjoint serves five images and more: 4 bytes per (padded pixel, detector)
     assert b[5] - b[4] >= per_batch(5) - per_batch(4) + 4 * 128 * 128 * D
+
+
+@pytest.mark.parametrize("sir", [False, True])
+def test_tables_that_do_not_fit_are_left_out(cuda, sir):
+    import torch
+    n, D, W = (160, 256, 5) if sir else (320, 192, 5)
+    rng = np.random.default_rng(3)
+    tab = None
+    if sir:
+        idx = rng.integers(1, 5, (D, n * n)).astype(np.int32)
+        tab = (rng.standard_normal((4, 31)), np.tile(np.int32([[1, 31]]), (4, 1)), idx)
+
+    def model():
+        return make_pair(n=n, n_det=D, n_samples=T, radius=0.02, fov_half=0.006, norm=2e-5,
+                         max_batch=W, sir_tables=tab)[0]
+
+    y = torch.tensor(rng.standard_normal((W, D, T)), dtype=torch.float32).cuda()
+    m = model()
+    want, full = m.transpose(y), _bytes(m)
+    del m
+    tables = (24 if sir else 4) * D * n * n  # SIR: 32 bytes a pair for the 8 of k_sir_fwd
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    hog = torch.empty(free - (full - tables // 2), dtype=torch.uint8, device="cuda")
+    m = model()
+    del hog
+    torch.cuda.empty_cache()
+    assert _bytes(m) < full - 0.9 * tables
+    got = m.transpose(y)
+    assert float((got - want).norm() / want.norm()) < 1e-5

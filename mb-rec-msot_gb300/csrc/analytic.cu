@@ -326,13 +326,17 @@ static cudaMemPool_t analytic_pool() {
     return pools[dev];
 }
 
+// Host tables are copied asynchronously and, where the GPU reads pageable memory
+// itself, without a staging copy: they live here until the copies are done.
 struct DevMem {
     cudaStream_t st;
     std::vector<void *> ptrs;
+    std::vector<std::vector<char>> host;
     explicit DevMem(cudaStream_t s) : st(s) {}
     DevMem(const DevMem &) = delete;
     DevMem &operator=(const DevMem &) = delete;
     ~DevMem() {
+        if (!host.empty()) cudaStreamSynchronize(st);
         for (void *p : ptrs) cudaFreeAsync(p, st);
     }
     template <class T>
@@ -352,7 +356,10 @@ struct DevMem {
     int put(T **p, const T *h, size_t n) {
         int rc = get(p, n);
         if (rc) return rc;
-        MSOT_CUDA_TRY(cudaMemcpyAsync(*p, h, n * sizeof(T), cudaMemcpyHostToDevice, st));
+        const char *b = reinterpret_cast<const char *>(h);
+        host.emplace_back(b, b + n * sizeof(T));
+        MSOT_CUDA_TRY(
+            cudaMemcpyAsync(*p, host.back().data(), n * sizeof(T), cudaMemcpyHostToDevice, st));
         return MSOT_OK;
     }
 };

@@ -317,6 +317,10 @@ int msot_backproject_waveeq(const float *d_sig, int W, int D, int T, const doubl
                             double coverage_deg, double radius, const double *psf, int psf_m,
                             int psf_n, const float *d_K, int K_n, float *d_out, void *stream);
 
+/* The two calls above keep up to 512 MiB of workspace per device for the next
+ * call.  This waits for the device and gives back what no call in flight uses. */
+int msot_release_workspaces(void);
+
 /* ------------------------------------------------------------------------ */
 /* Learned warm start (no counterpart in the reference): a U-Net that maps an
  * image (e.g. the adjoint of the data) to an NNLS start.  levels, base

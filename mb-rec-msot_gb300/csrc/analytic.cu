@@ -303,16 +303,16 @@ static std::vector<double> reciprocal_steps(const double *x, int n) {
 // Workspaces of one call, from a stream-ordered pool of the library's own
 // (one per device) instead of a dozen cudaMalloc / cudaFree, which synchronise, per
 // call.  The pool keeps at most POOL_KEEP bytes between calls, the rest goes
-// back at the call's synchronisation.
+// back at the call's synchronisation; msot_release_workspaces gives back what it keeps.
 constexpr uint64_t POOL_KEEP = 512ull << 20;
+constexpr int POOL_DEVICES = 64;
+static cudaMemPool_t g_pools[POOL_DEVICES] = {};
+static std::mutex g_pools_mu;
 static cudaMemPool_t analytic_pool() {
-    constexpr int kMaxDev = 64;
-    static cudaMemPool_t pools[kMaxDev] = {};
-    static std::mutex mu;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return nullptr;
-    std::lock_guard<std::mutex> g(mu);
-    if (!pools[dev]) {
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= POOL_DEVICES) return nullptr;
+    std::lock_guard<std::mutex> g(g_pools_mu);
+    if (!g_pools[dev]) {
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -321,9 +321,9 @@ static cudaMemPool_t analytic_pool() {
         if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
         uint64_t keep = POOL_KEEP;
         cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-        pools[dev] = p;
+        g_pools[dev] = p;
     }
-    return pools[dev];
+    return g_pools[dev];
 }
 
 // Host tables are copied asynchronously and, where the GPU reads pageable memory
@@ -431,6 +431,21 @@ static int index_table(DevMem &m, int D, int T, const double *x, int nx, const d
 using namespace msot;
 
 extern "C" {
+
+int msot_release_workspaces(void) {
+    std::lock_guard<std::mutex> g(g_pools_mu);
+    for (int dev = 0; dev < POOL_DEVICES; ++dev) {
+        if (!g_pools[dev]) continue;
+        int was = 0;
+        MSOT_CUDA_TRY(cudaGetDevice(&was));
+        MSOT_CUDA_TRY(cudaSetDevice(dev));
+        cudaError_t e = cudaDeviceSynchronize();  // frees of calls just made
+        if (e == cudaSuccess) e = cudaMemPoolTrimTo(g_pools[dev], 0);
+        cudaSetDevice(was);
+        MSOT_CUDA_TRY(e);
+    }
+    return MSOT_OK;
+}
 
 int msot_dmas_cf(const float *d_sig, int W, int D, int T, const double *x, int nx,
                  const double *z, int nz, double c, double fs, double n_crop, double coverage_deg,

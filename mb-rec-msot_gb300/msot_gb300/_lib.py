@@ -149,6 +149,7 @@ SIGNATURES = {
     "msot_prep_destroy": (C.c_int, [_vp]),
     "msot_butter_response": (C.c_int, [C.c_int, C.c_int, C.c_double, C.c_double, C.c_int, C.c_int,
                                        _dp]),
+    "msot_release_workspaces": (C.c_int, []),
     "msot_dmas_cf": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int, _dp, C.c_int, _dp, C.c_int,
                                C.c_double, C.c_double, C.c_double, C.c_double, C.c_double,
                                _vp, _vp, _vp, _vp, _vp]),

@@ -128,3 +128,9 @@ def bp_kernel_device(t, device="cuda"):
     takes directly."""
     K = bp_kernel(t)
     return torch.tensor(np.ascontiguousarray(K.T), dtype=torch.float32, device=device)
+
+
+def release_workspaces():
+    """msot_release_workspaces: give back the device memory (up to 512 MiB) that dmas_cf
+    and backproject_waveeq keep between calls."""
+    _lib.check(_lib.load().msot_release_workspaces())

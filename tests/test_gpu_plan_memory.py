@@ -61,3 +61,27 @@ def test_tables_that_do_not_fit_are_left_out(cuda, sir):
     assert _bytes(m) < full - 0.9 * tables
     got = m.transpose(y)
     assert float((got - want).norm() / want.norm()) < 1e-5
+
+
+def test_analytic_workspaces_are_given_back(cuda):
+    import torch
+    from msot_gb300 import dmas_cf
+    from msot_gb300.analytic import release_workspaces
+    sig = torch.randn(4, 64, 1200, device="cuda")
+    x = np.linspace(-0.005, 0.005, 256)
+
+    def call():  # the index table alone is 16 MiB
+        out = dmas_cf(sig, x, x, 1500.0, 4e7, 0.0, 135.0, 0.015)
+        torch.cuda.synchronize()
+        return out
+
+    kept = call()  # results and modules stay
+    release_workspaces()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    again = call()
+    assert torch.cuda.mem_get_info()[0] <= free - (16 << 20)
+    release_workspaces()
+    del kept, again
+    torch.cuda.empty_cache()
+    assert torch.cuda.mem_get_info()[0] >= free

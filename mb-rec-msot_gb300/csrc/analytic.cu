@@ -173,7 +173,40 @@ __global__ void __launch_bounds__(32 * CT_WARPS) k_cumtrapz(const float *__restr
     __syncwarp();
     const int a = min(lane * per, T), b = min(a + per, T);
     Sum1 own;
-    for (int t = a; t < b; ++t) own.add(buf[t]);
+    float big = 0.f;
+    for (int t = a; t < b; ++t) {
+        own.add(buf[t]);
+        big = fmaxf(big, fabsf(buf[t]));
+    }
+    if (__any_sync(0xffffffffu, !(big * T < 1e38f))) {
+        // twice the sum may leave FP32's range: the trapezoids in FP64
+        double acc = 0.0;
+        float prev = a > 0 && a < T ? buf[a - 1] : first;
+        const float before = prev;
+        for (int t = a; t < b; prev = buf[t++])
+            if (t) acc += 0.5 * ((double)buf[t] + (double)prev);
+        double run = acc;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const double u = __shfl_up_sync(0xffffffffu, run, k);
+            if (lane >= k) run += u;
+        }
+        run = __shfl_up_sync(0xffffffffu, run, 1);
+        acc = lane ? run : 0.0;
+        prev = before;
+        __syncwarp();  // every lane has read its neighbour's last sample
+        for (int t = a; t < b; ++t) {
+            const float v = buf[t];
+            if (t) acc += 0.5 * ((double)v + (double)prev);
+            prev = v;
+            const float2 f = __ldg(fac + t);
+            buf[t] = t ? (float)(2.0 * acc * ((double)f.x + (double)f.y)) : 0.f;
+        }
+        __syncwarp();
+        if (staged)
+            for (int t = lane; t < T; t += 32) o[t] = buf[t];
+        return;
+    }
     // exclusive scan of the lanes' sums (FP64: five steps per column)
     double run = own.value();
 #pragma unroll

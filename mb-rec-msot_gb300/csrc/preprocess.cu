@@ -91,12 +91,20 @@ static double zpk_mag(const std::vector<cd> &z, const std::vector<cd> &p, double
     return std::abs(h);
 }
 
-// the warp's FP64 sum of the lanes' pairs of floats, in every lane
-__device__ __forceinline__ double warp_total(const Sum1 &q) {
-    double v = q.value();
+// the warp's FP64 sum of the lanes' values, in every lane
+__device__ __forceinline__ double warp_total(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+// the sum of a warp's column from the lanes' pairs of floats; where they left
+// FP32's range (sums above 3.4e38, infinities) again in FP64
+__device__ __forceinline__ double column_total(const Sum1 &q, const float *col, int T) {
+    const double v = warp_total(q.value());
+    if (isfinite(v)) return v;  // the same in every lane
+    double a = 0.0;
+    for (int t = threadIdx.x & 31; t < T; t += 32) a += (double)col[t];
+    return warp_total(a);
 }
 
 // One warp per column: x = raw[n_crop .. n_crop + T); window; demean.  The
@@ -121,7 +129,7 @@ __global__ void __launch_bounds__(32 * PC_WARPS) k_prep_columns(
         s.add(v);
     }
     if (win) {
-        const double m = warp_total(s) / T;
+        const double m = column_total(s, col, T) / T;
         const float mh = (float)m, ml = (float)(m - (double)mh);
         s = Sum1();
         for (int t = lane; t < T; t += 32) {
@@ -140,7 +148,7 @@ __global__ void __launch_bounds__(32 * PC_WARPS) k_prep_columns(
         }
     }
     float *dst = out + (size_t)c * ldo;
-    const float m = demean ? (float)(warp_total(s) / T) : 0.f;
+    const float m = demean ? (float)(column_total(s, col, T) / T) : 0.f;
     for (int t = lane; t < T; t += 32) dst[t] = demean ? col[t] - m : col[t];
 }
 

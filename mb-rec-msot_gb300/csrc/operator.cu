@@ -150,7 +150,7 @@ __global__ void k_prefilter(const float *__restrict__ in, float *__restrict__ ou
 // us); batch 64 at 128 x 128 px 23 -> 14 to 16 us, the stores were the bound.
 //
 // XF: x first, then z (IPC = 1, out_mode 0).  The transpose takes the axes in the
-// order that launch_prefilter2d names, so that its sums round as they did.
+// order that prefilter2d_km names, so that its sums round as they did.
 // ---------------------------------------------------------------------------
 constexpr int PF_T = 32, PF_RZ = 8, PF_RX = 4, PF_THREADS = 256;
 

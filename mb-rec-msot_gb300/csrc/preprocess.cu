@@ -18,8 +18,8 @@
 // MATLAB's and scipy's butter; the responses are evaluated from the
 // zero-pole-gain form.  Host FP64.
 //
-// GPU: k_prep_columns (one CTA per column: crop, window, demean; FP64 means)
-// and, for the zero-phase filter, the circular convolution with
+// GPU: k_prep_columns (one warp per column: crop, window, demean; means from
+// sums in pairs of floats) and, for the zero-phase filter, the circular convolution with
 // h = ifft(|H|^2) as one FP32 GEMM with the T x T circulant on the tensor
 // cores (gemm_tc.cu): 2 T^2 flops per column instead of an arbitrary-length
 // FFT.

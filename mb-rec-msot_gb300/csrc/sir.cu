@@ -77,7 +77,10 @@ __global__ void __launch_bounds__(128) k_sir_table(const float *__restrict__ sir
 
 // Every load of the two kernels has an address inside its array, also where the
 // value is not used: no load depends on a predicate for that (windows reach far
-// past both ends of a row's table and of the sinogram).
+// past both ends of a row's table and of the sinogram).  A precaution: an earlier
+// form, which predicated these loads instead, met a memory fault, and reading
+// its entries, rows, offsets and indices did not show why (a load that is
+// predicated off reads nothing).
 
 // window start (low 16 bits hold the length)
 __device__ __forceinline__ int se_start(int v) { return v >> 16; }

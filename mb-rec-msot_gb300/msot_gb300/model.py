@@ -372,7 +372,8 @@ class MSOTmodel:
 
     def autotune(self, batch: int | None = None, stream=None) -> dict:
         """msot_autotune: time the kernel variants on this model's geometry at
-        ``batch`` instances (default max_batch) and keep the fastest."""
+        ``batch`` instances (default max_batch) and keep, for batches of that
+        size, those that beat the built-in choice."""
         t = _lib.Tuning()
         _lib.check(_lib.load().msot_autotune(self.plan, int(batch or self.max_batch),
                                              _stream_ptr(stream), C.byref(t)))

@@ -1,5 +1,7 @@
 """Device memory of a plan: nothing that its batches cannot use, and the kernels with
 tables of their own are left out where those do not fit."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -50,6 +52,7 @@ def test_tables_that_do_not_fit_are_left_out(cuda, sir):
     m = model()
     want, full = m.transpose(y), _bytes(m)
     del m
+    gc.collect()  # models refer to themselves: this one and other tests' now, not later
     tables = (24 if sir else 4) * D * n * n  # SIR: 32 bytes a pair for the 8 of k_sir_fwd
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
@@ -75,6 +78,7 @@ def test_analytic_workspaces_are_given_back(cuda):
         torch.cuda.synchronize()
         return out
 
+    gc.collect()
     kept = call()  # results and modules stay
     release_workspaces()
     torch.cuda.synchronize()

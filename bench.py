@@ -848,7 +848,7 @@ def run_bp(args):
                                    "gemm_flops": flops,
                                    "gemm_tflops_fp32_equiv_upper_bound": flops / (bp_ms * 1e9)},
             "dmas_cf": {"ms_per_256_frames": dm_ms, "frames_per_s": F / (dm_ms / 1e3)},
-            "steps": args.steps, "warmup": args.warmup, "dtype": "f32 (FP64 indices / sums)",
+            "steps": args.steps, "warmup": args.warmup, "dtype": "f32 (FP64 indices, sums in pairs of floats)",
             "data": "synthetic Gaussian noise sinograms",
             "config": {"workload": f"{F} frames, {D} det x {T} samples, {n} x {n} px"}}
 
